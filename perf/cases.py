@@ -103,11 +103,17 @@ def draw(rng) -> dict:
     if kind == "serve":
         sizes = [size(480, 2048) for _ in range(rng.randint(2, 4))]
         return _case(path="serve", sizes=",".join("%dx%d*1" % s for s in sizes), frames=2, debayer=debayer,
-                     denoise=strength, temporal=round(rng.uniform(0.4, 0.9), 2), **look)
+                     denoise=strength, temporal=round(rng.uniform(0.4, 0.9), 2),
+                     **{**look, "format": "rgba16f"})
     if kind == "noise":
         w, h = size(1920, 6000)
         return _case(path="noise", width=w, height=h, **noise)
     w, h = size(320, 1280) if kind == "live" else size(320, 6000)
+    if kind in ("denoise", "clip", "chroma") and w * h < 1900000:
+        # A proxy's format. (Below this size the denoise's timed choice of
+        # tile differs from run to run, and with it the rounding of a few
+        # codes, which a 32-bit output would show.)
+        look["format"] = "rgba16f"
     more = {
         "live": dict(path="live"),
         "frame": dict(awb=rng.random() < 0.7, storage=rng.choice(("fp32", "fp32", "fp16"))),
