@@ -927,9 +927,8 @@ def debug_rcd_tma(on: bool) -> bool:
 
 
 def debug_rcd_strips(mode: int) -> int:
-    """RCD interior by 64x16 tiles (0), by strips unless the colour stage
-    has the gamut compression (1, the default), or by strips wherever they
-    apply (2); -1 only reads. Returns the previous setting."""
+    """RCD interior by 64x16 tiles (0) or by walking strips (1, the default,
+    and 2); -1 only reads. Returns the previous setting."""
     return int(lib().craw_debug_rcd_strips(int(mode)))
 
 

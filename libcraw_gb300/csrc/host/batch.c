@@ -126,7 +126,6 @@ static int batch_autotune(CRAWBatch *b)
             F->dn.inv_range[s] = 16.0f;
             F->dn.range[s] = 0.0625f;
             F->dv.inv_range[s] = 16.0f;
-            F->dv.range[s] = 0.0625f;
             F->dv.wbs[s] = 1.0f;
         }
         F->dio.src = mosaic;

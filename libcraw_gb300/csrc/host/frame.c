@@ -101,7 +101,6 @@ int craw_develop_consts(CRAWContext *ctx, uint32_t w, uint32_t h, int debayer, b
             return CRAW_ERROR(EINVAL);
         }
         dk->black[s] = fp->profile->black_level[s];
-        dk->range[s] = range;
         dk->inv_range[s] = 1.0f / range;
         dk->wbs[s] = frame.wb[chan[s]];
     }
@@ -123,6 +122,7 @@ int craw_develop_consts(CRAWContext *ctx, uint32_t w, uint32_t h, int debayer, b
             dk->color.m[i][j] *= scale;
         dk->color.gc_thr[i] = gc.thr[i];
         dk->color.gc_scl[i] = gc.scl[i];
+        dk->color.gc_iscl[i] = 1.0f / gc.scl[i];
     }
     dk->color.gc_pwr = gc.pwr;
     dk->color.gc_inv_pwr = gc.inv_pwr;

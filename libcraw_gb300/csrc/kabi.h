@@ -154,13 +154,13 @@ int craw_k_plain_denoise(const CRAWKDenoise *k, const CRAWKDenoiseIO *io,
 /* The colour stage (the reference's CRAWColorPush, lib/pipeline.c:1905-1931). */
 typedef struct CRAWKColor {
     float m[3][3];        /* rows of M_out * cam_to_xyz * gain * 2^stops */
-    float gc_thr[3], gc_scl[3], gc_pwr, gc_inv_pwr;
+    float gc_thr[3], gc_scl[3], gc_iscl[3], gc_pwr, gc_inv_pwr;   /* gc_iscl = 1 / gc_scl */
     uint32_t flags;       /* CRAW_K_COLOR_* */
 } CRAWKColor;
 
 typedef struct CRAWKDevelop {
     int32_t width, height;
-    float black[4], range[4], inv_range[4], wbs[4];   /* per site; wbs = gain of the site's channel */
+    float black[4], inv_range[4], wbs[4];   /* per site; wbs = gain of the site's channel */
     float clip;                         /* 1.0 */
     int32_t method;                     /* CRAW_DEBAYER_* */
     int32_t fp16;                       /* intermediate values rounded to half */
@@ -229,10 +229,9 @@ int craw_k_develop_prepare(int method);
  * tile copy; 0: with plain loads (craw_debug_rcd_tma). */
 extern int craw_k_rcd_tma;
 
-/* The RCD's interior by 64x16 tiles (0), by strips (one quad column a
- * thread walking down a segment of quad rows) unless the colour stage
- * has the gamut compression (1, the default), or by strips wherever they
- * apply (2): craw_debug_rcd_strips. The two give the same bits. */
+/* The RCD's interior by 64x16 tiles (0) or by walking strips (one quad
+ * column a lane walking down a segment of quad rows: 1, the default, and
+ * 2): craw_debug_rcd_strips. The two give the same bits. */
 extern int craw_k_rcd_strips;
 
 /* ------------------------------------------------------------- chroma */

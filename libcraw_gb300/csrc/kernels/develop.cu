@@ -7,14 +7,14 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "develop_strip.cuh"
 #include "develop_tile.cuh"
+#include "develop_walk.cuh"
 #include "tma.cuh"
 
 /* Whether the RCD interior tiles load their mosaic by TMA (1, the
  * default) or by plain loads (0, for comparison and tests); whether the
- * interior runs by 64x16 tiles (0), by strips where they are the faster
- * (1, the default) or by strips wherever they apply (2). */
+ * interior runs by 64x16 tiles (0, for comparison and tests) or by walking
+ * strips (1, the default; 2). */
 extern "C" {
 int craw_k_rcd_tma = 1;
 int craw_k_rcd_strips = 1;
@@ -126,14 +126,19 @@ k_develop_rcd_quads_tma(const CRAWKDevelop k, const CRAWKDevelopIO io, const Qua
     epilogue<QTW, QTH, QNT>(k, io, x0, y0, t.rgb);
 }
 
-/* The interior by strips (develop_strip.cuh): SOUT x seg output quads a
- * CTA, four CTAs an SM (55 KB of shared memory each). */
-__global__ void __launch_bounds__(SNT, 4)
-k_develop_rcd_strips(const CRAWKDevelop k, const CRAWKDevelopIO io, const StripGrid g)
+/* The interior by walking warps (develop_walk.cuh), WALK_CTAS CTAs an SM:
+ * 168 registers a thread and no spills (four CTAs an SM: 128 registers, up
+ * to 340 bytes of spills). */
+constexpr int WALK_CTAS = 3;
+
+template <int FMT, bool RGC, bool MORE>
+__global__ void __launch_bounds__(WALK_NT, WALK_CTAS)
+k_develop_rcd_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
 {
-    extern __shared__ __align__(16) float smem[];
+    __shared__ WalkSmem<RW_NQ> smem[WALK_WARPS];
     release_border();
-    rcd_strip(k, io, g, blockIdx.x, blockIdx.y, *reinterpret_cast<StripSmem *>(smem));
+    const int warp = threadIdx.x >> 5;
+    rcd_walk<FMT, RGC, MORE>(k, io, g, blockIdx.x * WALK_WARPS + warp, smem[warp]);
 }
 
 /* The per-pixel RCD on the ring of border quad tiles, BTW x BTH pixels a
@@ -192,12 +197,27 @@ int craw_sm_count()
 int prepare_rcd()
 {
     constexpr size_t smem = RcdQuads<QTW, QTH, QNT>::floats * sizeof(float);
-    static std::atomic<uint64_t> attr_plain{ 0 }, attr_tma{ 0 }, attr_strips{ 0 };
+    static std::atomic<uint64_t> attr_plain{ 0 }, attr_tma{ 0 };
     if (craw_smem_attr(k_develop_rcd_quads, smem, attr_plain) < 0 ||
-        craw_smem_attr(k_develop_rcd_quads_tma, smem, attr_tma) < 0 ||
-        craw_smem_attr(k_develop_rcd_strips, sizeof(StripSmem), attr_strips) < 0)
+        craw_smem_attr(k_develop_rcd_quads_tma, smem, attr_tma) < 0)
         return -5;
     return 0;
+}
+
+/* The walking kernel for a frame's output. */
+auto walk_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io)
+{
+    const bool rgc = k->color.flags & CRAW_K_COLOR_RGC;
+    if (k->fp16 || io->inter || io->quarter || !io->dst)
+        return k_develop_rcd_walk<0, false, true>;
+    switch (io->dst_fmt) {
+    case CRAW_K_OUT_RGBA16F:
+        return rgc ? k_develop_rcd_walk<CRAW_K_OUT_RGBA16F, true, false> : k_develop_rcd_walk<CRAW_K_OUT_RGBA16F, false, false>;
+    case CRAW_K_OUT_RGB32F:
+        return rgc ? k_develop_rcd_walk<CRAW_K_OUT_RGB32F, true, false> : k_develop_rcd_walk<CRAW_K_OUT_RGB32F, false, false>;
+    default:
+        return rgc ? k_develop_rcd_walk<CRAW_K_OUT_RGBA32F, true, false> : k_develop_rcd_walk<CRAW_K_OUT_RGBA32F, false, false>;
+    }
 }
 
 int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
@@ -207,29 +227,23 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
         return -5;
     QuadGrid g;
     g.init(k->width, k->height);
-    /* Strips unless the colour stage carries the gamut compression (its
-     * long chains of MUFU work sit in front of every step's barrier with
-     * 16 warps an SM to hide them: the strips take 0.260 ms against the
-     * tiles' 0.255 ms at 5760x3240 with it, 0.213 against 0.250 without),
-     * or the chroma path (the tiles' epilogue writes its block means). */
-    const bool strips = craw_k_rcd_strips == 2 ||
-                        (craw_k_rcd_strips == 1 && !(k->color.flags & CRAW_K_COLOR_RGC));
-    if (g.interior_x() > 0 && g.interior_y() > 0 && strips && !io->quarter) {
-        /* The interior tiles' region as strips. */
-        StripGrid sg;
-        sg.qx0 = g.c_lo * (QTW / 2);
-        sg.nqx = g.interior_x() * (QTW / 2);
-        sg.qy0 = g.r_lo * (QTH / 2);
-        sg.nqy = g.interior_y() * (QTH / 2);
-        /* Segments as tall as one wave of four CTAs an SM allows (a taller
-         * segment recomputes less of its passes' first rows), at least 8
-         * quad rows. */
-        const int gx = (sg.nqx + SOUT - 1) / SOUT;
-        const int nseg = (4 * craw_sm_count()) / gx > 1 ? (4 * craw_sm_count()) / gx : 1;
-        sg.seg = 4 * ((sg.nqy / 4 + nseg - 1) / nseg);
-        sg.seg = sg.seg < 8 ? 8 : sg.seg;
-        const dim3 grid(gx, (sg.nqy + sg.seg - 1) / sg.seg);
-        k_develop_rcd_strips<<<grid, SNT, sizeof(StripSmem), s>>>(*k, *io, sg);
+    if (g.interior_x() > 0 && g.interior_y() > 0 && craw_k_rcd_strips) {
+        /* The interior tiles' region by walking warps, in segments of one
+         * wave of the device (a segment repeats the passes of six quad rows
+         * to start, so it is as tall as one wave allows), at least 8 quad
+         * rows. */
+        WalkGrid w;
+        w.qx0 = g.c_lo * (QTW / 2);
+        w.nqx = g.interior_x() * (QTW / 2);
+        w.qy0 = g.r_lo * (QTH / 2);
+        w.nqy = g.interior_y() * (QTH / 2);
+        w.nx = (w.nqx + RW_NQ - 1) / RW_NQ;
+        const int room = craw_sm_count() * WALK_CTAS * WALK_WARPS / w.nx;
+        const int nseg = room > 1 ? room : 1;
+        w.seg = 4 * ((w.nqy / 4 + nseg - 1) / nseg);
+        w.seg = w.seg < 8 ? 8 : w.seg;
+        const int warps = w.nx * ((w.nqy + w.seg - 1) / w.seg);
+        walk_rcd(k, io)<<<(warps + WALK_WARPS - 1) / WALK_WARPS, WALK_NT, 0, s>>>(*k, *io, w);
         if (cudaGetLastError() != cudaSuccess)
             return -5;
     } else if (g.interior_x() > 0 && g.interior_y() > 0) {

@@ -272,7 +272,7 @@ struct RcdTile {
 /* ------------------------------------------- RCD arithmetic of the quads */
 
 /* The RCD formulas of reference lib/ref/ref_debayer.c:204-395 as the quad
- * forms (tiles and strips) evaluate them, every rounding explicit, so that
+ * forms (tiles and walking strips) evaluate them, every rounding explicit, so that
  * both give the same bits whatever the compiler contracts around them. */
 
 /* 1/x on the MUFU (x >= 1e-5 wherever it is used: no denormals). */

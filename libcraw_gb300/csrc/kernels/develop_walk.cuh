@@ -1,0 +1,535 @@
+/*
+ * The develop stage by walking warps: a warp owns a strip of quad columns,
+ * one column a lane, and walks down a segment of it one quad row (two
+ * pixel rows) a step. What a column needs of its neighbours comes by warp
+ * shuffles and what it needs of earlier rows stays in registers, so a step
+ * has no barrier, no shared-memory ring and no index arithmetic beyond its
+ * row pointers. The epilogue (intermediate, colour stage, stores, AWB
+ * statistic) takes the quad's four pixels from the lane's registers.
+ *
+ * A strip has NQ output columns on lanes A .. A + NQ - 1; the lanes outside
+ * them are the strip's apron and compute values that only their inner
+ * neighbours read.
+ *
+ * Bound: instruction issue. The RCD takes 555 warp instructions a step of
+ * 24 quads (110 M at 5760x3240, 74 % of the issue slots busy, 128 us), where
+ * a column-a-thread kernel that passed its rows through shared-memory rings
+ * between two barriers a step took 156 M (173 us) and 64x16 tiles 204 M
+ * (233 us with the gamut compression, 140 us here): a third to a half of
+ * their instructions were ring and tile addressing and the tiles' aprons.
+ * Two steps a round of the loop halve the moves from one step's registers
+ * to the next's; four (100 M instructions) wait longer on the spills and
+ * loads than they save.
+ */
+#pragma once
+
+#include <string.h>
+
+#include "develop_tile.cuh"
+
+namespace craw_dev {
+
+/* The frame's part the strips cover, in quads: columns qx0 .. qx0 + nqx,
+ * rows qy0 .. qy0 + nqy, in segments of `seg` rows a warp, `nx` strips
+ * across. qx0, qy0, seg and a strip's output columns are multiples of 4, so
+ * that strips and segments start on 8x8 AWB blocks. */
+struct WalkGrid {
+    int qx0, nqx, qy0, nqy, seg, nx;
+};
+
+constexpr int WALK_WARPS = 4, WALK_NT = 32 * WALK_WARPS;   /* warps (strips) a CTA */
+
+CRAW_DEV float walk_left(float v)    /* the left neighbour's v */
+{
+    return __shfl_up_sync(0xffffffffu, v, 1);
+}
+CRAW_DEV float walk_right(float v)
+{
+    return __shfl_down_sync(0xffffffffu, v, 1);
+}
+
+/* A row's sample pair, a step before it is used: volatile, so that the load
+ * stays where it is written. */
+CRAW_DEV uint32_t walk_ld(const char *p)
+{
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
+/* Eight floats to a 32-byte aligned address in one store. */
+CRAW_DEV void walk_store8(float *p, float a, float b, float c, float d, float e, float f, float g, float h)
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h) : "memory");
+}
+
+/* Shared memory of one warp: the camera RGB of the AWB block row in
+ * progress (eight pixel rows, planar a row: 4 floats of padding after 32
+ * spread the blocks a fold reads over the banks), and the sums of the
+ * blocks that wait for their statistic. */
+template <int NQ>
+struct WalkSmem {
+    static constexpr int PW = 2 * NQ, PITCH = PW + 4 * ((PW - 1) / 32);
+    static constexpr int NB = NQ / 4, HOLD = 32 / NB;      /* blocks a row; block rows held */
+    alignas(16) float a[8][3][PITCH];
+    float sum[HOLD * NB][3];
+    float cnt[HOLD * NB];
+    int where[HOLD * NB];
+    CRAW_DEV static int col(int x) { return x + 4 * (x >> 5); }
+};
+
+/* The epilogue of one warp: takes the camera RGB of the four pixels of each
+ * lane's quad, a quad row at a time. FMT (a CRAW_K_OUT_* layout), RGC (the
+ * gamut compression): fixed per kernel, so that a step's code stays small
+ * enough for the instruction cache; MORE: any layout, FP16 storage, the
+ * kept intermediate and the chroma path's block means, by tests. */
+template <int NQ, int A, int FMT, bool RGC, bool MORE>
+struct WalkOut {
+    using S = WalkSmem<NQ>;
+    const CRAWKDevelop &k;
+    const CRAWKDevelopIO &io;
+    S &s;
+    int lane, nout;          /* the strip's output columns (a multiple of 4 but at the frame's right edge) */
+    int qx, qy;              /* the strip's first output quad, the segment's first quad row */
+    bool mine;               /* the lane has an output column */
+    int held;                /* AWB blocks waiting for their statistic */
+    char *dst, *inter;       /* the row pair to store next: the strip's first pixel */
+    float qs[3];             /* chroma: this lane's 4x4 block sums */
+
+    CRAW_DEV WalkOut(const CRAWKDevelop &k_, const CRAWKDevelopIO &io_, S &s_, int nout_, int qx_, int qy_)
+        : k(k_), io(io_), s(s_), lane(threadIdx.x & 31), nout(nout_), qx(qx_), qy(qy_), held(0)
+    {
+        mine = lane >= A && lane < A + nout;
+        dst = (char *)io.dst + (size_t)(2 * qy) * io.dst_pitch + (size_t)(2 * qx) * bytes(fmt());
+        inter = (char *)io.inter + (size_t)(2 * qy) * io.inter_pitch +
+                (size_t)(2 * qx) * (k.fp16 ? 8 : 16);
+        qs[0] = qs[1] = qs[2] = 0.0f;
+    }
+    CRAW_DEV static int bytes(int f) { return f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16); }
+    CRAW_DEV int fmt() const { return MORE ? io.dst_fmt : FMT; }
+
+    /* The colour stage of the quad's four pixels (craw_color, the gamut
+     * compression a channel at a time for all four, where any lane's pixel
+     * needs it: branch-free, so the four chains interleave). The test for
+     * it needs no division: a distance clearly below its threshold, beyond
+     * any rounding of the compression's own reciprocal, leaves the channel
+     * alone. */
+    CRAW_DEV void colour(const float v[2][2][3], float o[2][2][3]) const
+    {
+        const CRAWKColor &c = k.color;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float *in = v[i >> 1][i & 1];
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+                o[i >> 1][i & 1][r] = c.m[r][0] * in[0] + c.m[r][1] * in[1] + c.m[r][2] * in[2];
+        }
+        if (MORE ? (c.flags & CRAW_K_COLOR_RGC) != 0 : RGC) {
+            float ach[4];
+            bool need[3] = { false, false, false };
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float *p = o[i >> 1][i & 1];
+                ach[i] = fmaxf(p[0], fmaxf(p[1], p[2]));
+                const float mag = fabsf(ach[i]) * (1.0f - 1e-6f);
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+                    need[r] |= !(ach[i] - p[r] < c.gc_thr[r] * mag);
+            }
+            if (__any_sync(0xffffffffu, mine && (need[0] || need[1] || need[2]))) {
+                float inv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    inv[i] = craw_rcp(fabsf(ach[i]));
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    if (!__any_sync(0xffffffffu, mine && need[r]))
+                        continue;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        float &x = o[i >> 1][i & 1][r];
+                        const float y = craw_gamut_channel(c, r, ach[i], fabsf(ach[i]), inv[i], x);
+                        x = ach[i] == 0.0f ? x : y;
+                    }
+                }
+            }
+        }
+        if (c.flags & CRAW_K_COLOR_CLAMP) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+                    o[i >> 1][i & 1][r] = fmaxf(o[i >> 1][i & 1][r], 0.0f);
+        }
+    }
+
+    /* A row pair of an RGB image of layout `f` from `at` (the strip's first
+     * pixel of it), two pixels a lane and row: v[row][pixel][channel]. */
+    CRAW_DEV void store(char *at, size_t pitch, int f, int r, const float v[2][2][3])
+    {
+        const bool ok = craw_in_bounds(qx >= 0 && 2 * (qx + nout) <= k.width && 2 * (qy + r) >= 0 &&
+                                       2 * (qy + r) + 1 < k.height, io.err);
+        if (f == CRAW_K_OUT_RGB32F) {
+            if (mine && ok) {
+#pragma unroll
+                for (int b = 0; b < 2; b++) {
+                    float2 *p = reinterpret_cast<float2 *>(at + b * pitch) + 3 * (lane - A);
+                    p[0] = make_float2(v[b][0][0], v[b][0][1]);
+                    p[1] = make_float2(v[b][0][2], v[b][1][0]);
+                    p[2] = make_float2(v[b][1][1], v[b][1][2]);
+                }
+            }
+        } else if (mine && ok) {
+            at += (lane - A) * (f == CRAW_K_OUT_RGBA16F ? 16 : 32);
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                const float *p = v[b][0], *q = v[b][1];
+                char *d = at + b * pitch;
+                if (f == CRAW_K_OUT_RGBA16F) {
+                    const __half2 h0 = __floats2half2_rn(p[0], p[1]), h1 = __floats2half2_rn(p[2], 1.0f);
+                    const __half2 h2 = __floats2half2_rn(q[0], q[1]), h3 = __floats2half2_rn(q[2], 1.0f);
+                    uint4 u;
+                    u.x = *reinterpret_cast<const uint32_t *>(&h0);
+                    u.y = *reinterpret_cast<const uint32_t *>(&h1);
+                    u.z = *reinterpret_cast<const uint32_t *>(&h2);
+                    u.w = *reinterpret_cast<const uint32_t *>(&h3);
+                    *reinterpret_cast<uint4 *>(d) = u;
+                } else if (!((uintptr_t)d & 31)) {
+                    walk_store8(reinterpret_cast<float *>(d), p[0], p[1], p[2], 1.0f, q[0], q[1], q[2], 1.0f);
+                } else {
+                    reinterpret_cast<float4 *>(d)[0] = make_float4(p[0], p[1], p[2], 1.0f);
+                    reinterpret_cast<float4 *>(d)[1] = make_float4(q[0], q[1], q[2], 1.0f);
+                }
+            }
+        }
+    }
+
+    /* 4x4 block means of (R - G, B - G, G), added row by row over the
+     * pixels inside the frame (reference lib/ref/ref_chroma.c:49-74): the
+     * left lane of a block's two adds its two pixels of a row to the
+     * block's sums, the right lane its two after them. */
+    CRAW_DEV void quarter(int r, bool last, const float v[2][2][3])
+    {
+        const bool right = (lane - A) & 1, in = mine;
+        if (!((qy + r) & 1))
+            qs[0] = qs[1] = qs[2] = 0.0f;
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float d[2];
+#pragma unroll
+                for (int p = 0; p < 2; p++)
+                    d[p] = c == 2 ? v[b][p][1] : __fsub_rn(v[b][p][2 * c], v[b][p][1]);
+                float t = __fadd_rn(__fadd_rn(qs[c], d[0]), d[1]);
+                const float u = __fadd_rn(__fadd_rn(walk_left(t), d[0]), d[1]);
+                if (right && in)
+                    t = u;
+                const float back = walk_right(t);
+                /* The left lane goes on from the right one's sum where the
+                 * frame has that column. */
+                qs[c] = !right && lane + 1 < A + nout ? back : t;
+            }
+        if (!(((qy + r) & 1) || last) || right || !in)
+            return;
+        const int bx = (qx + lane - A) >> 1, by = (qy + r) >> 1;
+        const int nx = min(4, k.width - 4 * bx), ny = min(4, k.height - 4 * by);
+        const float n = (float)(nx * ny);
+        if (craw_in_bounds(bx >= 0 && bx < (k.width + 3) / 4 && by >= 0 && by < (k.height + 3) / 4, io.err))
+            craw_store_rgba(io.quarter, io.quarter_pitch, bx, by, k.fp16, __fdiv_rn(qs[0], n), __fdiv_rn(qs[1], n),
+                            __fdiv_rn(qs[2], n));
+    }
+
+    /* The AWB block sums of the eight (at the frame's bottom fewer) rows
+     * staged so far, row by row (reference lib/awb.c:239-253): lane
+     * c NB + b sums channel c of block b. The statistic of a block is over
+     * a hundred instructions, so blocks are held until a warp's worth has
+     * gathered (or the segment ends). */
+    CRAW_DEV void awb_rows(int r, int rows, bool last)
+    {
+        __syncwarp();
+        const int b = lane % S::NB, c = lane / S::NB;
+        const int w = min(8, 2 * nout - 8 * b);
+        const bool sums = c < 3 && w > 0;
+        if (sums) {
+            float t = 0.0f;
+            if (w == 8) {
+#pragma unroll 2
+                for (int j = 0; j < rows; j++) {
+                    const float *p = &s.a[j][c][S::col(8 * b)];
+                    const float4 q0 = *reinterpret_cast<const float4 *>(p), q1 = *reinterpret_cast<const float4 *>(p + 4);
+                    t = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(t, q0.x), q0.y), q0.z), q0.w);
+                    t = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(t, q1.x), q1.y), q1.z), q1.w);
+                }
+            } else {
+                for (int j = 0; j < rows; j++)
+                    for (int i = 0; i < w; i++)
+                        t = __fadd_rn(t, s.a[j][c][S::col(8 * b) + i]);
+            }
+            s.sum[held + b][c] = t;
+            if (c == 0) {
+                s.cnt[held + b] = (float)(w * rows);
+                s.where[held + b] = (qy + r) / 4 * ((k.width + 7) / 8) + qx / 4 + b;
+            }
+        }
+        held += (2 * nout + 7) / 8;
+        __syncwarp();
+        if (!last && held + S::NB <= S::HOLD * S::NB)
+            return;
+        if (lane < held) {
+            const float n = s.cnt[lane];
+            const int ri = s.where[lane];
+            if (craw_in_bounds(ri >= 0 && (uint32_t)ri < craw_awb_blocks(k.width, k.height), io.err))
+                io.awb.rec[ri] = craw_awb_block(__fdiv_rn(s.sum[lane][0], n), __fdiv_rn(s.sum[lane][1], n),
+                                                __fdiv_rn(s.sum[lane][2], n), k.awb_wb, io.awb.deferred,
+                                                io.awb.nb_deferred, craw_awb_blocks(k.width, k.height));
+        }
+        held = 0;
+        __syncwarp();
+    }
+
+    /* Quad row r of the segment (`last`: its last), v[row][pixel][channel]
+     * the camera RGB of the lane's quad. The whole warp calls this, for the
+     * rows of the segment in order. */
+    CRAW_DEV void quad_row(int r, bool last, float v[2][2][3])
+    {
+        if constexpr (MORE) {
+            if (k.fp16) {
+#pragma unroll
+                for (int b = 0; b < 2; b++)
+#pragma unroll
+                    for (int p = 0; p < 2; p++)
+#pragma unroll
+                        for (int c = 0; c < 3; c++)
+                            v[b][p][c] = craw_round_half(v[b][p][c]);
+            }
+            if (io.inter) {
+                store(inter, io.inter_pitch, k.fp16 ? CRAW_K_OUT_RGBA16F : CRAW_K_OUT_RGBA32F, r, v);
+                inter += 2 * io.inter_pitch;
+            }
+            if (io.quarter) {
+                quarter(r, last, v);
+                return;
+            }
+        }
+        if (io.awb.rec && mine) {
+            float *a = &s.a[2 * (r & 3)][0][S::col(2 * (lane - A))];
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+                    *reinterpret_cast<float2 *>(a + (3 * b + c) * S::PITCH) = make_float2(v[b][0][c], v[b][1][c]);
+        }
+        if (!MORE || io.dst) {
+            float o[2][2][3];
+            colour(v, o);
+            store(dst, io.dst_pitch, fmt(), r, o);
+            dst += 2 * io.dst_pitch;
+        }
+        if (io.awb.rec && ((r & 3) == 3 || last))
+            awb_rows(r, 2 * (r & 3) + 2, last);
+    }
+};
+
+/* One raw row pair of samples (one row of a quad) prepped; row parity `py`. */
+CRAW_DEV float2 walk_prep(const CRAWKDevelop &k, const CRAWKDevelopIO &io, uint32_t raw, int py)
+{
+    if (io.src_f16)   /* rebuilt highlights: fp16, already prepped */
+        return __half22float2(*reinterpret_cast<const __half2 *>(&raw));
+    return make_float2(craw_prep(k, (uint16_t)(raw & 0xffff), 2 * py),
+                       craw_prep(k, (uint16_t)(raw >> 16), 2 * py + 1));
+}
+
+/* ----------------------------------------------------------------- RCD */
+
+/* The RCD of the frame's interior (reference lib/ref/ref_debayer.c:204-395)
+ * by walking warps, evaluated by the rq_* helpers as the tiles evaluate it,
+ * so both give the same bits. Step s forms
+ *   D, L of quad row s       (the four discriminations of the quad's
+ *                            pixels, the low pass at R and B),
+ *   W, G of row s - 1        (the weights from the 3x3 sums of D kept down
+ *                            the column, green at R and B) and the colour
+ *                            differences KR = R - G, KB = B - G there,
+ *   C of row s - 2           (the missing colour at R and B) and its
+ *                            differences JR = B - G at R, JB = R - G at B,
+ *   the pixels of row s - 3.
+ * Every neighbour's term is one of the differences, so each is formed once
+ * and crosses the lanes once. Interior strips only: every sample read that
+ * a result depends on, down to six pixels outside the strip's output, lies
+ * inside the frame; reads past the frame's edge are clamped to it and only
+ * feed values nothing reads. */
+constexpr int RW_NQ = 24, RW_A = 4;
+
+struct RcdWalk {
+    float v[6][6];                    /* pixel rows 2s-2 .. 2s+3, columns X-2 .. X+3 (X: the lane's R) */
+    float q2[4], q3[4];               /* the quads of rows s-2, s-3: R, Gr, Gb, B */
+    float2 l1, l2;                    /* L of rows s-1, s-2 */
+    float4 h[3][2];                   /* 3-wide row sums of D, pixel rows 2s-3 .. 2s-1, two pixels */
+    float2 wg2, wg3;                  /* weights at (Gr, Gb), rows s-2, s-3 */
+    float2 wp2;                       /* diagonal weights at (R, B), row s-2 */
+    float2 g2, g3;                    /* green at (R, B), rows s-2, s-3 */
+    float kr2, kr3, krr2, krr3;       /* KR of rows s-2, s-3; the right neighbour's */
+    float kb2, kb3, kb4, kbl2, kbl3;  /* KB of rows s-2 .. s-4; the left neighbour's */
+    float jr3, jrr3, jb3, jb4, jbl3;  /* JR of row s-3, the right's; JB of rows s-3, s-4, the left's */
+    float2 c3;                        /* C of row s-3 */
+
+    /* The two new pixel rows, 2s+2 and 2s+3. */
+    CRAW_DEV void rows(float2 a, float2 b)
+    {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float2 t = i ? b : a;
+            v[4 + i][0] = walk_left(t.x);
+            v[4 + i][1] = walk_left(t.y);
+            v[4 + i][2] = t.x;
+            v[4 + i][3] = t.y;
+            v[4 + i][4] = walk_right(t.x);
+            v[4 + i][5] = walk_right(t.y);
+        }
+    }
+
+    /* One step; o: the pixels of row s - 3. */
+    CRAW_DEV void step(float o[2][2][3])
+    {
+        /* D, L of row s. */
+        float2 l0;
+        float lo[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int y = 2 + e, x = 2 + e;
+            lo[e] = rq_lowpass(v[y][x], v[y - 1][x], v[y + 1][x], v[y][x - 1], v[y][x + 1], v[y - 1][x - 1],
+                               v[y - 1][x + 1], v[y + 1][x - 1], v[y + 1][x + 1]);
+        }
+        l0 = make_float2(lo[0], lo[1]);
+        float4 hn[2][2];
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            float4 d[2];
+#pragma unroll
+            for (int a = 0; a < 2; a++) {
+                auto win = [&](int r, int c) { return v[b + r][a + c]; };
+                d[a] = rq_disc4(win);
+            }
+            const float4 mid = rq_add4(d[0], d[1]);
+            const float4 dl = make_float4(walk_left(d[1].x), walk_left(d[1].y), walk_left(d[1].z), walk_left(d[1].w));
+            const float4 dr = make_float4(walk_right(d[0].x), walk_right(d[0].y), walk_right(d[0].z),
+                                          walk_right(d[0].w));
+            hn[b][0] = rq_add4(dl, mid);
+            hn[b][1] = rq_add4(mid, dr);
+        }
+        /* W, G of row s - 1: the 3x3 sums of its first pixel row are h[0..2],
+         * of its second h[1], h[2], hn[0]. */
+        float4 sum[2][2];
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+            const float4 mid = rq_add4(h[1][a], h[2][a]);
+            sum[0][a] = rq_add4(h[0][a], mid);
+            sum[1][a] = rq_add4(hn[0][a], mid);
+        }
+        const float2 wp1 = make_float2(rq_wp(sum[0][0]), rq_wp(sum[1][1]));
+        const float2 wg1 = make_float2(rq_wv(sum[0][1]), rq_wv(sum[1][0]));
+        const float2 ll = make_float2(walk_left(l1.x), walk_left(l1.y));
+        const float2 lr = make_float2(walk_right(l1.x), walk_right(l1.y));
+        const float2 g1 = make_float2(
+            rq_green(rq_wv(sum[0][0]), l1.x, q2[2], l2.x, v[1][2], l0.x, v[0][1], ll.x, v[0][3], lr.x),
+            rq_green(rq_wv(sum[1][1]), l1.y, v[0][3], l2.y, v[2][3], l0.y, v[1][2], ll.y, v[1][4], lr.y));
+        const float kr1 = __fsub_rn(v[0][2], g1.x), kb1 = __fsub_rn(v[1][3], g1.y);
+        const float krr1 = walk_right(kr1), kbl1 = walk_left(kb1);
+        /* C of row s - 2. */
+        const float2 c2 = make_float2(rq_cross(wp2.x, g2.x, kbl2, kb3, kbl3, kb2),
+                                      rq_cross(wp2.y, g2.y, kr1, krr2, kr2, krr1));
+        const float jr2 = __fsub_rn(c2.x, g2.x), jb2 = __fsub_rn(c2.y, g2.y);
+        const float jrr2 = walk_right(jr2), jbl2 = walk_left(jb2);
+        /* The pixels of row s - 3. */
+        o[0][0][0] = q3[0]; o[0][0][1] = g3.x;  o[0][0][2] = c3.x;
+        o[0][1][1] = q3[1];
+        rq_green_site(wg3.x, q3[1], kr3, krr3, jb4, jb3, kb4, kb3, jr3, jrr3, o[0][1][0], o[0][1][2]);
+        o[1][0][1] = q3[2];
+        rq_green_site(wg3.y, q3[2], kbl3, kb3, jr3, jr2, kr3, kr2, jbl3, jb3, o[1][0][2], o[1][0][0]);
+        o[1][1][0] = c3.y;  o[1][1][1] = g3.y;  o[1][1][2] = q3[3];
+        /* A row on. */
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            q3[i] = q2[i];
+        q2[0] = v[0][2]; q2[1] = v[0][3]; q2[2] = v[1][2]; q2[3] = v[1][3];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 6; c++)
+                v[r][c] = v[r + 2][c];
+        l2 = l1; l1 = l0;
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+            h[0][a] = h[2][a];
+            h[1][a] = hn[0][a];
+            h[2][a] = hn[1][a];
+        }
+        wg3 = wg2; wg2 = wg1;
+        wp2 = wp1;
+        g3 = g2; g2 = g1;
+        kr3 = kr2; kr2 = kr1; krr3 = krr2; krr2 = krr1;
+        kb4 = kb3; kb3 = kb2; kb2 = kb1; kbl3 = kbl2; kbl2 = kbl1;
+        jb4 = jb3; jb3 = jb2; jbl3 = jbl2; jr3 = jr2; jrr3 = jrr2;
+        c3 = c2;
+    }
+};
+
+/* The strip of warp `wid` of the grid. */
+template <int FMT, bool RGC, bool MORE>
+CRAW_DEV void rcd_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const WalkGrid &g, int wid,
+                       WalkSmem<RW_NQ> &smem)
+{
+    const int sx = wid % g.nx, sy = wid / g.nx;
+    if (sy * g.seg >= g.nqy)
+        return;
+    const int nrows = min(g.seg, g.nqy - sy * g.seg);
+    WalkOut<RW_NQ, RW_A, FMT, RGC, MORE> out(k, io, smem, min(RW_NQ, g.nqx - sx * RW_NQ), g.qx0 + sx * RW_NQ,
+                                             g.qy0 + sy * g.seg);
+    const int q = min(out.qx - RW_A + out.lane, k.width / 2 - 1), y0 = 2 * out.qy;
+    const char *src = (const char *)io.src + 4 * (size_t)q;
+    auto fetch = [&](int yr) {
+        const int y = min(y0 + yr, k.height - 1);
+        if (!craw_in_bounds(q >= 0 && 2 * q + 1 < k.width && y >= 0, io.err))
+            return 0u;
+        return walk_ld(src + (size_t)y * io.src_pitch);
+    };
+    RcdWalk t;
+    memset(&t, 0, sizeof(t));
+    /* Steps -3 .. nrows + 2, two a round (the first fills the pipeline
+     * only); the rows of step -3 are -4 and -3, and four rows come before. */
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        t.rows(walk_prep(k, io, fetch(-8 + 2 * i), 0), walk_prep(k, io, fetch(-7 + 2 * i), 1));
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            t.v[2 * i][c] = t.v[4][c];
+            t.v[2 * i + 1][c] = t.v[5][c];
+        }
+    }
+    uint32_t raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        raw[i] = fetch(-4 + i);
+#pragma unroll 1
+    for (int s = -3; s <= nrows + 2; s += 2) {
+        uint32_t next[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            next[i] = fetch(2 * s + 6 + i);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            float o[2][2][3];
+            t.rows(walk_prep(k, io, raw[2 * u], 0), walk_prep(k, io, raw[2 * u + 1], 1));
+            t.step(o);
+            const int r = s + u - 3;
+            if (r >= 0 && r < nrows)
+                out.quad_row(r, r == nrows - 1, o);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            raw[i] = next[i];
+    }
+}
+
+} // namespace craw_dev
