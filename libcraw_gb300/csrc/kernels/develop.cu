@@ -157,22 +157,20 @@ k_develop_rcd_border(const CRAWKDevelop k, const CRAWKDevelopIO io, const QuadGr
     pixel_tile<kRcd, BTW, BTH, 256>(k, io, x0, y0, smem);
 }
 
-/* Eight CTAs an SM (full occupancy at 256 threads): the bilinear and MHC
- * tiles are bound by HBM and need every warp in flight. */
-template <int METHOD, int TW, int TH, int NT>
-__global__ void __launch_bounds__(NT, 2048 / NT)
-k_develop(const CRAWKDevelop k, const CRAWKDevelopIO io)
+/* Every bilinear and MHC frame: CTAs an SM (5 of 96 registers for MHC and 6
+ * of 80 for bilinear, a few spilled, run 7 % faster at 5760x3240 than 4 and
+ * 5 without a spill). */
+template <int METHOD, int EPI> constexpr int linear_ctas()
 {
-    extern __shared__ __align__(16) float smem[];
-    pixel_tile<METHOD, TW, TH, NT>(k, io, blockIdx.x * TW, blockIdx.y * TH, smem);
+    return EPI == LW_ANY ? 3 : (METHOD == kMhc ? 5 : 6);
 }
 
-template <int METHOD, int TW, int TH, int NT>
-int launch(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+template <int METHOD, int EPI>
+__global__ void __launch_bounds__(WALK_NT, (linear_ctas<METHOD, EPI>()))
+k_develop_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
 {
-    dim3 grid((k->width + TW - 1) / TW, (k->height + TH - 1) / TH);
-    k_develop<METHOD, TW, TH, NT><<<grid, NT, PixelSmem<METHOD, TW, TH, NT>::floats * sizeof(float), s>>>(*k, *io);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    LinearWalk<METHOD, EPI> t(k, io);
+    t.run(g, blockIdx.x * WALK_WARPS + (threadIdx.x >> 5));
 }
 
 /* The current device's SM count, kept per device ordinal below 64 (152,
@@ -190,6 +188,47 @@ int craw_sm_count()
     if (dev >= 0 && dev < 64)
         known[dev].store(sms, std::memory_order_relaxed);
     return sms;
+}
+
+/* Segments of one wave of `ctas` CTAs an SM: as tall as that allows (a
+ * segment reads, and for the RCD computes, its first rows' surroundings
+ * again), a multiple of 4 quad rows, at least `least`; g.nx strips are
+ * set. Returns the CTAs. */
+unsigned walk_segments(WalkGrid &g, int ctas, int least)
+{
+    const int room = craw_sm_count() * ctas * WALK_WARPS / g.nx;
+    const int nseg = room > 1 ? room : 1;
+    g.seg = 4 * (((g.nqy + 3) / 4 + nseg - 1) / nseg);
+    g.seg = g.seg < least ? least : g.seg;
+    const int warps = g.nx * ((g.nqy + g.seg - 1) / g.seg);
+    return (unsigned)((warps + WALK_WARPS - 1) / WALK_WARPS);
+}
+
+template <int METHOD, int EPI>
+int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+{
+    WalkGrid g;
+    g.qx0 = g.qy0 = 0;
+    g.nqx = k->width / 2;
+    g.nqy = k->height / 2;
+    g.nx = (k->width + LW_P * LW_N - 1) / (LW_P * LW_N);
+    const unsigned grid = walk_segments(g, linear_ctas<METHOD, EPI>(), 4);
+    k_develop_walk<METHOD, EPI><<<grid, WALK_NT, 0, s>>>(*k, *io, g);
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+template <int METHOD>
+int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+{
+    if (io->quarter && io->inter)
+        return launch_linear<METHOD, LW_CHROMA>(k, io, s);
+    if (io->inter || !io->dst)
+        return launch_linear<METHOD, LW_ANY>(k, io, s);
+    switch (io->dst_fmt) {
+    case CRAW_K_OUT_RGBA16F: return launch_linear<METHOD, CRAW_K_OUT_RGBA16F>(k, io, s);
+    case CRAW_K_OUT_RGB32F:  return launch_linear<METHOD, CRAW_K_OUT_RGB32F>(k, io, s);
+    default:                 return launch_linear<METHOD, CRAW_K_OUT_RGBA32F>(k, io, s);
+    }
 }
 
 /* The RCD kernels' shared-memory sizes, set once per device; this also
@@ -228,22 +267,15 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
     QuadGrid g;
     g.init(k->width, k->height);
     if (g.interior_x() > 0 && g.interior_y() > 0 && craw_k_rcd_strips) {
-        /* The interior tiles' region by walking warps, in segments of one
-         * wave of the device (a segment repeats the passes of six quad rows
-         * to start, so it is as tall as one wave allows), at least 8 quad
-         * rows. */
+        /* The interior tiles' region by walking warps. */
         WalkGrid w;
         w.qx0 = g.c_lo * (QTW / 2);
         w.nqx = g.interior_x() * (QTW / 2);
         w.qy0 = g.r_lo * (QTH / 2);
         w.nqy = g.interior_y() * (QTH / 2);
         w.nx = (w.nqx + RW_NQ - 1) / RW_NQ;
-        const int room = craw_sm_count() * WALK_CTAS * WALK_WARPS / w.nx;
-        const int nseg = room > 1 ? room : 1;
-        w.seg = 4 * ((w.nqy / 4 + nseg - 1) / nseg);
-        w.seg = w.seg < 8 ? 8 : w.seg;
-        const int warps = w.nx * ((w.nqy + w.seg - 1) / w.seg);
-        walk_rcd(k, io)<<<(warps + WALK_WARPS - 1) / WALK_WARPS, WALK_NT, 0, s>>>(*k, *io, w);
+        const unsigned ctas = walk_segments(w, WALK_CTAS, 8);
+        walk_rcd(k, io)<<<ctas, WALK_NT, 0, s>>>(*k, *io, w);
         if (cudaGetLastError() != cudaSuccess)
             return -5;
     } else if (g.interior_x() > 0 && g.interior_y() > 0) {
@@ -299,8 +331,8 @@ extern "C" int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, i
         return -5;
     (void)shape;
     switch (k->method) {
-    case kBilinear: return launch<kBilinear, 64, 16, 256>(k, io, s);
-    case kMhc:      return launch<kMhc, 64, 16, 256>(k, io, s);
+    case kBilinear: return launch_linear<kBilinear>(k, io, s);
+    case kMhc:      return launch_linear<kMhc>(k, io, s);
     case kRcd:      return launch_rcd(k, io, s);
     default:        return -22;
     }

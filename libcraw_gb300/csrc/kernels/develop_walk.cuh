@@ -64,6 +64,62 @@ CRAW_DEV void walk_store8(float *p, float a, float b, float c, float d, float e,
                  :: "l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e), "f"(f), "f"(g), "f"(h) : "memory");
 }
 
+/* The colour stage of four pixels of a lane (craw_color; RGC: with the
+ * gamut compression, without it, or -1: by its flag), the gamut compression
+ * a channel at a time for all four, where any lane's pixel needs it:
+ * branch-free, so the four chains interleave. The test for it needs no
+ * division: a distance clearly below its threshold, beyond any rounding of
+ * the compression's own reciprocal, leaves the channel alone. (A pixel at a
+ * time with a branch a channel: 5760x3240 AP1 284 us a frame, against 197
+ * this way and 174 without the compression.) The whole warp calls this;
+ * `mine`: the lane's pixels count. */
+template <int RGC>
+CRAW_DEV void walk_colour(const CRAWKColor &c, bool mine, float o[4][3])
+{
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float in[3] = { o[i][0], o[i][1], o[i][2] };
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            o[i][r] = c.m[r][0] * in[0] + c.m[r][1] * in[1] + c.m[r][2] * in[2];
+    }
+    if (RGC < 0 ? (c.flags & CRAW_K_COLOR_RGC) != 0 : RGC) {
+        float ach[4];
+        bool need[3] = { false, false, false };
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            ach[i] = fmaxf(o[i][0], fmaxf(o[i][1], o[i][2]));
+            const float mag = fabsf(ach[i]) * (1.0f - 1e-6f);
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+                need[r] |= !(ach[i] - o[i][r] < c.gc_thr[r] * mag);
+        }
+        if (__any_sync(0xffffffffu, mine && (need[0] || need[1] || need[2]))) {
+            float inv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                inv[i] = craw_rcp(fabsf(ach[i]));
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                if (!__any_sync(0xffffffffu, mine && need[r]))
+                    continue;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float y = craw_gamut_channel(c, r, ach[i], fabsf(ach[i]), inv[i], o[i][r]);
+                    o[i][r] = ach[i] == 0.0f ? o[i][r] : y;
+                }
+            }
+        }
+    }
+    if (c.flags & CRAW_K_COLOR_CLAMP) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+                o[i][r] = fmaxf(o[i][r], 0.0f);
+    }
+}
+
 /* Shared memory of one warp: the camera RGB of the AWB block row in
  * progress (eight pixel rows, planar a row: 4 floats of padding after 32
  * spread the blocks a fold reads over the banks), and the sums of the
@@ -109,59 +165,20 @@ struct WalkOut {
     CRAW_DEV static int bytes(int f) { return f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16); }
     CRAW_DEV int fmt() const { return MORE ? io.dst_fmt : FMT; }
 
-    /* The colour stage of the quad's four pixels (craw_color, the gamut
-     * compression a channel at a time for all four, where any lane's pixel
-     * needs it: branch-free, so the four chains interleave). The test for
-     * it needs no division: a distance clearly below its threshold, beyond
-     * any rounding of the compression's own reciprocal, leaves the channel
-     * alone. */
     CRAW_DEV void colour(const float v[2][2][3], float o[2][2][3]) const
     {
-        const CRAWKColor &c = k.color;
+        float q[4][3];
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const float *in = v[i >> 1][i & 1];
+        for (int i = 0; i < 4; i++)
 #pragma unroll
-            for (int r = 0; r < 3; r++)
-                o[i >> 1][i & 1][r] = c.m[r][0] * in[0] + c.m[r][1] * in[1] + c.m[r][2] * in[2];
-        }
-        if (MORE ? (c.flags & CRAW_K_COLOR_RGC) != 0 : RGC) {
-            float ach[4];
-            bool need[3] = { false, false, false };
+            for (int c = 0; c < 3; c++)
+                q[i][c] = v[i >> 1][i & 1][c];
+        walk_colour<MORE ? -1 : RGC>(k.color, mine, q);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float *p = o[i >> 1][i & 1];
-                ach[i] = fmaxf(p[0], fmaxf(p[1], p[2]));
-                const float mag = fabsf(ach[i]) * (1.0f - 1e-6f);
+        for (int i = 0; i < 4; i++)
 #pragma unroll
-                for (int r = 0; r < 3; r++)
-                    need[r] |= !(ach[i] - p[r] < c.gc_thr[r] * mag);
-            }
-            if (__any_sync(0xffffffffu, mine && (need[0] || need[1] || need[2]))) {
-                float inv[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    inv[i] = craw_rcp(fabsf(ach[i]));
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    if (!__any_sync(0xffffffffu, mine && need[r]))
-                        continue;
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        float &x = o[i >> 1][i & 1][r];
-                        const float y = craw_gamut_channel(c, r, ach[i], fabsf(ach[i]), inv[i], x);
-                        x = ach[i] == 0.0f ? x : y;
-                    }
-                }
-            }
-        }
-        if (c.flags & CRAW_K_COLOR_CLAMP) {
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-                    o[i >> 1][i & 1][r] = fmaxf(o[i >> 1][i & 1][r], 0.0f);
-        }
+            for (int c = 0; c < 3; c++)
+                o[i >> 1][i & 1][c] = q[i][c];
     }
 
     /* A row pair of an RGB image of layout `f` from `at` (the strip's first
@@ -497,20 +514,24 @@ CRAW_DEV void rcd_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const Wa
     RcdWalk t;
     memset(&t, 0, sizeof(t));
     /* Steps -3 .. nrows + 2, two a round (the first fills the pipeline
-     * only); the rows of step -3 are -4 and -3, and four rows come before. */
+     * only); the rows of step -3 are -4 and -3, and four rows come before.
+     * Every load is issued before the first is used. */
+    uint32_t first[4], raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        first[i] = fetch(-8 + i);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        raw[i] = fetch(-4 + i);
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-        t.rows(walk_prep(k, io, fetch(-8 + 2 * i), 0), walk_prep(k, io, fetch(-7 + 2 * i), 1));
+        t.rows(walk_prep(k, io, first[2 * i], 0), walk_prep(k, io, first[2 * i + 1], 1));
 #pragma unroll
         for (int c = 0; c < 6; c++) {
             t.v[2 * i][c] = t.v[4][c];
             t.v[2 * i + 1][c] = t.v[5][c];
         }
     }
-    uint32_t raw[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        raw[i] = fetch(-4 + i);
 #pragma unroll 1
     for (int s = -3; s <= nrows + 2; s += 2) {
         uint32_t next[4];
@@ -531,5 +552,339 @@ CRAW_DEV void rcd_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const Wa
             raw[i] = next[i];
     }
 }
+
+/* ------------------------------------------------------ bilinear, MHC */
+
+/* The bilinear and MHC debayers of the whole frame by walking warps whose
+ * lanes own four pixel columns each: one 4x4 block of the chroma path, half
+ * an AWB block. A warp has LW_N output lanes (whole AWB blocks) and an apron
+ * lane on either side. Outside the frame a sample is the one its position
+ * mirrors to: the rows turn back at the frame's last row, and the lanes at
+ * its left and right edge take the mirrored columns from their own.
+ *
+ * Bound: instruction issue for half-float output, DRAM and its latency for
+ * the float layouts. At 5760x3240 (a frame without denoise, AWB on) MHC
+ * takes 100 us with RGBA32F and 90 with RGBA16F out, against 155 by 64x16
+ * tiles of shared memory with a pixel a thread. Two columns a lane (with the
+ * block sums through shared memory) spend a third of their instructions on
+ * addresses, constants and branches: 104 and 97 us; eight take too many
+ * registers and too long a body for the instruction cache: 135 and 115. */
+constexpr int LW_N = 30, LW_P = 4;
+
+/* The four samples of a row from `p`, in the frame (8-byte aligned). */
+CRAW_DEV uint2 walk_ld4(const char *p)
+{
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+
+/* What a frame's epilogue is, fixed per kernel so that a row's code stays
+ * small: the colour stage to one output layout (a CRAW_K_OUT_*); the chroma
+ * path's (intermediate and block means); or any of it by tests (a kept
+ * intermediate). */
+constexpr int LW_CHROMA = 3, LW_ANY = 4;
+
+template <int METHOD, int EPI>
+struct LinearWalk {
+    static constexpr bool CHROMA = EPI == LW_CHROMA, ANY = EPI == LW_ANY;
+    static constexpr int RAD = METHOD == kMhc ? 2 : 1;   /* pixels around a quad that its debayer reads */
+    static constexpr int WR = 2 + 2 * RAD, WC = LW_P + 2 * RAD;
+    const CRAWKDevelop &k;
+    const CRAWKDevelopIO &io;
+    float v[WR][WC];         /* pixel rows 2r - RAD .. 2r + 1 + RAD, columns x0 - RAD .. x0 + 3 + RAD */
+    int x0, nv;              /* the lane's first column; its columns inside the frame (output lanes) */
+    bool edge;               /* the warp reaches the frame's left or right edge */
+    bool inside, partial;    /* the lane's four columns are in the frame; its first two only */
+    bool mine, right;        /* an output lane; the second of its AWB block */
+    float as[3], hs[3];      /* the AWB block's sums so far; the block's above, waiting */
+    int held;                /* whether hs waits: then its row of blocks + 1 */
+    float qs[3];             /* chroma: the sums of the 4x4 block so far */
+    char *dst, *inter;       /* the lane's pixels in the row to store next */
+
+    CRAW_DEV LinearWalk(const CRAWKDevelop &k_, const CRAWKDevelopIO &io_) : k(k_), io(io_) {}
+
+    CRAW_DEV float at(int x, int y) const { return v[y][x]; }
+
+    /* A row's four samples; of a lane that hangs over the right edge by two,
+     * its two; of a lane outside the frame, none. (No lane combines what it
+     * loads before it is used, a round later.) */
+    CRAW_DEV uint2 load(const char *row) const
+    {
+        uint2 u = make_uint2(0u, 0u);
+        if (!craw_in_bounds(row >= (const char *)io.src &&
+                            row <= (const char *)io.src + (size_t)(k.height - 1) * io.src_pitch, io.err))
+            return u;
+        if (inside)
+            u = walk_ld4(row + 2 * (size_t)x0);
+        else if (partial)
+            u.x = walk_ld(row + 2 * (size_t)x0);
+        return u;
+    }
+
+    /* A raw row of parity py into window row `r`. The columns outside the
+     * frame mirror into the lane's own or its left neighbour's. */
+    CRAW_DEV void put(int r, uint2 raw, int py)
+    {
+        const float2 a = walk_prep(k, io, raw.x, py), b = walk_prep(k, io, raw.y, py);
+        float p[LW_P] = { a.x, a.y, b.x, b.y }, l[RAD], q[RAD];   /* q: to the right */
+#pragma unroll
+        for (int i = 0; i < RAD; i++) {
+            l[i] = walk_left(p[LW_P - RAD + i]);
+            q[i] = walk_right(p[i]);
+        }
+        if (edge) {
+            if (x0 == 0)
+#pragma unroll
+                for (int i = 0; i < RAD; i++)
+                    l[i] = p[RAD - i];                   /* column -RAD + i */
+            if (partial) {
+                p[2] = p[0];                             /* column w: w - 2 */
+                p[3] = l[RAD - 1];                       /* column w + 1: w - 3 */
+            }
+            if (x0 + LW_P == k.width)
+#pragma unroll
+                for (int i = 0; i < RAD; i++)
+                    q[i] = p[LW_P - 2 - i];              /* column w + i: w - 2 - i */
+        }
+#pragma unroll
+        for (int i = 0; i < RAD; i++) {
+            v[r][i] = l[i];
+            v[r][RAD + LW_P + i] = q[i];
+        }
+#pragma unroll
+        for (int i = 0; i < LW_P; i++)
+            v[r][RAD + i] = p[i];
+    }
+
+    /* The lane's pixels of a row of an RGB image of layout f at `d`. */
+    CRAW_DEV void store(char *d, int f, const float o[LW_P][3]) const
+    {
+        if (!mine)
+            return;
+        if (nv == LW_P) {
+            float *p = reinterpret_cast<float *>(d);
+            if (f == CRAW_K_OUT_RGB32F) {
+#pragma unroll
+                for (int i = 0; i < 12; i += 4)
+                    *reinterpret_cast<float4 *>(p + i) = make_float4(o[i / 3][i % 3], o[(i + 1) / 3][(i + 1) % 3],
+                                                                     o[(i + 2) / 3][(i + 2) % 3],
+                                                                     o[(i + 3) / 3][(i + 3) % 3]);
+            } else if (f == CRAW_K_OUT_RGBA16F) {
+                uint32_t w[8];
+#pragma unroll
+                for (int i = 0; i < LW_P; i++) {
+                    const __half2 a = __floats2half2_rn(o[i][0], o[i][1]), b = __floats2half2_rn(o[i][2], 1.0f);
+                    w[2 * i] = *reinterpret_cast<const uint32_t *>(&a);
+                    w[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&b);
+                }
+                reinterpret_cast<uint4 *>(d)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                reinterpret_cast<uint4 *>(d)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+            } else if (!((uintptr_t)d & 31)) {
+#pragma unroll
+                for (int i = 0; i < LW_P; i += 2)
+                    walk_store8(p + 4 * i, o[i][0], o[i][1], o[i][2], 1.0f, o[i + 1][0], o[i + 1][1], o[i + 1][2],
+                                1.0f);
+            } else {
+#pragma unroll
+                for (int i = 0; i < LW_P; i++)
+                    reinterpret_cast<float4 *>(p)[i] = make_float4(o[i][0], o[i][1], o[i][2], 1.0f);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < LW_P; i++)
+                if (i < nv)
+                    craw_store_rgba(d, 0, i, 0, f, o[i][0], o[i][1], o[i][2]);
+        }
+    }
+
+    /* The 4x4 block means of (R - G, B - G, G), added row by row over the
+     * pixels inside the frame (reference lib/ref/ref_chroma.c:49-74). */
+    CRAW_DEV void quarter(int y, bool last, bool odd, const float o[LW_P][3])
+    {
+        if (!(y & 3))
+            qs[0] = qs[1] = qs[2] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < LW_P; i++)
+            if (i < nv) {
+                qs[0] = __fadd_rn(qs[0], __fsub_rn(o[i][0], o[i][1]));
+                qs[1] = __fadd_rn(qs[1], __fsub_rn(o[i][2], o[i][1]));
+                qs[2] = __fadd_rn(qs[2], o[i][1]);
+            }
+        if (!odd || !((y & 3) == 3 || last) || !mine)
+            return;
+        const int bx = x0 / 4, by = y / 4;
+        const float n = (float)(nv * ((y & 3) + 1));
+        if (craw_in_bounds(bx >= 0 && bx < (k.width + 3) / 4 && by >= 0 && by < (k.height + 3) / 4, io.err))
+            craw_store_rgba(io.quarter, io.quarter_pitch, bx, by, k.fp16, __fdiv_rn(qs[0], n), __fdiv_rn(qs[1], n),
+                            __fdiv_rn(qs[2], n));
+    }
+
+    /* The statistic of the block whose sums are s, of `rows` pixel rows in
+     * block row `by`, on the lanes that `go`. */
+    CRAW_DEV void statistic(const float s[3], int by, int rows, bool go)
+    {
+        const int bx = x0 >> 3, nx = min(8, k.width - 8 * bx);
+        const float n = (float)(nx * rows);
+        const int ri = by * ((k.width + 7) / 8) + bx;
+        if (go && craw_in_bounds(ri >= 0 && (uint32_t)ri < craw_awb_blocks(k.width, k.height), io.err))
+            io.awb.rec[ri] = craw_awb_block(__fdiv_rn(s[0], n), __fdiv_rn(s[1], n), __fdiv_rn(s[2], n), k.awb_wb,
+                                            io.awb.deferred, io.awb.nb_deferred, craw_awb_blocks(k.width, k.height));
+    }
+
+    /* The AWB sums of a row, in the reference's order (lib/awb.c:239-253):
+     * the left lane of a block adds its four pixels, the right lane its
+     * four after them. The left lanes hold the sums; every second row of
+     * blocks the right lanes take the row above's, so that the statistic
+     * (over a hundred instructions) runs on all lanes at once. */
+    CRAW_DEV void awb_row(int y, bool end, bool odd, const float o[LW_P][3])
+    {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            float t = as[c];
+#pragma unroll
+            for (int i = 0; i < LW_P; i++)
+                t = nv == LW_P || i < nv ? __fadd_rn(t, o[i][c]) : t;
+            float u = walk_left(t);
+#pragma unroll
+            for (int i = 0; i < LW_P; i++)
+                u = nv == LW_P || i < nv ? __fadd_rn(u, o[i][c]) : u;
+            as[c] = walk_right(u);
+        }
+        if (!odd || ((y & 7) != 7 && !end))
+            return;
+        const int by = y >> 3;
+        if (!held && !end) {
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+                hs[c] = as[c];
+            held = by + 1;
+        } else {
+            float s[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const float above = walk_left(hs[c]);
+                s[c] = right ? above : as[c];
+            }
+            statistic(s, right ? held - 1 : by, right ? 8 : (y & 7) + 1,
+                      right ? held && x0 - LW_P < k.width && mine_pair() : mine);
+            held = 0;
+        }
+        as[0] = as[1] = as[2] = 0.0f;
+    }
+    /* Whether the lane's AWB block is an output of the strip (its right
+     * lane may lie past the frame's edge). */
+    CRAW_DEV bool mine_pair() const
+    {
+        const int lane = threadIdx.x & 31;
+        return lane >= 1 && lane <= LW_N;
+    }
+
+    /* The epilogue of frame row y (`end`: the segment's last; `odd`: its
+     * parity, constant where it is inlined): o the lane's camera RGB. */
+    CRAW_DEV void row(int y, bool end, bool odd, float o[LW_P][3])
+    {
+        if (k.fp16) {
+#pragma unroll
+            for (int i = 0; i < LW_P; i++)
+#pragma unroll
+                for (int c = 0; c < 3; c++)
+                    o[i][c] = craw_round_half(o[i][c]);
+        }
+        if (CHROMA || (ANY && io.inter)) {
+            store(inter, k.fp16 ? CRAW_K_OUT_RGBA16F : CRAW_K_OUT_RGBA32F, o);
+            inter += io.inter_pitch;
+        }
+        if constexpr (CHROMA) {
+            quarter(y, end, odd, o);
+            return;
+        }
+        if (io.awb.rec)
+            awb_row(y, end, odd, o);
+        if (!ANY || io.dst) {
+            walk_colour<-1>(k.color, mine, o);
+            store(dst, ANY ? io.dst_fmt : EPI, o);
+            dst += io.dst_pitch;
+        }
+    }
+
+    /* The strip of warp `wid` of the grid: the whole frame's, in strips of
+     * LW_N lanes and segments of g.seg quad rows. */
+    CRAW_DEV void run(const WalkGrid &g, int wid)
+    {
+        const int lane = threadIdx.x & 31, sx = wid % g.nx, sy = wid / g.nx;
+        if (sy * g.seg >= g.nqy)
+            return;
+        const int y0 = 2 * sy * g.seg, rows = 2 * min(g.seg, g.nqy - sy * g.seg);
+        x0 = LW_P * (sx * LW_N - 1 + lane);
+        edge = sx == 0 || LW_P * (sx * LW_N + 31) >= k.width;
+        inside = x0 >= 0 && x0 + LW_P <= k.width;
+        partial = x0 + 2 == k.width;
+        mine = lane >= 1 && lane <= LW_N && x0 < k.width;
+        right = !(lane & 1);
+        nv = min(LW_P, k.width - x0);
+        held = 0;
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            as[c] = hs[c] = qs[c] = 0.0f;
+        const int f = ANY ? io.dst_fmt : EPI;
+        dst = (char *)io.dst + (size_t)y0 * io.dst_pitch +
+              (ptrdiff_t)x0 * (f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16));
+        inter = (char *)io.inter + (size_t)y0 * io.inter_pitch + (ptrdiff_t)x0 * (k.fp16 ? 8 : 16);
+
+        int y = y0;
+        const char *src = (const char *)io.src + (size_t)y0 * io.src_pitch;
+        auto fetch = [&]() {
+            const uint2 u = load(src);
+            y++;
+            src += y < k.height ? (ptrdiff_t)io.src_pitch : -(ptrdiff_t)io.src_pitch;
+            return u;
+        };
+        /* The window's first rows, and the first two steps' two each; every
+         * load is issued before the first is used. */
+        uint2 first[2 * RAD], next[2][2];
+#pragma unroll
+        for (int i = 0; i < RAD; i++)
+            first[i] = load((const char *)io.src + (size_t)craw_mirror(y0 - RAD + i, k.height) * io.src_pitch);
+#pragma unroll
+        for (int i = RAD; i < 2 * RAD; i++)
+            first[i] = fetch();
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            next[i >> 1][i & 1] = fetch();
+#pragma unroll
+        for (int i = 0; i < 2 * RAD; i++)
+            put(i, first[i], (i + RAD) & 1);
+#pragma unroll 1
+        for (int r = 0; r < rows; r += 2) {
+            put(2 * RAD, next[0][0], RAD & 1);
+            put(2 * RAD + 1, next[0][1], (RAD + 1) & 1);
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                next[0][i] = next[1][i];
+                next[1][i] = fetch();
+            }
+#pragma unroll
+            for (int b = 0; b < 2; b++) {
+                float o[LW_P][3];
+#pragma unroll
+                for (int i = 0; i < LW_P; i++) {
+                    if constexpr (METHOD == kMhc)
+                        mhc_px(*this, RAD + i, RAD + b, 2 * b + (i & 1), o[i]);
+                    else
+                        bilinear_px(*this, RAD + i, RAD + b, 2 * b + (i & 1), o[i]);
+                }
+                /* A segment has whole quad rows: only their second row can
+                 * end a block or the segment. */
+                row(y0 + r + b, b && r + 2 == rows, b, o);
+            }
+#pragma unroll
+            for (int i = 0; i < 2 * RAD; i++)
+#pragma unroll
+                for (int c = 0; c < WC; c++)
+                    v[i][c] = v[i + 2][c];
+        }
+    }
+};
 
 } // namespace craw_dev

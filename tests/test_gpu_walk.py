@@ -3,14 +3,18 @@ segment of rows a warp) where their dispatch branches: the RCD's interior
 against its 64x16 tiles, bit for bit (the two evaluate the same formulas
 with the same roundings), for every output layout, an output whose rows are
 16-byte but not 32-byte aligned, the chroma path's block means (through the
-whole chroma denoise), and the gamut compression on saturated colours."""
+whole chroma denoise), and the gamut compression on saturated colours; the
+bilinear and MHC frames against the batch's per-pixel tiles, bit for bit, at
+the widths where a lane or an AWB block hangs over the edge, their histogram
+against the CPU builder, and their chroma path against the oracle."""
 import numpy as np
 import pytest
 import torch
 
 import libcraw_gb300 as L
 from libcraw_gb300 import workloads as W
-from gpu_util import develop, upload_mosaic
+from gpu_util import alloc_rgba, develop, download_image, upload_mosaic
+from oracle import Oracle, max_rel
 
 pytestmark = pytest.mark.gpu
 
@@ -112,3 +116,58 @@ def test_gamut_compression_against_float64(ctx):
     want = np.where(d < thr, x, ach - (thr + scl * nd / (1 + nd ** p) ** (1 / p)) * np.abs(ach))
     assert (d >= thr).mean() > 0.001, "the scene has no saturated colours"
     assert (np.abs(out[0] - want) <= 4e-6 * np.abs(ach)).all()
+
+
+# The smallest frame; widths of every remainder by 8 (and by the strips of
+# 120 columns: one short, whole, one over); heights of every remainder by 8.
+LINEAR = [(8, 8), (10, 12), (118, 18), (120, 24), (122, 38), (244, 62), (366, 50), (1030, 20)]
+
+
+@pytest.mark.parametrize("w,h", LINEAR)
+@pytest.mark.parametrize("deb", [L.DEBAYER_BILINEAR, L.DEBAYER_MHC])
+@pytest.mark.parametrize("fmt", [L.FORMAT_RGBA32F, L.FORMAT_RGB32F, L.FORMAT_RGBA16F])
+def test_linear_frames_equal_tiles(ctx, w, h, deb, fmt):
+    m = W.synth_frame(w, h, 11 * w + h, rects=12, noise_a_dn=4.0, noise_b_dn=40.0)
+    fp = L.frame_params(W.make_profile())
+    space = L.CS_ACES_AP1 if w % 4 else L.CS_BT2020
+    if min(w, h) >= 12:                       # a batch takes frames from 12 pixels a side
+        _, src = upload_mosaic(m)
+        out, dst = alloc_rgba(w, h, fmt)
+        with L.Batch(ctx, L.batch_params(w, h, max_frames=1, debayer=deb, out_space=space, out_format=fmt,
+                                         direct_pixels=L.BATCH_ALL_PERSISTENT)) as b:
+            b.record(torch.cuda.current_stream().cuda_stream, [src], [dst], [fp])
+            torch.cuda.synchronize()
+        want = out.float().cpu().numpy()
+    pp = L.pipeline_params(w, h, debayer=deb, out_space=space, out_format=fmt, flags=L.FLAG_AWB_HISTOGRAM)
+    with L.Pipeline(ctx, pp) as pipe:
+        got = develop(pipe, m, fp, fmt)
+        hist = pipe.awb_histogram()
+        assert pipe.kernel_errors() == 0
+    if min(w, h) >= 12:
+        assert np.array_equal(got.view(np.uint8), want.view(np.uint8))
+    # The same frame with its intermediate kept (another epilogue).
+    pp = L.pipeline_params(w, h, debayer=deb, out_space=space, out_format=fmt,
+                           flags=L.FLAG_AWB_HISTOGRAM | L.FLAG_KEEP_INTERMEDIATE)
+    with L.Pipeline(ctx, pp) as pipe:
+        kept = develop(pipe, m, fp, fmt)
+        rgb = download_image(pipe.intermediate()[0], "rgba32f")
+        hist2 = pipe.awb_histogram()
+    assert np.array_equal(got.view(np.uint8), kept.view(np.uint8))
+    cnt, wgt, brt = L.awb_histogram_from_rgb(rgb, W.WB)
+    for x in (hist, hist2):
+        assert np.array_equal(x.count, cnt) and np.array_equal(x.weight, wgt) and \
+            np.array_equal(x.weight_bright, brt)
+
+
+@pytest.mark.parametrize("w,h", [(20, 20), (118, 22), (122, 26), (244, 62)])
+@pytest.mark.parametrize("deb", [L.DEBAYER_BILINEAR, L.DEBAYER_MHC])
+def test_linear_chroma_vs_oracle(ctx, w, h, deb):
+    """The bound is the stage's own (the float oracle within 2e-4)."""
+    m = W.synth_frame(w, h, 13 * w + h, rects=12, noise_a_dn=4.0, noise_b_dn=40.0)
+    pp = L.pipeline_params(w, h, debayer=deb, out_space=L.CS_BT709, out_format=L.FORMAT_RGBA32F,
+                           flags=L.FLAG_CHROMA_DENOISE)
+    fp = L.frame_params(W.make_profile(), denoise_chroma_strength=0.8)
+    with L.Pipeline(ctx, pp) as pipe:
+        got = develop(pipe, m, fp)
+        assert pipe.kernel_errors() == 0
+    assert max_rel(got, Oracle().process(m, pp, fp, "f32")) <= 2e-4
