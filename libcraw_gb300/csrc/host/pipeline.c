@@ -90,6 +90,8 @@ struct CRAWPipeline {
     float *lvl[2];    size_t lvl_pitch;
     uint8_t *var[2];  size_t var_pitch;
     int tn_prev, tn_cur;
+    float *dn_planes;         /* spatial + temporal: the averaged planes of the frame
+                               * being denoised, craw_k_denoise_planes bytes */
     void *inter;      size_t inter_pitch;
     void *q, *qf;     size_t q_pitch;
     int qw, qh;
@@ -154,7 +156,7 @@ static void release(CRAWPipeline *p)
     void *bufs[] = {
         p->clean, p->lvl[0], p->lvl[1], p->var[0], p->var[1], p->inter, p->q, p->qf,
         p->awb_rec, p->awb_dev, p->kerr, p->p_v, p->p_scratch, p->p_t, p->p_var,
-        p->hl_mosaic, p->hl_levels, p->round_flags, p->round_stats, p->round_list,
+        p->hl_mosaic, p->hl_levels, p->dn_planes, p->round_flags, p->round_stats, p->round_list,
     };
     cudaSetDevice(ctx->device);
     for (size_t i = 0; i < CRAW_ARRAY_ELEMS(bufs); i++)
@@ -237,7 +239,7 @@ static void tune_release(CRAWPipeline *p)
 }
 
 static int time_denoise(CRAWPipeline *p, const CRAWKDenoise *k, const CRAWKDenoiseIO *io, int shape,
-                        float *ms)
+                        float *planes, float *ms)
 {
     CRAWContext *ctx = p->ctx;
     cudaEvent_t e0, e1;
@@ -253,7 +255,7 @@ static int time_denoise(CRAWPipeline *p, const CRAWKDenoise *k, const CRAWKDenoi
     for (int r = 0; r < 4 && ret == 0; r++) {
         float t = 0.0f;
         cudaEventRecord(e0, ctx->stream);
-        ret = craw_k_denoise(k, io, shape, NULL, NULL, ctx->stream);
+        ret = craw_k_denoise(k, io, shape, NULL, planes, NULL, ctx->stream);
         cudaEventRecord(e1, ctx->stream);
         if (ret == 0 && cudaEventSynchronize(e1) == cudaSuccess &&
             cudaEventElapsedTime(&t, e0, e1) == cudaSuccess && r > 0 && t < *ms)
@@ -269,7 +271,7 @@ static int autotune(CRAWPipeline *p)
     CRAWContext *ctx = p->ctx;
     const uint32_t w = p->params.width, h = p->params.height;
     uint16_t *mosaic = NULL;
-    float *lvl = NULL;
+    float *lvl = NULL, *planes = NULL;
     uint8_t *var = NULL;
     size_t mp, lp, vp;
     int ret = 0;
@@ -296,7 +298,9 @@ static int autotune(CRAWPipeline *p)
 
     if ((ret = alloc_pitched(p, (void **)&mosaic, &mp, (size_t)w * 2, h)) < 0 ||
         (ret = alloc_pitched(p, (void **)&lvl, &lp, (size_t)w * 4, h)) < 0 ||
-        (ret = alloc_pitched(p, (void **)&var, &vp, (size_t)w, h)) < 0)
+        (ret = alloc_pitched(p, (void **)&var, &vp, (size_t)w, h)) < 0 ||
+        (need[1] && !p->dn_planes &&
+         (ret = craw_dev_alloc(ctx, (void **)&planes, craw_k_denoise_planes((int32_t)(w / 2), (int32_t)(h / 2)))) < 0))
         goto done;
     /* A mid-grey mosaic, a state of level 0.25 and unit variance. */
     cudaMemset2DAsync(mosaic, mp, 0x08, (size_t)w * 2, h, ctx->stream);
@@ -325,7 +329,7 @@ static int autotune(CRAWPipeline *p)
             continue;
         for (int shape = 0; shape < CRAW_K_DN_SHAPE_NB; shape++) {
             float ms;
-            if ((ret = time_denoise(p, &k, &io, shape, &ms)) < 0)
+            if ((ret = time_denoise(p, &k, &io, shape, p->dn_planes ? p->dn_planes : planes, &ms)) < 0)
                 goto done;
             if (ms < best) {
                 best = ms;
@@ -355,6 +359,7 @@ static int autotune(CRAWPipeline *p)
     pthread_mutex_unlock(&tune_lock);
 done:
     craw_dev_free(ctx, mosaic);
+    craw_dev_free(ctx, planes);
     craw_dev_free(ctx, lvl);
     craw_dev_free(ctx, var);
     if (craw_dev_sync(ctx) < 0 && ret == 0)
@@ -507,6 +512,10 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
                 (ret = alloc_pitched(p, (void **)&p->var[i], &p->var_pitch, (size_t)w, h)) < 0)
                 goto fail;
         }
+        if (p->has_denoise && !p->plain &&
+            (ret = craw_dev_alloc(ctx, (void **)&p->dn_planes,
+                                  craw_k_denoise_planes((int32_t)(w / 2), (int32_t)(h / 2)))) < 0)
+            goto fail;
     }
     if (p->has_chroma || p->keep || p->plain) {
         size_t bpp = p->fp16 ? 8 : 16;
@@ -765,7 +774,7 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
         prof_begin(&pc, ST_DENOISE);
         ret = p->plain ? craw_k_plain_denoise(&dnk, &io, p->p_t, p->p_var, s)
                        : craw_k_denoise(&dnk, &io, p->dn_shape[(dn_mode & CRAW_K_DN_HISTORY) != 0],
-                                        exact ? &rd : NULL, p->kerr, s);
+                                        exact ? &rd : NULL, p->dn_planes, p->kerr, s);
         prof_end(&pc);
         if (ret < 0)
             goto launch_fail;

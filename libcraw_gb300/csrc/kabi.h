@@ -116,10 +116,15 @@ typedef struct CRAWKDenoiseExact {
  * the undecided ones), for a frame of plane size pw x ph. */
 #define CRAW_K_ROUND_LIST(pw, ph) (((size_t)4 * (pw) * (ph)) / 16 + 65536)
 
-/* rd: NULL, or the marking of samples near a code boundary. err: NULL,
- * or a device word for CRAW_K_ERR_* bits. */
+/* rd: NULL, or the marking of samples near a code boundary. planes: the
+ * scratch of the packed shapes with a history (craw_k_denoise_planes bytes;
+ * else NULL). err: NULL, or a device word for CRAW_K_ERR_* bits. */
 int craw_k_denoise(const CRAWKDenoise *k, const CRAWKDenoiseIO *io, int shape,
-                   const CRAWKRound *rd, uint32_t *err, cudaStream_t s);
+                   const CRAWKRound *rd, float *planes, uint32_t *err, cudaStream_t s);
+
+/* Bytes of the padded stabilised and variance planes of a frame of plane
+ * size pw x ph (150 MB at 5760x3240). */
+size_t craw_k_denoise_planes(int32_t pw, int32_t ph);
 
 /* 1 (default): the packed spatial denoise kernels bring each interior
  * tile's mosaic in with one TMA tile copy; 0: with plain loads

@@ -24,10 +24,21 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tma.cuh"
 
 namespace craw_dn {
+
+/* A pair from shared memory, loaded where it is written (volatile: not
+ * kept in registers across a loop). */
+CRAW_DEV f2x f2_lds(const float *p)
+{
+    f2x v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    return v;
+}
 
 
 constexpr int S = 3;     /* search radius, reference lib/pipeline.c:261 */
@@ -59,7 +70,18 @@ CRAW_DEV float level(const CRAWKDenoise &k, uint32_t raw, int pl)
     return ((float)raw * (1.0f / 65535.0f) - k.black[pl]) * k.inv_range[pl];
 }
 
-/* The four plane samples of mosaic quad (qx, qy): R, Gr, Gb, B. */
+/* A filtered level back as a 16-bit code position (not yet rounded) after
+ * the highlight guard toward the sample's own raw value (reference
+ * lib/ref/ref_denoise.c:285-323); blk, irng, rng: the plane's constants. */
+CRAW_DEV float encode(const CRAWKDenoise &k, float u, uint16_t raw0, float blk, float irng, float rng)
+{
+    float u0 = ((float)raw0 * (1.0f / 65535.0f) - blk) * irng;
+    float gr = fminf(fmaxf((u0 - k.guard_lo) * k.guard_inv, 0.0f), 1.0f);
+    u = u + (u0 - u) * gr;
+    float ro = fminf(fmaxf(blk + u * rng, 0.0f), 1.0f);
+    return ro * 65535.0f;
+}
+
 /* The quad at plane position (qx, qy): its two mosaic rows as 32-bit
  * pairs (a: R, Gr; b: Gb, B) and the four samples. */
 CRAW_DEV void load_quad_u16(const CRAWKDenoise &k, const CRAWKDenoiseIO &io, int qx, int qy, uint32_t q[4],
@@ -385,6 +407,100 @@ struct SearchX2 {
     }
 };
 
+/* The same search of 2 columns x 8 rows, row by row and without the patch
+ * block in registers: a window row's squared differences and row sums for
+ * all seven dx, then the column sums that the row completes, their weights
+ * and the weighted sums. Live beside the sums: a row's window pairs, two
+ * rows of row sums, the centres of the row before. The patch block's rows
+ * are read again from the tile by every dy (two loads in some hundred
+ * instructions). That takes 124 registers instead of 154, four CTAs an SM
+ * instead of three: 413 -> 401 us at 5760x3240, where the FMA pipe is the
+ * bound (70 % active on average, saturated during the search). Same values
+ * in the same order as SearchX2. TO: the shifted copy's distance from the
+ * tile, in floats; with a history V is the variance's, and `lvc` is log2(e)
+ * over the thread's centres' (rows of LVS floats). */
+template <int R, int TS, bool HISTORY, int TO, int V = 0, int LVS = 32>
+struct SearchRows {
+    static constexpr int M = 8, N = 2 * S + 1;
+    static_assert(R - 1 == S, "window origin");
+    f2x acc[M], wsum[M];
+    f2x c1, c0;                       /* with a history c1 is -1/(9h^2) */
+
+    CRAW_DEV void init(float inv_h2)
+    {
+        const float kd = (1.0f / 9.0f) * inv_h2;
+        c1 = HISTORY ? f2_pack(-kd, -kd) : f2_pack(-kLog2e * kd, -kLog2e * kd);
+        c0 = HISTORY ? f2_pack(kLog2e, kLog2e) : f2_pack(2.0f * kLog2e, 2.0f * kLog2e);
+#pragma unroll
+        for (int m = 0; m < M; m++)
+            acc[m] = wsum[m] = f2_pack(0.0f, 0.0f);
+    }
+
+    /* `at0`: the tile at the thread's (ox0, oy0). */
+    CRAW_DEV void step_dy(const float *at0, const float *lvc, int dy)
+    {
+        const float *atd = at0 + dy * TS;
+        f2x h0[N], h1[N], mid[N];     /* row sums of rows r - 2 and r - 1; the shared column pair */
+        f2x q[N];                     /* the shifted centres of row r - 1 */
+#pragma unroll
+        for (int r = 0; r < M + 2; r++) {
+            const float *at = atd + (R - 1 + r) * TS;
+            /* Window columns c, c + 1 as a pair: even starts from the tile,
+             * odd ones from its copy shifted by one. */
+            f2x w[N + 2], h[N];
+#pragma unroll
+            for (int c = 0; c < N + 2; c++)
+                w[c] = f2_ld(at + ((c & 1) ? TO - 1 : 0) + c);
+            const float *row = at0 + TO + (R - 1 + r) * TS + S - 1;
+            const f2x own0 = f2_lds(row), own1 = f2_lds(row + 2);
+#pragma unroll
+            for (int o = 0; o < N; o++) {
+                const f2x d0 = f2_sub(own0, w[o]), d1 = f2_sub(own1, w[o + 2]);
+                const f2x e0 = f2_mul(d0, d0), e1 = f2_mul(d1, d1);
+                /* Row sums of three, the middle pair shared. */
+                const float m3 = f2_hi(e0) + f2_lo(e1);
+                h[o] = f2_pack(f2_lo(e0) + m3, m3 + f2_hi(e1));
+            }
+            if (r >= 2) {
+                const int m = r - 2;
+                f2x nkl = c1, lv = c1;
+                if constexpr (HISTORY) {
+                    lv = f2_lds(lvc + LVS * m);
+                    nkl = f2_mul(c1, lv);
+                }
+#pragma unroll
+                for (int o = 0; o < N; o++) {
+                    /* Column sums of three, the middle pair shared by two rows. */
+                    f2x d2, x;
+                    if (!(r & 1)) {
+                        mid[o] = f2_add(h1[o], h[o]);
+                        d2 = f2_add(h0[o], mid[o]);
+                    } else {
+                        d2 = f2_add(mid[o], h[o]);
+                    }
+                    if constexpr (HISTORY) {
+                        /* The shifted centres' variance, window columns 1 + o, 2 + o. */
+                        const float *vs = atd + V + (R + m) * TS + 1 + o;
+                        const f2x vq = (o & 1) ? f2_ld(vs) : f2_pack(vs[0], vs[1]);
+                        x = f2_fma(d2, nkl, f2_fma(vq, lv, c0));
+                    } else {
+                        x = f2_fma(d2, nkl, c0);
+                    }
+                    const f2x wt = f2_pack(craw_ex2(fminf(f2_lo(x), 0.0f)), craw_ex2(fminf(f2_hi(x), 0.0f)));
+                    wsum[m] = f2_add(wsum[m], wt);
+                    acc[m] = f2_fma(wt, q[o], acc[m]);
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < N; o++) {
+                h0[o] = h1[o];
+                h1[o] = h[o];
+                q[o] = w[o + 1];
+            }
+        }
+    }
+};
+
 /* One tile (tile column bx, tile row by) of all four planes; the whole
  * CTA takes part. `smem` holds Cfg::smem_floats floats. MARK (spatial
  * only): `rd` is the marking of samples whose code lies near a rounding
@@ -554,12 +670,22 @@ CRAW_DEV void denoise_tile(const CRAWKDenoise &k, const CRAWKDenoiseIO &io, int 
 
     if constexpr (C::PACKED) {
         const float *To = smem + C::TO_OFF + pl * C::TN;
-        const float *Vp = V + pl * C::TN, *Vo = smem + C::VO_OFF + pl * C::TN;
-        SearchX2<M, R, TS, HISTORY, MARK> st;
-        st.init(To, Vp, ox0, oy0, k.inv_h2);
+        /* Eight rows a thread with uncentred sums: row by row (its history
+         * has a kernel of its own, denoise_history.cuh). */
+        std::conditional_t<M == 8 && !MARK && !HISTORY, SearchRows<R, TS, false, C::TO_OFF>,
+                           SearchX2<M, R, TS, HISTORY, MARK>> st;
+        if constexpr (M == 8 && !MARK && !HISTORY) {
+            st.init(k.inv_h2);
 #pragma unroll 1
-        for (int dy = -S; dy <= S; dy++)
-            st.step_dy(Tp, To, Vp, Vo, ox0, oy0, dy);
+            for (int dy = -S; dy <= S; dy++)
+                st.step_dy(Tp + oy0 * TS + ox0, nullptr, dy);
+        } else {
+            const float *Vp = V + pl * C::TN, *Vo = smem + C::VO_OFF + pl * C::TN;
+            st.init(To, Vp, ox0, oy0, k.inv_h2);
+#pragma unroll 1
+            for (int dy = -S; dy <= S; dy++)
+                st.step_dy(Tp, To, Vp, Vo, ox0, oy0, dy);
+        }
 #pragma unroll
         for (int m = 0; m < M; m++) {
             res[m][0] = __fdiv_rn(f2_lo(st.acc[m]), f2_lo(st.wsum[m]));
@@ -629,11 +755,7 @@ CRAW_DEV void denoise_tile(const CRAWKDenoise &k, const CRAWKDenoiseIO &io, int 
                 raw0 = *cell;
             else
                 raw0 = __ldg((const uint16_t *)((const char *)io.src + (size_t)my * io.src_pitch) + mx);
-            float u0 = ((float)raw0 * (1.0f / 65535.0f) - blk) * irng;
-            float gr = fminf(fmaxf((u0 - k.guard_lo) * k.guard_inv, 0.0f), 1.0f);
-            u = u + (u0 - u) * gr;
-            float ro = fminf(fmaxf(blk + u * rng, 0.0f), 1.0f);
-            const float xv = ro * 65535.0f;
+            const float xv = encode(k, u, raw0, blk, irng, rng);
             const uint16_t code = (uint16_t)rintf(xv);
             if (mark) {
                 /* Within the float error of a rounding boundary: the exact

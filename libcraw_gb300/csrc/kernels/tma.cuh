@@ -46,6 +46,24 @@ __device__ __forceinline__ void load_2d(void *dst, const CUtensorMap *tmap, int 
                  : "memory");
 }
 
+/* One thread: the 3-D boxes of two tensor maps at element coordinates (x, y,
+ * z) into `a` and `b` (`bytes` of both), completing on `bar`. x times the
+ * element size must be a multiple of 16 bytes; the caller checks. */
+__device__ __forceinline__ void load_3d2(void *a, const CUtensorMap *ma, void *b, const CUtensorMap *mb, int x, int y,
+                                         int z, uint64_t *bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                 :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(smem_u32(a)), "l"(reinterpret_cast<uint64_t>(ma)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                 " [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(smem_u32(b)), "l"(reinterpret_cast<uint64_t>(mb)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 /* Waits (a bounded number of tries) for phase `parity` of `bar`; false if
  * it did not complete. */
 __device__ __forceinline__ bool wait(uint64_t *bar, uint32_t parity)
@@ -70,3 +88,8 @@ __device__ __forceinline__ bool wait(uint64_t *bar, uint32_t parity)
  * thread. False where the driver call is not available or refuses the
  * layout (src and pitch must be 16-byte aligned). */
 bool craw_tmap_u16(const void *src, size_t pitch, int w, int h, int bw, int bh, CUtensorMap *out);
+
+/* The tensor map of four float planes (w x h each, one after another, rows
+ * of a multiple of 16 bytes) for boxes of bw x bh samples of all four;
+ * false as above. */
+bool craw_tmap_f32x4(const float *src, int w, int h, int bw, int bh, CUtensorMap *out);
