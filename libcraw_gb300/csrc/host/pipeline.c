@@ -8,12 +8,12 @@
  *
  *   denoise   mosaic (+ state) -> denoised mosaic (+ next state)
  *   develop   mosaic -> dst directly (prep, debayer, colour and the AWB
- *             block records fused); with the chroma denoise, mosaic ->
+ *             histogram fused); with the chroma denoise, mosaic ->
  *             intermediate + quarter-resolution block means instead
  *   [blur]    quarter -> filtered quarter
- *   [up]      intermediate + quarters -> dst (+ AWB block records)
- *   awb       block records -> histogram, then a copy into the pinned
- *             host slot of this recording
+ *   [up]      intermediate + quarters -> dst (+ AWB histogram)
+ *   awb       the histogram's copy into the pinned host slot of this
+ *             recording
  *
  * The library never synchronises the caller's stream. Intermediates come
  * from a CUDA memory pool (cudaMallocFromPoolAsync on the context's own
@@ -54,16 +54,16 @@ static const char *const plain_stage_names[ST_NB] = {
     "denoise_round",
 };
 
-/* One AWB slot. On the host, pinned: the three histograms, the count of
- * deferred blocks and the first CRAW_K_AWB_DEFER_MAX of them, filled by
- * two async copies. On the device: the slot's whole list of deferred
- * blocks (its count, then one entry per 8x8 block of the frame at most),
- * from which a count above CRAW_K_AWB_DEFER_MAX is read on demand. */
-#define SLOT_BYTES (HIST_BYTES + 16 + DEFER_BYTES)
+/* One AWB slot: the three histograms, the count of deferred blocks and the
+ * blocks themselves. On the device room for every 8x8 block of the frame; on
+ * the host, pinned, the first CRAW_K_AWB_DEFER_MAX of them, filled by one
+ * async copy (a count above that is read from the device on demand). The
+ * device's histograms and count are zeroed by one fill before the frame. */
+#define ZERO_BYTES (HIST_BYTES + 16)
+#define SLOT_BYTES (ZERO_BYTES + DEFER_BYTES)
 struct awb_slot {
     uint8_t *host;            /* SLOT_BYTES */
-    uint8_t *list;            /* device: the count (16 B), then room for
-                               * max(nb_blocks, CRAW_K_AWB_DEFER_MAX) entries */
+    uint8_t *dev;             /* the same layout, max(nb_blocks, CRAW_K_AWB_DEFER_MAX) entries */
     bool folded;              /* deferred blocks already binned */
 };
 
@@ -95,8 +95,6 @@ struct CRAWPipeline {
     void *inter;      size_t inter_pitch;
     void *q, *qf;     size_t q_pitch;
     int qw, qh;
-    uint64_t *awb_rec;
-    uint8_t *awb_dev;         /* HIST_BYTES: the histograms being built */
     uint32_t nb_blocks;
     uint32_t *kerr;           /* CRAW_K_ERR_* bits the kernels set */
     uint32_t *round_flags;    /* marks of the exact rounding, CRAW_K_ROUND_WORDS */
@@ -155,7 +153,7 @@ static void release(CRAWPipeline *p)
     tune_release(p);
     void *bufs[] = {
         p->clean, p->lvl[0], p->lvl[1], p->var[0], p->var[1], p->inter, p->q, p->qf,
-        p->awb_rec, p->awb_dev, p->kerr, p->p_v, p->p_scratch, p->p_t, p->p_var,
+        p->kerr, p->p_v, p->p_scratch, p->p_t, p->p_var,
         p->hl_mosaic, p->hl_levels, p->dn_planes, p->round_flags, p->round_stats, p->round_list,
     };
     cudaSetDevice(ctx->device);
@@ -163,7 +161,7 @@ static void release(CRAWPipeline *p)
         craw_dev_free(ctx, bufs[i]);
     craw_dev_sync(ctx);
     for (uint32_t i = 0; i < 4; i++) {
-        craw_dev_free(ctx, p->slots[i].list);
+        craw_dev_free(ctx, p->slots[i].dev);
         if (p->slots[i].host)
             cudaFreeHost(p->slots[i].host);
     }
@@ -546,15 +544,12 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
     }
     if (p->awb) {
         p->nb_blocks = ((w + 7) / 8) * ((h + 7) / 8);
-        if ((ret = craw_dev_alloc(ctx, (void **)&p->awb_rec, (size_t)p->nb_blocks * 8)) < 0 ||
-            (ret = craw_dev_alloc(ctx, (void **)&p->awb_dev, HIST_BYTES)) < 0)
-            goto fail;
         for (uint32_t i = 0; i < p->nb_slots; i++) {
             /* Room for every block, and at least for the part the slot's
              * async copy reads. */
             const size_t entries = CRAW_MAX((size_t)p->nb_blocks, (size_t)CRAW_K_AWB_DEFER_MAX);
-            if ((ret = craw_dev_alloc(ctx, (void **)&p->slots[i].list,
-                                      16 + entries * sizeof(CRAWKAwbDeferred))) < 0)
+            if ((ret = craw_dev_alloc(ctx, (void **)&p->slots[i].dev,
+                                      ZERO_BYTES + entries * sizeof(CRAWKAwbDeferred))) < 0)
                 goto fail;
             if (cudaHostAlloc((void **)&p->slots[i].host, SLOT_BYTES, cudaHostAllocDefault) != cudaSuccess) {
                 ret = CRAW_ERROR(ENOMEM);
@@ -742,16 +737,13 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
         pc.slot->nb = 0;
     }
 
-    uint8_t *awb_hist = NULL;
     CRAWKAwbOut awb = { 0 };
     if (p->awb) {
-        uint8_t *list = p->slots[p->nb_recorded % p->nb_slots].list;
-        awb_hist = p->awb_dev;
-        awb.rec = p->plain ? NULL : p->awb_rec;
-        awb.deferred = (CRAWKAwbDeferred *)(list + 16);
-        awb.nb_deferred = (uint32_t *)list;
-        if (cudaMemsetAsync(awb_hist, 0, HIST_BYTES, s) != cudaSuccess ||
-            cudaMemsetAsync(awb.nb_deferred, 0, 4, s) != cudaSuccess)
+        uint8_t *dev = p->slots[p->nb_recorded % p->nb_slots].dev;
+        awb.hist = (uint32_t *)dev;
+        awb.nb_deferred = (uint32_t *)(dev + HIST_BYTES);
+        awb.deferred = (CRAWKAwbDeferred *)(dev + ZERO_BYTES);
+        if (cudaMemsetAsync(dev, 0, ZERO_BYTES, s) != cudaSuccess)
             return CRAW_ERROR(EIO);
     }
 
@@ -844,7 +836,7 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
         dio.dst_fmt = craw_out_layout(dst->format);
         prof_begin(&pc, ST_DEVELOP);
         ret = craw_k_plain_develop(&dk, &dio, chroma ? &ck : NULL, p->p_v, p->inter, p->inter_pitch,
-                                   p->p_scratch, p->q, p->qf, p->awb ? (uint32_t *)awb_hist : NULL, s);
+                                   p->p_scratch, p->q, p->qf, awb.hist, s);
         prof_end(&pc);
         if (ret < 0)
             goto launch_fail;
@@ -889,16 +881,13 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
 
     if (p->awb) {
         struct awb_slot *slot = &p->slots[p->nb_recorded % p->nb_slots];
-        if (!p->plain) {
+        cudaError_t e;
+        if (!p->plain)
             prof_begin(&pc, ST_AWB);
-            ret = craw_k_awb_reduce(p->awb_rec, p->nb_blocks, (uint32_t *)awb_hist, s);
+        e = cudaMemcpyAsync(slot->host, slot->dev, SLOT_BYTES, cudaMemcpyDeviceToHost, s);
+        if (!p->plain)
             prof_end(&pc);
-            if (ret < 0)
-                goto launch_fail;
-        }
-        if (cudaMemcpyAsync(slot->host, p->awb_dev, HIST_BYTES, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaMemcpyAsync(slot->host + HIST_BYTES, slot->list, 16 + DEFER_BYTES, cudaMemcpyDeviceToHost,
-                            s) != cudaSuccess) {
+        if (e != cudaSuccess) {
             ret = CRAW_ERROR(EIO);
             goto launch_fail;
         }
@@ -949,7 +938,7 @@ CRAW_API int craw_pipeline_get_awb_histogram_n(CRAWPipeline *p, uint32_t frames_
          * first CRAW_K_AWB_DEFER_MAX came with the slot, the rest (a frame
          * with that many blocks on bin edges) are read from the slot's
          * device list now. */
-        const CRAWKAwbDeferred *d = (const CRAWKAwbDeferred *)(slot->host + HIST_BYTES + 16);
+        const CRAWKAwbDeferred *d = (const CRAWKAwbDeferred *)(slot->host + ZERO_BYTES);
         const uint32_t nd = *(const uint32_t *)(slot->host + HIST_BYTES);
         const uint32_t nd0 = CRAW_MIN(nd, (uint32_t)CRAW_K_AWB_DEFER_MAX);
         for (uint32_t i = 0; i < nd0; i++)
@@ -959,7 +948,7 @@ CRAW_API int craw_pipeline_get_awb_histogram_n(CRAWPipeline *p, uint32_t frames_
             if (!rest)
                 return CRAW_ERROR(ENOMEM);
             cudaSetDevice(p->ctx->device);
-            if (cudaMemcpy(rest, slot->list + 16 + (size_t)nd0 * sizeof(*rest), (size_t)(nd - nd0) * sizeof(*rest),
+            if (cudaMemcpy(rest, slot->dev + ZERO_BYTES + (size_t)nd0 * sizeof(*rest), (size_t)(nd - nd0) * sizeof(*rest),
                            cudaMemcpyDeviceToHost) != cudaSuccess) {
                 free(rest);
                 return CRAW_ERROR(EIO);

@@ -173,14 +173,14 @@ typedef struct CRAWKDevelop {
     float awb_wb[3];                    /* white balance divided out of the block means */
 } CRAWKDevelop;
 
-/* One record per 8x8 block of the AWB histogram. 0 means "no sample".
+/* The statistic of one 8x8 block of the AWB histogram. 0 means "no sample".
  * Otherwise bit 46 set, bits 0-13 the bin, 14-29 the 16.16 weight
- * min(g, 0.5), 30-45 the 16.16 weight g^4. Blocks whose bin is within
- * rounding of a bin edge are not binned on the device: their raw ratios go
- * to the deferred list and the host bins them with its own logf, so the
- * histogram is bit for bit the CPU builder's. The host copy of a slot
- * holds the first CRAW_K_AWB_DEFER_MAX; more are read from the device
- * list when the histogram is asked for. */
+ * min(g, 0.5), 30-45 the 16.16 weight g^4; the kernels add it to the
+ * histograms. Blocks whose bin is within rounding of a bin edge are not
+ * binned on the device: their raw ratios go to the deferred list and the
+ * host bins them with its own logf, so the histogram is bit for bit the CPU
+ * builder's. The host copy of a slot holds the first CRAW_K_AWB_DEFER_MAX;
+ * more are read from the device list when the histogram is asked for. */
 #define CRAW_K_AWB_VALID (1ull << 46)
 #define CRAW_K_AWB_DEFER_MAX 4096
 
@@ -190,7 +190,7 @@ typedef struct CRAWKAwbDeferred {
 } CRAWKAwbDeferred;
 
 typedef struct CRAWKAwbOut {
-    uint64_t *rec;                 /* ceil(w/8) * ceil(h/8) records, or NULL */
+    uint32_t *hist;                /* three 128^2 histograms, zeroed before the frame; or NULL */
     CRAWKAwbDeferred *deferred;    /* room for one entry per 8x8 block of the frame */
     uint32_t *nb_deferred;         /* counter, zeroed before the frame */
 } CRAWKAwbOut;
@@ -220,7 +220,7 @@ typedef struct CRAWKDevelopIO {
 #define CRAW_K_ERR_TMA_WAIT 1u
 #define CRAW_K_ERR_BOUNDS 2u
 
-/* Prep + debayer + (colour to dst | chroma block means) + AWB records +
+/* Prep + debayer + (colour to dst | chroma block means) + AWB statistic +
  * optional intermediate, in one kernel. */
 int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int shape,
                    cudaStream_t s);
@@ -252,19 +252,13 @@ typedef struct CRAWKChroma {
 int craw_k_chroma_blur(const CRAWKChroma *c, const void *q, size_t q_pitch,
                        void *qf, size_t qf_pitch, cudaStream_t s);
 
-/* The band back into every pixel of the intermediate, then the AWB records
+/* The band back into every pixel of the intermediate, then the AWB statistic
  * and the colour stage; `inter_out` (optional) keeps the result. */
 int craw_k_chroma_up_color(const CRAWKDevelop *k, const CRAWKChroma *c,
                            const void *inter, size_t inter_pitch,
                            const void *q, const void *qf, size_t q_pitch,
                            void *dst, size_t dst_pitch, int dst_fmt,
                            void *inter_out, const CRAWKAwbOut *awb, cudaStream_t s);
-
-/* ---------------------------------------------------------------- awb */
-
-/* Folds `n` block records into the three 128^2 histograms (zeroed by the
- * caller), through shared-memory histograms with warp-aggregated atomics. */
-int craw_k_awb_reduce(const uint64_t *rec, uint32_t n, uint32_t *hist, cudaStream_t s);
 
 /* ------------------------------------------------------ highlights */
 

@@ -122,10 +122,9 @@ k_chroma_up_color(const CRAWKDevelop k, const CRAWKChroma c, const void *inter, 
         craw_color(k.color, o, co);
         craw_store_rgba(dst, dst_pitch, x, y, dst_fmt, co[0], co[1], co[2]);
     }
-    if (!awb.rec)
+    if (!awb.hist)
         return;
     __syncthreads();
-    const int blocks_x = (c.width + 7) / 8;
     for (int b = threadIdx.x; b < (TW / 8) * (TH / 8); b += NT) {
         int bx = b % (TW / 8), by = b / (TW / 8);
         if (x0 + bx * 8 >= c.width || y0 + by * 8 >= c.height)
@@ -162,12 +161,8 @@ k_chroma_up_color(const CRAWKDevelop k, const CRAWKChroma c, const void *inter, 
                 }
         }
         float n = (float)(xe * ye);
-        const size_t ri = (size_t)(y0 / 8 + by) * blocks_x + x0 / 8 + bx;
-        if (!craw_in_bounds(ri < craw_awb_blocks(k.width, k.height), c.err))
-            continue;
-        awb.rec[ri] =
-            craw_awb_block(__fdiv_rn(s0, n), __fdiv_rn(s1, n), __fdiv_rn(s2, n), k.awb_wb,
-                           awb.deferred, awb.nb_deferred, craw_awb_blocks(k.width, k.height));
+        craw_awb_add(awb.hist, craw_awb_block(__fdiv_rn(s0, n), __fdiv_rn(s1, n), __fdiv_rn(s2, n), k.awb_wb,
+                                              awb.deferred, awb.nb_deferred, craw_awb_blocks(k.width, k.height)));
     }
 }
 

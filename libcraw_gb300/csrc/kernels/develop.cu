@@ -1,6 +1,6 @@
 /*
  * The fused develop kernels (tile bodies in develop_tile.cuh): prep +
- * debayer + colour + AWB records in one launch, with the RCD's interior
+ * debayer + colour + AWB statistic in one launch, with the RCD's interior
  * tiles done by CFA quads and the rest per pixel; and their launcher.
  */
 #include <cuda.h>

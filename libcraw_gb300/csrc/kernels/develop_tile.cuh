@@ -8,9 +8,8 @@
  * writes the caller's RGBA image, or (chroma denoise on) writes the
  * camera RGB intermediate and the 4x4 block means the chroma pass works
  * on. The AWB statistic of every 8x8 block is formed from the tile in
- * shared memory in the same pass. The only HBM traffic is the mosaic in
- * (2 B/px) and the output (16 or 8 B/px), plus 8 B per 64 px of AWB
- * records.
+ * shared memory in the same pass and added to the frame's histograms. The
+ * only HBM traffic is the mosaic in (2 B/px) and the output (16 or 8 B/px).
  *
  * Borders: every array of the RCD holds at a position outside the frame
  * the value its pass computed at the position that mirrors there, which
@@ -643,7 +642,7 @@ CRAW_DEV void awb_blocks(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0
 
 /* From the tile's camera RGB (planar in shared memory, fp32, complete):
  * the intermediate as it would be stored, then the colour stage into dst,
- * or the chroma block means, and the AWB block records. */
+ * or the chroma block means, and the AWB statistic. */
 template <int TW, int TH, int NT>
 CRAW_DEV void epilogue(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0, int y0, float *rgb)
 {
@@ -654,7 +653,7 @@ CRAW_DEV void epilogue(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0, 
      * the last warp makes them while the others run the colour stage: the
      * sums are long sequential chains over a few threads, and the tile's
      * slot on the SM is held until they end. */
-    const bool awb_apart = !k.fp16 && !chroma && io.awb.rec && NT > 64;
+    const bool awb_apart = !k.fp16 && !chroma && io.awb.hist && NT > 64;
     const int ncol = awb_apart ? NT - 32 : NT;
     if (awb_apart && (int)threadIdx.x >= ncol) {
         awb_blocks<TW, TH, 32>(k, io, x0, y0, rgb, threadIdx.x - ncol);
@@ -680,7 +679,7 @@ CRAW_DEV void epilogue(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0, 
             craw_store_rgba(io.dst, io.dst_pitch, x, y, io.dst_fmt, o[0], o[1], o[2]);
         }
     }
-    if ((!chroma && !io.awb.rec) || awb_apart)
+    if ((!chroma && !io.awb.hist) || awb_apart)
         return;
     if (k.fp16)
         __syncthreads();
@@ -716,14 +715,13 @@ CRAW_DEV void epilogue(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0, 
     awb_blocks<TW, TH, NT>(k, io, x0, y0, rgb, threadIdx.x);
 }
 
-/* The AWB records of the tile's 8x8 blocks, block means summed row by row
+/* The AWB statistic of the tile's 8x8 blocks, block means summed row by row
  * (reference lib/awb.c:239-253); thread t of NTH takes blocks t, t + NTH, ... */
 template <int TW, int TH, int NTH>
 CRAW_DEV void awb_blocks(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0, int y0, const float *rgb,
                          int t)
 {
     constexpr int P = TW * TH;
-    const int blocks_x = (k.width + 7) / 8;
     for (int b = t; b < (TW / 8) * (TH / 8); b += NTH) {
         int bx = b % (TW / 8), by = b / (TW / 8);
         if (x0 + bx * 8 >= k.width || y0 + by * 8 >= k.height)
@@ -763,13 +761,9 @@ CRAW_DEV void awb_blocks(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int x0
                 }
         }
         float n = (float)(xe * ye);
-        const size_t ri = (size_t)(y0 / 8 + by) * blocks_x + x0 / 8 + bx;
-        if (!craw_in_bounds(ri < craw_awb_blocks(k.width, k.height), io.err))
-            continue;
-        io.awb.rec[ri] =
-            craw_awb_block(__fdiv_rn(s0, n), __fdiv_rn(s1, n), __fdiv_rn(s2, n), k.awb_wb,
-                           io.awb.deferred, io.awb.nb_deferred,
-                           craw_awb_blocks(k.width, k.height));
+        craw_awb_add(io.awb.hist, craw_awb_block(__fdiv_rn(s0, n), __fdiv_rn(s1, n), __fdiv_rn(s2, n), k.awb_wb,
+                                                 io.awb.deferred, io.awb.nb_deferred,
+                                                 craw_awb_blocks(k.width, k.height)));
     }
 }
 

@@ -131,7 +131,6 @@ struct WalkSmem {
     alignas(16) float a[8][3][PITCH];
     float sum[HOLD * NB][3];
     float cnt[HOLD * NB];
-    int where[HOLD * NB];
     CRAW_DEV static int col(int x) { return x + 4 * (x >> 5); }
 };
 
@@ -285,23 +284,22 @@ struct WalkOut {
                         t = __fadd_rn(t, s.a[j][c][S::col(8 * b) + i]);
             }
             s.sum[held + b][c] = t;
-            if (c == 0) {
+            if (c == 0)
                 s.cnt[held + b] = (float)(w * rows);
-                s.where[held + b] = (qy + r) / 4 * ((k.width + 7) / 8) + qx / 4 + b;
-            }
         }
         held += (2 * nout + 7) / 8;
         __syncwarp();
         if (!last && held + S::NB <= S::HOLD * S::NB)
             return;
+        uint64_t rec = 0;
         if (lane < held) {
             const float n = s.cnt[lane];
-            const int ri = s.where[lane];
-            if (craw_in_bounds(ri >= 0 && (uint32_t)ri < craw_awb_blocks(k.width, k.height), io.err))
-                io.awb.rec[ri] = craw_awb_block(__fdiv_rn(s.sum[lane][0], n), __fdiv_rn(s.sum[lane][1], n),
-                                                __fdiv_rn(s.sum[lane][2], n), k.awb_wb, io.awb.deferred,
-                                                io.awb.nb_deferred, craw_awb_blocks(k.width, k.height));
+            rec = craw_awb_block(__fdiv_rn(s.sum[lane][0], n), __fdiv_rn(s.sum[lane][1], n),
+                                 __fdiv_rn(s.sum[lane][2], n), k.awb_wb, io.awb.deferred, io.awb.nb_deferred,
+                                 craw_awb_blocks(k.width, k.height));
         }
+        __syncwarp();
+        craw_awb_add(io.awb.hist, rec);
         held = 0;
         __syncwarp();
     }
@@ -330,7 +328,7 @@ struct WalkOut {
                 return;
             }
         }
-        if (io.awb.rec && mine) {
+        if (io.awb.hist && mine) {
             float *a = &s.a[2 * (r & 3)][0][S::col(2 * (lane - A))];
 #pragma unroll
             for (int b = 0; b < 2; b++)
@@ -344,7 +342,7 @@ struct WalkOut {
             store(dst, io.dst_pitch, fmt(), r, o);
             dst += 2 * io.dst_pitch;
         }
-        if (io.awb.rec && ((r & 3) == 3 || last))
+        if (io.awb.hist && ((r & 3) == 3 || last))
             awb_rows(r, 2 * (r & 3) + 2, last);
     }
 };
@@ -598,7 +596,7 @@ struct LinearWalk {
     bool inside, partial;    /* the lane's four columns are in the frame; its first two only */
     bool mine, right;        /* an output lane; the second of its AWB block */
     float as[3], hs[3];      /* the AWB block's sums so far; the block's above, waiting */
-    int held;                /* whether hs waits: then its row of blocks + 1 */
+    bool held;               /* whether hs waits */
     float qs[3];             /* chroma: the sums of the 4x4 block so far */
     char *dst, *inter;       /* the lane's pixels in the row to store next */
 
@@ -720,16 +718,17 @@ struct LinearWalk {
                             __fdiv_rn(qs[2], n));
     }
 
-    /* The statistic of the block whose sums are s, of `rows` pixel rows in
-     * block row `by`, on the lanes that `go`. */
-    CRAW_DEV void statistic(const float s[3], int by, int rows, bool go)
+    /* The statistic of the block whose sums are s, of `rows` pixel rows, on
+     * the lanes that `go`. */
+    CRAW_DEV void statistic(const float s[3], int rows, bool go)
     {
-        const int bx = x0 >> 3, nx = min(8, k.width - 8 * bx);
-        const float n = (float)(nx * rows);
-        const int ri = by * ((k.width + 7) / 8) + bx;
-        if (go && craw_in_bounds(ri >= 0 && (uint32_t)ri < craw_awb_blocks(k.width, k.height), io.err))
-            io.awb.rec[ri] = craw_awb_block(__fdiv_rn(s[0], n), __fdiv_rn(s[1], n), __fdiv_rn(s[2], n), k.awb_wb,
-                                            io.awb.deferred, io.awb.nb_deferred, craw_awb_blocks(k.width, k.height));
+        const float n = (float)(min(8, k.width - (x0 & ~7)) * rows);
+        uint64_t rec = 0;
+        if (go)
+            rec = craw_awb_block(__fdiv_rn(s[0], n), __fdiv_rn(s[1], n), __fdiv_rn(s[2], n), k.awb_wb,
+                                 io.awb.deferred, io.awb.nb_deferred, craw_awb_blocks(k.width, k.height));
+        __syncwarp();
+        craw_awb_add(io.awb.hist, rec);
     }
 
     /* The AWB sums of a row, in the reference's order (lib/awb.c:239-253):
@@ -753,12 +752,11 @@ struct LinearWalk {
         }
         if (!odd || ((y & 7) != 7 && !end))
             return;
-        const int by = y >> 3;
         if (!held && !end) {
 #pragma unroll
             for (int c = 0; c < 3; c++)
                 hs[c] = as[c];
-            held = by + 1;
+            held = true;
         } else {
             float s[3];
 #pragma unroll
@@ -766,9 +764,9 @@ struct LinearWalk {
                 const float above = walk_left(hs[c]);
                 s[c] = right ? above : as[c];
             }
-            statistic(s, right ? held - 1 : by, right ? 8 : (y & 7) + 1,
+            statistic(s, right ? 8 : (y & 7) + 1,
                       right ? held && x0 - LW_P < k.width && mine_pair() : mine);
-            held = 0;
+            held = false;
         }
         as[0] = as[1] = as[2] = 0.0f;
     }
@@ -799,7 +797,7 @@ struct LinearWalk {
             quarter(y, end, odd, o);
             return;
         }
-        if (io.awb.rec)
+        if (io.awb.hist)
             awb_row(y, end, odd, o);
         if (!ANY || io.dst) {
             walk_colour<-1>(k.color, mine, o);
@@ -823,7 +821,7 @@ struct LinearWalk {
         mine = lane >= 1 && lane <= LW_N && x0 < k.width;
         right = !(lane & 1);
         nv = min(LW_P, k.width - x0);
-        held = 0;
+        held = false;
 #pragma unroll
         for (int c = 0; c < 3; c++)
             as[c] = hs[c] = qs[c] = 0.0f;
