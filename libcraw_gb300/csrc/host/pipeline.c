@@ -56,15 +56,18 @@ static const char *const plain_stage_names[ST_NB] = {
 
 /* One AWB slot: the three histograms, the count of deferred blocks and the
  * blocks themselves. On the device room for every 8x8 block of the frame; on
- * the host, pinned, the first CRAW_K_AWB_DEFER_MAX of them, filled by one
- * async copy (a count above that is read from the device on demand). The
- * device's histograms and count are zeroed by one fill before the frame. */
+ * the host, pinned, the first CRAW_K_AWB_DEFER_MAX of them (a count above
+ * that is read from the device on demand). A frame's last kernel fills the
+ * host copy and leaves the device's histograms and count zeroed for the
+ * slot's next frame; after a recording that failed on the way they are
+ * zeroed by a fill. */
 #define ZERO_BYTES (HIST_BYTES + 16)
 #define SLOT_BYTES (ZERO_BYTES + DEFER_BYTES)
 struct awb_slot {
     uint8_t *host;            /* SLOT_BYTES */
     uint8_t *dev;             /* the same layout, max(nb_blocks, CRAW_K_AWB_DEFER_MAX) entries */
     bool folded;              /* deferred blocks already binned */
+    bool dirty;               /* the device's part is not zeros */
 };
 
 struct prof_slot {
@@ -556,6 +559,10 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
                 goto fail;
             }
             memset(p->slots[i].host, 0, SLOT_BYTES);
+            if (cudaMemsetAsync(p->slots[i].dev, 0, ZERO_BYTES, ctx->stream) != cudaSuccess) {
+                ret = CRAW_ERROR(EIO);
+                goto fail;
+            }
         }
     }
     if ((ret = craw_dev_alloc(ctx, (void **)&p->kerr, 16)) < 0)
@@ -738,13 +745,15 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
     }
 
     CRAWKAwbOut awb = { 0 };
+    struct awb_slot *slot = &p->slots[p->nb_recorded % p->nb_slots];
     if (p->awb) {
-        uint8_t *dev = p->slots[p->nb_recorded % p->nb_slots].dev;
+        uint8_t *dev = slot->dev;
         awb.hist = (uint32_t *)dev;
         awb.nb_deferred = (uint32_t *)(dev + HIST_BYTES);
         awb.deferred = (CRAWKAwbDeferred *)(dev + ZERO_BYTES);
-        if (cudaMemsetAsync(dev, 0, ZERO_BYTES, s) != cudaSuccess)
+        if (slot->dirty && cudaMemsetAsync(dev, 0, ZERO_BYTES, s) != cudaSuccess)
             return CRAW_ERROR(EIO);
+        slot->dirty = true;
     }
 
     mosaic = src->data;
@@ -880,17 +889,14 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
     }
 
     if (p->awb) {
-        struct awb_slot *slot = &p->slots[p->nb_recorded % p->nb_slots];
-        cudaError_t e;
         if (!p->plain)
             prof_begin(&pc, ST_AWB);
-        e = cudaMemcpyAsync(slot->host, slot->dev, SLOT_BYTES, cudaMemcpyDeviceToHost, s);
+        ret = craw_k_awb_publish(&awb, slot->host, slot->host + HIST_BYTES, slot->host + ZERO_BYTES, s);
         if (!p->plain)
             prof_end(&pc);
-        if (e != cudaSuccess) {
-            ret = CRAW_ERROR(EIO);
+        if (ret < 0)
             goto launch_fail;
-        }
+        slot->dirty = false;
         slot->folded = false;
         p->nb_recorded++;
     }

@@ -190,9 +190,10 @@ typedef struct CRAWKAwbDeferred {
 } CRAWKAwbDeferred;
 
 typedef struct CRAWKAwbOut {
-    uint32_t *hist;                /* three 128^2 histograms, zeroed before the frame; or NULL */
+    uint32_t *hist;                /* three 128^2 histograms, zeros before the frame; or NULL */
     CRAWKAwbDeferred *deferred;    /* room for one entry per 8x8 block of the frame */
-    uint32_t *nb_deferred;         /* counter, zeroed before the frame */
+    uint32_t *nb_deferred;         /* counter, zero before the frame; then a word for
+                                    * craw_k_awb_publish, zero too */
 } CRAWKAwbOut;
 
 /* Layouts of an RGB image a kernel stores: four floats (alpha 1), four
@@ -259,6 +260,14 @@ int craw_k_chroma_up_color(const CRAWKDevelop *k, const CRAWKChroma *c,
                            const void *q, const void *qf, size_t q_pitch,
                            void *dst, size_t dst_pitch, int dst_fmt,
                            void *inter_out, const CRAWKAwbOut *awb, cudaStream_t s);
+
+/* ---------------------------------------------------------------- awb */
+
+/* After the frame's kernels: the histograms, the count of deferred blocks
+ * and the first CRAW_K_AWB_DEFER_MAX of them into pinned host memory (16-byte
+ * aligned), and the device's histograms and count back to zeros. */
+int craw_k_awb_publish(const CRAWKAwbOut *awb, void *host_hist, void *host_head, void *host_deferred,
+                       cudaStream_t s);
 
 /* ------------------------------------------------------ highlights */
 
