@@ -1,10 +1,9 @@
 /*
  * Noise-model estimation (reference lib/noise.c:125-504). The frame is
  * binned on the GPU (kernels/noise.cu): per bin the count, the exact sum
- * of the 9x9 means and the median |high-pass|. The least-trimmed-squares
- * cost of every pair of bins is evaluated on the GPU too, one warp per
- * pair; the host picks the seed in the reference's order, re-measures the
- * chosen pair's cost with its own log, and runs the reweighted
+ * of the 9x9 means and the median |high-pass|. The pair of bins of the least
+ * least-trimmed-squares cost, the seed, is found on the GPU too; the host
+ * re-measures the pair's cost with its own log, and runs the reweighted
  * Gauss-Newton refinement (40 steps of a few hundred logs at most).
  */
 #include <errno.h>
@@ -74,8 +73,8 @@ static int ne_cmp_d(const void *a, const void *b)
 /* The bins the fit uses: level, variance, sample count, ln variance. */
 typedef struct NeBins {
     int nb;
-    double m[CRAW_NOISE_MAX_BINS], v[CRAW_NOISE_MAX_BINS], c[CRAW_NOISE_MAX_BINS];
-    double lv[CRAW_NOISE_MAX_BINS];
+    double m[CRAW_NOISE_MAX_BINS], v[CRAW_NOISE_MAX_BINS], lv[CRAW_NOISE_MAX_BINS];   /* copied as one */
+    double c[CRAW_NOISE_MAX_BINS];
 } NeBins;
 
 /* Bins with at least min_n samples and a positive spread (reference
@@ -197,14 +196,16 @@ static int ne_run(const CRAWKNoise *k, const void *src, size_t pitch, uint32_t m
     const size_t scratch = craw_k_noise_scratch(k->width, k->height, nbins);
     const size_t bins_at = (scratch + 255) / 256 * 256;
     const size_t fit_at = bins_at + (size_t)CRAW_K_NOISE_MAX_BINS * sizeof(CRAWKNoiseBin);
-    const size_t cost_at = fit_at + (size_t)3 * CRAW_NOISE_MAX_BINS * sizeof(double);
-    const size_t total = cost_at + (size_t)CRAW_NOISE_MAX_BINS * CRAW_NOISE_MAX_BINS * sizeof(double);
+    const size_t lts_at = fit_at + (size_t)3 * CRAW_NOISE_MAX_BINS * sizeof(double);
+    const size_t best_at = (lts_at + craw_k_noise_lts_scratch(nbins) + 255) / 256 * 256;
+    const size_t total = best_at + 2 * sizeof(int32_t);
     CRAWKNoiseBin *kb = malloc((size_t)nbins * sizeof(*kb));
-    NeBins *B = malloc(sizeof(*B));
-    double *cost = NULL, *work = malloc(2 * CRAW_NOISE_MAX_BINS * sizeof(double));
+    NeBins *B = calloc(1, sizeof(*B));
+    double *work = malloc(2 * CRAW_NOISE_MAX_BINS * sizeof(double));
     char *dev = NULL;
-    int ret = 0, nb, keep, bi = -1, bj = -1;
-    double a = 0.0, b = 0.0, best = INFINITY, scale, rms = 0.0, range0;
+    int32_t pair[2] = { -1, -1 };
+    int ret = 0, nb, keep;
+    double a = 0.0, b = 0.0, best, scale, rms = 0.0, range0;
     uint32_t nin = 0;
 
     if (!kb || !B || !work) {
@@ -234,34 +235,21 @@ static int ne_run(const CRAWKNoise *k, const void *src, size_t pitch, uint32_t m
 
     /* Every pair's cost on the device; the seed is the first pair, in
      * the reference's (i, j) order, whose cost is strictly the least. */
-    if (!(cost = malloc((size_t)nb * nb * sizeof(*cost)))) {
-        ret = CRAW_ERROR(ENOMEM);
-        goto done;
-    }
     {
         double *dm = (double *)(dev + fit_at), *dv = dm + CRAW_NOISE_MAX_BINS, *dl = dv + CRAW_NOISE_MAX_BINS;
-        double *dc = (double *)(dev + cost_at);
-        if ((ret = ne_cuda_err(cudaMemcpyAsync(dm, B->m, nb * sizeof(double), cudaMemcpyHostToDevice, s))) < 0 ||
-            (ret = ne_cuda_err(cudaMemcpyAsync(dv, B->v, nb * sizeof(double), cudaMemcpyHostToDevice, s))) < 0 ||
-            (ret = ne_cuda_err(cudaMemcpyAsync(dl, B->lv, nb * sizeof(double), cudaMemcpyHostToDevice, s))) < 0)
+        int32_t *db = (int32_t *)(dev + best_at);
+        if ((ret = ne_cuda_err(cudaMemcpyAsync(dm, B->m, (size_t)3 * CRAW_NOISE_MAX_BINS * sizeof(double),
+                                               cudaMemcpyHostToDevice, s))) < 0)
             goto done;
-        if (craw_k_noise_lts(dm, dv, dl, nb, keep, dc, s) < 0) {
+        if (craw_k_noise_lts(dm, dv, dl, nb, keep, dev + lts_at, db, s) < 0) {
             ret = CRAW_ERROR(EIO);
             goto done;
         }
-        if ((ret = ne_cuda_err(cudaMemcpyAsync(cost, dc, (size_t)nb * nb * sizeof(double),
-                                               cudaMemcpyDeviceToHost, s))) < 0 ||
+        if ((ret = ne_cuda_err(cudaMemcpyAsync(pair, db, sizeof(pair), cudaMemcpyDeviceToHost, s))) < 0 ||
             (ret = ne_cuda_err(cudaStreamSynchronize(s))) < 0)
             goto done;
     }
-    for (int i = 0; i < nb; i++)
-        for (int j = i + 1; j < nb; j++)
-            if (cost[(size_t)i * nb + j] < best) {
-                best = cost[(size_t)i * nb + j];
-                bi = i;
-                bj = j;
-            }
-    if (bi < 0 || !ne_pair(B, bi, bj, &a, &b) || !(a > 0.0)) {
+    if (pair[0] < 0 || !ne_pair(B, pair[0], pair[1], &a, &b) || !(a > 0.0)) {
         ret = CRAW_ERROR(ENODATA);
         goto done;
     }
@@ -293,7 +281,6 @@ done:
         if (cudaStreamSynchronize(s) != cudaSuccess && ret == 0)
             ret = CRAW_ERROR(EIO);
     }
-    free(cost);
     free(work);
     free(B);
     free(kb);

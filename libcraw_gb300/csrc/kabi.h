@@ -329,14 +329,16 @@ size_t craw_k_noise_scratch(int32_t width, int32_t height, int32_t nb_bins);
 int craw_k_noise_bins(const CRAWKNoise *k, const uint16_t *src, size_t src_pitch, void *scratch,
                       CRAWKNoiseBin *bins, cudaStream_t s);
 
-/* The least-trimmed-squares cost of the line through every pair of bins
- * i < j (the sum of the `keep` smallest squared log residuals, added in
- * ascending order): cost[i * nb + j], +inf where the pair gives no
- * physical line. m, v: the bins' mean level and variance; lv = ln v,
- * computed on the host. All device arrays; nb <= CRAW_K_NOISE_MAX_BINS. */
+/* The pair of bins i < j through whose line the least-trimmed-squares cost
+ * (the sum of the `keep` smallest squared log residuals, added in ascending
+ * order) is least, the first of equals in (i, j) order, into best (device
+ * memory); -1, -1 where no pair gives a physical line. m, v: the bins' mean
+ * level and variance; lv = ln v, computed on the host. All device arrays;
+ * nb <= CRAW_K_NOISE_MAX_BINS; scratch: craw_k_noise_lts_scratch(nb) bytes. */
 #define CRAW_K_NOISE_MAX_BINS 512
+size_t craw_k_noise_lts_scratch(int32_t nb);
 int craw_k_noise_lts(const double *m, const double *v, const double *lv, int32_t nb, int32_t keep,
-                     double *cost, cudaStream_t s);
+                     void *scratch, int32_t best[2], cudaStream_t s);
 
 /* ------------------------------------------------------------- batch */
 
