@@ -1,7 +1,7 @@
 /*
- * The fused develop kernels (tile bodies in develop_tile.cuh): prep +
- * debayer + colour + AWB statistic in one launch, with the RCD's interior
- * tiles done by CFA quads and the rest per pixel; and their launcher.
+ * The fused develop kernels (walking warps in develop_walk.cuh, tile bodies
+ * in develop_tile.cuh): prep + debayer + colour + AWB statistic in one launch,
+ * the RCD's interior and its border in one each; and their launcher.
  */
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -13,8 +13,8 @@
 
 /* Whether the RCD interior tiles load their mosaic by TMA (1, the
  * default) or by plain loads (0, for comparison and tests); whether the
- * interior runs by 64x16 tiles (0, for comparison and tests) or by walking
- * strips (1, the default; 2). */
+ * frame runs by 64x16 tiles with a per-pixel border (0, for comparison and
+ * tests) or by walking warps (1, the default; 2). */
 extern "C" {
 int craw_k_rcd_tma = 1;
 int craw_k_rcd_strips = 1;
@@ -70,11 +70,16 @@ struct QuadGrid {
 
 /* An interior kernel lets the border launch that follows it on the stream
  * begin at once (programmatic dependent launch): the two write disjoint
- * tiles, and the border CTAs take the SM slots that the interior's last
- * wave leaves idle. The launches after the border wait for both as usual. */
+ * tiles, and the border CTAs take the SM slots that the interior leaves
+ * free. The border ends no earlier than the interior, so that what comes
+ * after it on the stream, or depends on it in a graph, waits for both. */
 CRAW_DEV void release_border()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+CRAW_DEV void await_interior()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 __global__ void __launch_bounds__(QNT)
@@ -141,6 +146,17 @@ k_develop_rcd_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid
     rcd_walk<FMT, RGC, MORE>(k, io, g, blockIdx.x * WALK_WARPS + warp, smem[warp]);
 }
 
+/* The border by walking warps, in the same CTAs. */
+template <int FMT, bool RGC, bool MORE>
+__global__ void __launch_bounds__(WALK_NT, WALK_CTAS)
+k_develop_rcd_ring(const CRAWKDevelop k, const CRAWKDevelopIO io, const __grid_constant__ RingGrid ring)
+{
+    __shared__ WalkSmem<RW_NQ> smem[WALK_WARPS];
+    const int warp = threadIdx.x >> 5;
+    ring_walk<FMT, RGC, MORE>(k, io, ring, blockIdx.x * WALK_WARPS + warp, smem[warp]);
+    await_interior();
+}
+
 /* The per-pixel RCD on the ring of border quad tiles, BTW x BTH pixels a
  * CTA (QTW / BTW of them a quad tile). */
 __global__ void __launch_bounds__(256, 8)
@@ -152,9 +168,9 @@ k_develop_rcd_border(const CRAWKDevelop k, const CRAWKDevelopIO io, const QuadGr
     int col, row;
     g.border(blockIdx.x / PER, col, row);
     const int x0 = col * QTW + (blockIdx.x % PER) * BTW, y0 = row * QTH;
-    if (x0 >= k.width)
-        return;
-    pixel_tile<kRcd, BTW, BTH, 256>(k, io, x0, y0, smem);
+    if (x0 < k.width)
+        pixel_tile<kRcd, BTW, BTH, 256>(k, io, x0, y0, smem);
+    await_interior();
 }
 
 /* Every bilinear and MHC frame: CTAs an SM (5 of 96 registers for MHC and 6
@@ -204,6 +220,63 @@ unsigned walk_segments(WalkGrid &g, int ctas, int least)
     return (unsigned)((warps + WALK_WARPS - 1) / WALK_WARPS);
 }
 
+/* A part of the frame, in quads, as strips; false if it is empty. */
+bool walk_part(WalkGrid &g, int x0, int x1, int y0, int y1)
+{
+    g.qx0 = x0;
+    g.nqx = x1 - x0;
+    g.qy0 = y0;
+    g.nqy = y1 - y0;
+    g.nx = (g.nqx + RW_NQ - 1) / RW_NQ;
+    return g.nqx > 0 && g.nqy > 0;
+}
+
+/* Segments of at most `most` quad rows, alike; returns the part's warps. */
+int walk_cut(WalkGrid &g, int most)
+{
+    const int n = (g.nqy + most - 1) / most;
+    g.seg = 4 * (((g.nqy + 3) / 4 + n - 1) / n);
+    return g.nx * ((g.nqy + g.seg - 1) / g.seg);
+}
+
+/* The RCD of a w x h frame as strips: the interior's (w, its CTAs in inner;
+ * none if the frame has none) and the border's. Segments are a multiple of 4
+ * quad rows, at least 8. Either the interior takes one wave of WALK_CTAS
+ * CTAs an SM and the border, in segments as short as one wave of it allows,
+ * the next; or both share a wave, the border in segments half as long as the
+ * interior's (its steps take longer). A segment of n rows takes n + 6 steps,
+ * n + 5 in the border: the fewer in all. Frame times, sharing against taking
+ * turns: 115 and 124 us (1920x1080, denoise with history, AP0), 280 and 284
+ * (3840x2160, denoise); 737 and 706 (5760x3240, exact denoise, AP1). */
+void rcd_grids(int width, int height, const QuadGrid &q, WalkGrid &w, RingGrid &ring, int &inner, int &border)
+{
+    const int w2 = width / 2, h2 = height / 2, room = craw_sm_count() * WALK_CTAS;
+    const bool in = q.interior_x() > 0 && q.interior_y() > 0;
+    const int x0 = in ? q.c_lo * (QTW / 2) : w2, x1 = in ? (q.c_hi + 1) * (QTW / 2) : w2;
+    const int y0 = in ? q.r_lo * (QTH / 2) : h2, y1 = in ? (q.r_hi + 1) * (QTH / 2) : h2;
+    walk_part(w, x0, x1, y0, y1);
+    const bool any[4] = { walk_part(ring.g[0], 0, w2, 0, y0), walk_part(ring.g[1], 0, w2, y1, h2),
+                          walk_part(ring.g[2], 0, x0, y0, y1), walk_part(ring.g[3], x1, w2, y0, y1) };
+    auto ctas = [](int warps) { return (warps + WALK_WARPS - 1) / WALK_WARPS; };
+    auto cut_ring = [&](int most) {
+        ring.first[0] = 0;
+        for (int i = 0; i < 4; i++)
+            ring.first[i + 1] = ring.first[i] + (any[i] ? walk_cut(ring.g[i], most) : 0);
+        return ctas(ring.first[4]);
+    };
+    int turn = 8, turn_ring = 8, both = 8;
+    while (turn < h2 && in && ctas(walk_cut(w, turn)) > room)
+        turn += 4;
+    while (turn_ring < h2 && cut_ring(turn_ring) > room)
+        turn_ring += 4;
+    auto half = [](int n) { return n / 8 * 4 > 8 ? n / 8 * 4 : 8; };
+    while (both < h2 && in && ctas(walk_cut(w, both)) + cut_ring(half(both)) > room)
+        both += 4;
+    const bool share = in && both + 6 < turn + 6 + turn_ring + 5;
+    inner = in ? ctas(walk_cut(w, share ? both : turn)) : 0;
+    border = cut_ring(share ? half(both) : turn_ring);
+}
+
 template <int METHOD, int EPI>
 int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
 {
@@ -243,19 +316,54 @@ int prepare_rcd()
     return 0;
 }
 
-/* The walking kernel for a frame's output. */
-auto walk_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io)
+/* The border's launch after an interior launch (`after`), which it may
+ * overlap, or by itself. */
+template <typename... P, typename... A>
+int launch_border(void (*kernel)(P...), int ctas, int threads, size_t smem, bool after, cudaStream_t s, const A &...args)
 {
-    const bool rgc = k->color.flags & CRAW_K_COLOR_RGC;
-    if (k->fp16 || io->inter || io->quarter || !io->dst)
-        return k_develop_rcd_walk<0, false, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute early[1];
+    early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = early;
+    cfg.numAttrs = after ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess && cfg.numAttrs) {
+        /* A driver that refuses the early start: the plain launch after the
+         * interior, the launch's own error cleared. */
+        (void)cudaGetLastError();
+        cfg.numAttrs = 0;
+        (void)cudaLaunchKernelEx(&cfg, kernel, args...);
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+}
+
+/* The walking kernels of a frame. */
+template <int FMT, bool RGC, bool MORE>
+int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, const QuadGrid &g, cudaStream_t s)
+{
+    WalkGrid w;
+    RingGrid ring;
+    int inner, border;
+    rcd_grids(k->width, k->height, g, w, ring, inner, border);
+    if (inner > 0) {
+        k_develop_rcd_walk<FMT, RGC, MORE><<<inner, WALK_NT, 0, s>>>(*k, *io, w);
+        if (cudaGetLastError() != cudaSuccess)
+            return -5;
+    }
+    return launch_border(k_develop_rcd_ring<FMT, RGC, MORE>, border, WALK_NT, 0, inner > 0, s, *k, *io, ring);
+}
+
+template <bool RGC>
+int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, const QuadGrid &g, cudaStream_t s)
+{
     switch (io->dst_fmt) {
-    case CRAW_K_OUT_RGBA16F:
-        return rgc ? k_develop_rcd_walk<CRAW_K_OUT_RGBA16F, true, false> : k_develop_rcd_walk<CRAW_K_OUT_RGBA16F, false, false>;
-    case CRAW_K_OUT_RGB32F:
-        return rgc ? k_develop_rcd_walk<CRAW_K_OUT_RGB32F, true, false> : k_develop_rcd_walk<CRAW_K_OUT_RGB32F, false, false>;
-    default:
-        return rgc ? k_develop_rcd_walk<CRAW_K_OUT_RGBA32F, true, false> : k_develop_rcd_walk<CRAW_K_OUT_RGBA32F, false, false>;
+    case CRAW_K_OUT_RGBA16F: return launch_walk<CRAW_K_OUT_RGBA16F, RGC, false>(k, io, g, s);
+    case CRAW_K_OUT_RGB32F:  return launch_walk<CRAW_K_OUT_RGB32F, RGC, false>(k, io, g, s);
+    default:                 return launch_walk<CRAW_K_OUT_RGBA32F, RGC, false>(k, io, g, s);
     }
 }
 
@@ -266,19 +374,13 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
         return -5;
     QuadGrid g;
     g.init(k->width, k->height);
-    if (g.interior_x() > 0 && g.interior_y() > 0 && craw_k_rcd_strips) {
-        /* The interior tiles' region by walking warps. */
-        WalkGrid w;
-        w.qx0 = g.c_lo * (QTW / 2);
-        w.nqx = g.interior_x() * (QTW / 2);
-        w.qy0 = g.r_lo * (QTH / 2);
-        w.nqy = g.interior_y() * (QTH / 2);
-        w.nx = (w.nqx + RW_NQ - 1) / RW_NQ;
-        const unsigned ctas = walk_segments(w, WALK_CTAS, 8);
-        walk_rcd(k, io)<<<ctas, WALK_NT, 0, s>>>(*k, *io, w);
-        if (cudaGetLastError() != cudaSuccess)
-            return -5;
-    } else if (g.interior_x() > 0 && g.interior_y() > 0) {
+    if (craw_k_rcd_strips) {
+        if (k->fp16 || io->inter || io->quarter || !io->dst)
+            return launch_walk<0, false, true>(k, io, g, s);
+        return k->color.flags & CRAW_K_COLOR_RGC ? launch_walk<true>(k, io, g, s) : launch_walk<false>(k, io, g, s);
+    }
+    const bool interior = g.interior_x() > 0 && g.interior_y() > 0;
+    if (interior) {
         const dim3 grid(g.interior_x(), g.interior_y());
         CUtensorMap tmap;
         if (craw_k_rcd_tma && craw_tmap_u16(io->src, io->src_pitch, k->width, k->height, kBoxW, kBoxH, &tmap))
@@ -288,30 +390,10 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
         if (cudaGetLastError() != cudaSuccess)
             return -5;
     }
-    if (g.border_quads() > 0) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(g.border_quads() * (QTW / BTW)));
-        cfg.blockDim = dim3(256);
-        cfg.dynamicSmemBytes = PixelSmem<kRcd, BTW, BTH, 256>::floats * sizeof(float);
-        cfg.stream = s;
-        cudaLaunchAttribute early[1];
-        early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        early[0].val.programmaticStreamSerializationAllowed = 1;
-        /* After an interior launch only: it is the launch the border may
-         * overlap. */
-        cfg.attrs = early;
-        cfg.numAttrs = g.interior_x() > 0 && g.interior_y() > 0 ? 1 : 0;
-        if (cudaLaunchKernelEx(&cfg, k_develop_rcd_border, *k, *io, g) != cudaSuccess && cfg.numAttrs) {
-            /* A driver that refuses the early start: the plain launch
-             * after the interior, the launch's own error cleared. */
-            (void)cudaGetLastError();
-            cfg.numAttrs = 0;
-            (void)cudaLaunchKernelEx(&cfg, k_develop_rcd_border, *k, *io, g);
-        }
-        if (cudaGetLastError() != cudaSuccess)
-            return -5;
-    }
-    return 0;
+    return g.border_quads() > 0 ? launch_border(k_develop_rcd_border, g.border_quads() * (QTW / BTW), 256,
+                                                PixelSmem<kRcd, BTW, BTH, 256>::floats * sizeof(float), interior, s,
+                                                *k, *io, g)
+                                : 0;
 }
 
 } // namespace

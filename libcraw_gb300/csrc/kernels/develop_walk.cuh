@@ -376,6 +376,38 @@ CRAW_DEV float2 walk_prep(const CRAWKDevelop &k, const CRAWKDevelopIO &io, uint3
  * feed values nothing reads. */
 constexpr int RW_NQ = 24, RW_A = 4;
 
+/* The weights, and the colours at a green site, with the roundings of the
+ * per-pixel tiles (RcdTile), where the two forms differ. */
+CRAW_DEV float rp_wv(float4 s)
+{
+    const float hs = __fmul_rn(s.y, 1.0f / 9.0f);
+    return __fmul_rn(hs, rq_rcp(__fadd_rn(__fmaf_rn(s.x, 1.0f / 9.0f, hs), RCD_EPS)));
+}
+CRAW_DEV float rp_wp(float4 s)
+{
+    const float qs = __fmul_rn(s.w, 1.0f / 9.0f);
+    return __fmul_rn(qs, rq_rcp(__fadd_rn(__fmaf_rn(s.z, 1.0f / 9.0f, qs), RCD_EPS)));
+}
+CRAW_DEV void rp_green_site(float wt, float g00, float dh0, float dh1, float ev0, float ev1, float dv0,
+                            float dv1, float eh0, float eh1, float &ch, float &cv)
+{
+    ch = __fmaf_rn(__fsub_rn(1.0f, wt), rq_half_sum(g00, dh0, dh1), __fmul_rn(wt, rq_half_sum(g00, ev0, ev1)));
+    cv = rq_blend(wt, rq_half_sum(g00, dv0, dv1), rq_half_sum(g00, eh0, eh1));
+}
+CRAW_DEV float4 walk_left4(float4 v)
+{
+    return make_float4(walk_left(v.x), walk_left(v.y), walk_left(v.z), walk_left(v.w));
+}
+CRAW_DEV float4 walk_right4(float4 v)
+{
+    return make_float4(walk_right(v.x), walk_right(v.y), walk_right(v.z), walk_right(v.w));
+}
+/* s + a + b + c in that order. */
+CRAW_DEV float4 rp_add3(float4 s, float4 a, float4 b, float4 c)
+{
+    return rq_add4(rq_add4(rq_add4(s, a), b), c);
+}
+
 struct RcdWalk {
     float v[6][6];                    /* pixel rows 2s-2 .. 2s+3, columns X-2 .. X+3 (X: the lane's R) */
     float q2[4], q3[4];               /* the quads of rows s-2, s-3: R, Gr, Gb, B */
@@ -489,6 +521,225 @@ struct RcdWalk {
         c3 = c2;
     }
 };
+
+/* The same on the frame's border, the ring of 64x16 tiles that touch it, in
+ * the per-pixel tiles' arithmetic (the rp_* helpers where it differs; the 3x3 sums of D one
+ * term after another). Outside the frame every array of the RCD holds the
+ * value of the position that mirrors there, so:
+ *   a column outside is one that the lane at the edge, or its neighbour,
+ *   has (left: column -1 is 1, -2 is 2; right: w is w - 2, w + 1 is w - 3);
+ *   the quad row above the first gives the first's second row (and its low
+ *   pass two rows up is the one two rows down); the quad row below the last
+ *   gives the last's first row.
+ *
+ * Bound: the chain of a step (1.4 us with a warp or two a scheduler). The
+ * border by 32x16 tiles of a pixel a thread (920 instructions a pixel, a third
+ * of them addresses and mirrored positions) took 26 us after the interior of
+ * a 5760x3240 frame and 13 after a 1920x1080 one's; its warps take 21 and 15
+ * by themselves, and where they share the interior's wave next to nothing.
+ * In the interior's own launch they cost its code registers: 745 against
+ * 706 us a 5760x3240 frame. */
+struct RingWalk {
+    float v[6][6];                    /* as RcdWalk's */
+    float q2[4], q3[4];
+    float2 l1, l2;
+    float4 t[2], rr[2];               /* row 2s-1: the 3x3 sums' first six terms; its own three */
+    float4 d0[4];                     /* D of pixel row 2s-2: the left column's, the quad's two, the right's */
+    float wv0, wp0, wg0;              /* weights of pixel row 2s-2: at R vertical and diagonal, at Gr */
+    float2 wg2, wg3, wp2, g2, g3;
+    float kr2, kr3, krr2, krr3;
+    float kb2, kb3, kb4, kbl2, kbl3;
+    float jr3, jrr3, jb3, jb4, jbl3;
+    float2 c3;
+
+    CRAW_DEV void rows(float2 a, float2 b, bool first, bool last)
+    {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const float2 x = i ? b : a;
+            const float lx = walk_left(x.x), ly = walk_left(x.y), rx = walk_right(x.x), ry = walk_right(x.y);
+            v[4 + i][0] = first ? rx : lx;
+            v[4 + i][1] = first ? x.y : ly;
+            v[4 + i][2] = x.x;
+            v[4 + i][3] = x.y;
+            v[4 + i][4] = last ? x.x : rx;
+            v[4 + i][5] = last ? ly : ry;
+        }
+    }
+
+    /* Step s, `row` its quad row in the frame of h2; first, last: the lane's
+     * column is the frame's first, last. o: the pixels of row - 3. */
+    CRAW_DEV void step(int row, int h2, bool first, bool last, float o[2][2][3])
+    {
+        /* D, L of `row`. */
+        float lo[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int y = 2 + e, x = 2 + e;
+            lo[e] = rq_lowpass(v[y][x], v[y - 1][x], v[y + 1][x], v[y][x - 1], v[y][x + 1], v[y - 1][x - 1],
+                               v[y - 1][x + 1], v[y + 1][x - 1], v[y + 1][x + 1]);
+        }
+        float2 l0 = make_float2(lo[0], lo[1]);
+        float4 d[2][4];
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+#pragma unroll
+            for (int a = 0; a < 2; a++) {
+                auto win = [&](int r, int c) { return v[b + r][a + c]; };
+                d[b][1 + a] = rq_disc4(win);
+            }
+            const float4 l = walk_left4(d[b][2]), r = walk_right4(d[b][1]);
+            d[b][0] = first ? d[b][2] : l;
+            d[b][3] = last ? d[b][1] : r;
+        }
+        if (row == h2) {
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                d[0][c] = d0[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            d0[c] = d[0][c];
+        float4 r3[2][2], sb[2], sa[2];
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+            for (int a = 0; a < 2; a++)
+                r3[b][a] = rq_add4(rq_add4(d[b][a], d[b][a + 1]), d[b][a + 2]);
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+            const float4 up = row == 0 ? r3[1][a] : rr[a];
+            sb[a] = rp_add3(t[a], d[0][a], d[0][a + 1], d[0][a + 2]);          /* pixel row 2s - 1 */
+            sa[a] = rp_add3(rp_add3(up, d[0][a], d[0][a + 1], d[0][a + 2]), d[1][a], d[1][a + 1], d[1][a + 2]);
+            t[a] = rp_add3(r3[0][a], d[1][a], d[1][a + 1], d[1][a + 2]);
+            rr[a] = r3[1][a];
+        }
+        /* W, G of row - 1. */
+        const float2 wp1 = make_float2(wp0, rp_wp(sb[1])), wg1 = make_float2(wg0, rp_wv(sb[0]));
+        const float wv1 = wv0;
+        wv0 = rp_wv(sa[0]);
+        wp0 = rp_wp(sa[0]);
+        wg0 = rp_wv(sa[1]);
+        const float2 la = row == 1 ? make_float2(l0.x, l1.y) : l2;
+        const float2 lb = row == h2 ? make_float2(l1.x, l2.y) : l0;
+        const float2 le = make_float2(walk_left(l1.x), walk_left(l1.y));
+        const float2 ri = make_float2(walk_right(l1.x), walk_right(l1.y));
+        const float2 ll = first ? make_float2(ri.x, l1.y) : le, lr = last ? make_float2(l1.x, le.y) : ri;
+        const float2 g1 = make_float2(
+            rq_green(wv1, l1.x, q2[2], la.x, v[1][2], lb.x, v[0][1], ll.x, v[0][3], lr.x),
+            rq_green(rp_wv(sb[1]), l1.y, v[0][3], la.y, v[2][3], lb.y, v[1][2], ll.y, v[1][4], lr.y));
+        const float kr1 = __fsub_rn(v[0][2], g1.x), kb1 = __fsub_rn(v[1][3], g1.y);
+        const float krn = walk_right(kr1), kbn = walk_left(kb1);
+        const float krr1 = last ? kr1 : krn, kbl1 = first ? kb1 : kbn;
+        /* C of row - 2. */
+        const bool t2 = row == 2, b2 = row == h2 + 1;
+        const float2 c2 = make_float2(
+            rq_cross(wp2.x, g2.x, kbl2, t2 ? kb2 : kb3, t2 ? kbl2 : kbl3, kb2),
+            rq_cross(wp2.y, g2.y, b2 ? kr2 : kr1, krr2, kr2, b2 ? krr2 : krr1));
+        const float jr2 = __fsub_rn(c2.x, g2.x), jb2 = __fsub_rn(c2.y, g2.y);
+        const float jrn = walk_right(jr2), jbn = walk_left(jb2);
+        const float jrr2 = last ? jr2 : jrn, jbl2 = first ? jb2 : jbn;
+        /* The pixels of row - 3. */
+        const bool t3 = row == 3, b3 = row == h2 + 2;
+        o[0][0][0] = q3[0]; o[0][0][1] = g3.x;  o[0][0][2] = c3.x;
+        o[0][1][1] = q3[1];
+        rp_green_site(wg3.x, q3[1], kr3, krr3, t3 ? jb3 : jb4, jb3, t3 ? kb3 : kb4, kb3, jr3, jrr3, o[0][1][0],
+                      o[0][1][2]);
+        o[1][0][1] = q3[2];
+        rp_green_site(wg3.y, q3[2], kbl3, kb3, jr3, b3 ? jr3 : jr2, kr3, b3 ? kr3 : kr2, jbl3, jb3, o[1][0][2],
+                      o[1][0][0]);
+        o[1][1][0] = c3.y;  o[1][1][1] = g3.y;  o[1][1][2] = q3[3];
+        /* A row on. */
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            q3[i] = q2[i];
+        q2[0] = v[0][2]; q2[1] = v[0][3]; q2[2] = v[1][2]; q2[3] = v[1][3];
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int c = 0; c < 6; c++)
+                v[r][c] = v[r + 2][c];
+        l2 = l1; l1 = l0;
+        wg3 = wg2; wg2 = wg1;
+        wp2 = wp1;
+        g3 = g2; g2 = g1;
+        kr3 = kr2; kr2 = kr1; krr3 = krr2; krr2 = krr1;
+        kb4 = kb3; kb3 = kb2; kb2 = kb1; kbl3 = kbl2; kbl2 = kbl1;
+        jb4 = jb3; jb3 = jb2; jbl3 = jbl2; jr3 = jr2; jrr3 = jrr2;
+        c3 = c2;
+    }
+};
+
+/* The border's parts (above, below, left and right of the interior, or the
+ * whole of a frame without one) and the first warp of each. */
+struct RingGrid {
+    WalkGrid g[4];
+    int first[5];
+};
+
+template <int FMT, bool RGC, bool MORE>
+CRAW_DEV void ring_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const RingGrid &ring, int wid,
+                        WalkSmem<RW_NQ> &smem)
+{
+    if (wid >= ring.first[4])
+        return;
+    int part = 0;
+#pragma unroll
+    for (int i = 1; i < 4; i++)
+        if (wid >= ring.first[i])
+            part = i;
+    const WalkGrid &g = ring.g[part];
+    wid -= ring.first[part];
+    const int sx = wid % g.nx, sy = wid / g.nx;
+    const int nrows = min(g.seg, g.nqy - sy * g.seg);
+    WalkOut<RW_NQ, RW_A, FMT, RGC, MORE> out(k, io, smem, min(RW_NQ, g.nqx - sx * RW_NQ), g.qx0 + sx * RW_NQ,
+                                             g.qy0 + sy * g.seg);
+    const int w2 = k.width / 2, h2 = k.height / 2, col = out.qx - RW_A + out.lane;
+    const int q = max(0, min(col, w2 - 1)), y0 = 2 * out.qy;
+    const bool first = col == 0, last = col == w2 - 1;
+    const char *src = (const char *)io.src + 4 * (size_t)q;
+    auto fetch = [&](int yr) {
+        /* The rows that mirror two rows beyond the frame; farther out, any
+         * row (nothing reads what comes of it). */
+        const int m = abs(y0 + yr), y = max(0, min(m < k.height ? m : 2 * k.height - 2 - m, k.height - 1));
+        if (!craw_in_bounds(q >= 0 && 2 * q + 1 < k.width && y >= 0, io.err))
+            return 0u;
+        return walk_ld(src + (size_t)y * io.src_pitch);
+    };
+    RingWalk t;
+    memset(&t, 0, sizeof(t));
+    uint32_t init[4], raw[2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        init[i] = fetch(-6 + i);
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        raw[i] = fetch(-2 + i);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        t.rows(walk_prep(k, io, init[2 * i], 0), walk_prep(k, io, init[2 * i + 1], 1), first, last);
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            t.v[2 * i][c] = t.v[4][c];
+            t.v[2 * i + 1][c] = t.v[5][c];
+        }
+    }
+#pragma unroll 1
+    for (int s = -2; s <= nrows + 2; s++) {
+        uint32_t next[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            next[i] = fetch(2 * s + 4 + i);
+        float o[2][2][3];
+        t.rows(walk_prep(k, io, raw[0], 0), walk_prep(k, io, raw[1], 1), first, last);
+        t.step(out.qy + s, h2, first, last, o);
+        const int r = s - 3;
+        if (r >= 0 && r < nrows)
+            out.quad_row(r, r == nrows - 1, o);
+        raw[0] = next[0];
+        raw[1] = next[1];
+    }
+}
 
 /* The strip of warp `wid` of the grid. */
 template <int FMT, bool RGC, bool MORE>
