@@ -49,7 +49,7 @@ typedef struct CRAWBatchParams {
 #define CRAW_BATCH_DIRECT_PIXELS 4000000u
 
 typedef struct CRAWBatchInfo {
-    int denoise_shape;               /* the autotuned tile shape: 0 = 2x4, 1 = 2x8 */
+    int denoise_shape;               /* the last recording's tile shape: 0 = 2x4, 1 = 2x8 */
     int fused;                       /* one launch with a grid barrier */
     int graph;                       /* recordings replay a captured graph */
     uint64_t captures, replays;      /* graphs captured, replays launched */

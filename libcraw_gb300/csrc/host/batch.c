@@ -67,90 +67,53 @@ static void batch_release(CRAWBatch *b)
     free(b);
 }
 
-/* Items of each phase for a frame list, and every frame's place in them. */
-static void batch_layout(CRAWBatch *b, uint32_t nb, const uint32_t *w, const uint32_t *h,
-                         const bool *dn, CRAWKBatchFrame *F, int32_t *dn_items, int32_t *dv_items)
-{
-    int32_t dn_n = 0, dv_n = 0;
-    for (uint32_t i = 0; i < nb; i++) {
-        craw_k_batch_tiles((int32_t)w[i], (int32_t)h[i], b->shape, &F[i].dn_tx, &F[i].dn_ty,
-                           &F[i].dv_tx, &F[i].dv_ty);
-        if (!dn[i])
-            F[i].dn_tx = F[i].dn_ty = 0;
-        F[i].dn_first = dn_n;
-        F[i].dv_first = dv_n;
-        dn_n += F[i].dn_tx * F[i].dn_ty;
-        dv_n += F[i].dv_tx * F[i].dv_ty;
-    }
-    *dn_items = dn_n;
-    *dv_items = dv_n;
-}
-
-/* Times one max-size frame through each denoise tile shape and keeps the
- * faster (the work does not depend on the data). */
+/* Times a frame of the largest size through each of the single-frame
+ * kernel's denoise shapes, for the frames developed directly, and keeps the
+ * fastest (the work does not depend on the data). */
 static int batch_autotune(CRAWBatch *b)
 {
     CRAWContext *ctx = b->ctx;
     const uint32_t w = b->params.max_width, h = b->params.max_height;
     CRAWKBatchFrame *F = &b->table->f[0];
-    void *out = NULL;
-    uint16_t *mosaic;
-    size_t out_pitch = (((size_t)w * 16) + 255) / 256 * 256;
+    void *mosaic = NULL;
     cudaEvent_t e0 = NULL, e1 = NULL;
     float best = 1e30f;
     int ret = 0;
 
-    /* The output image, then a grey mosaic to denoise. */
-    if ((ret = craw_dev_alloc(ctx, &out, out_pitch * h + b->clean_pitch * h)) < 0)
+    if ((ret = craw_dev_alloc(ctx, &mosaic, b->clean_pitch * h)) < 0)
         return ret;
-    mosaic = (uint16_t *)((char *)out + out_pitch * h);
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
         ret = CRAW_ERROR(ENOMEM);
         goto done;
     }
     /* A grey frame with plausible constants. */
     cudaMemset2DAsync(mosaic, b->clean_pitch, 0x08, (size_t)w * 2, h, ctx->stream);
-    for (int shape = 0; shape < CRAW_K_BATCH_DN_NB; shape++) {
-        int32_t dn_items, dv_items;
-        bool dn = true;
+    memset(F, 0, sizeof(*F));
+    F->dn.pw = (int32_t)(w / 2);
+    F->dn.ph = (int32_t)(h / 2);
+    F->dn.gat_a = 1e-3f; F->dn.gat_c = 1e-6f; F->dn.gat_sc = 1e-3f; F->dn.gat_fwd = 2000.0f;
+    F->dn.gat_inv = 2.5e-4f; F->dn.gat_off = 1e-3f; F->dn.gat_t0 = 2.0f;
+    F->dn.inv_h2 = 1.0f; F->dn.guard_lo = 0.9f; F->dn.guard_inv = 10.0f;
+    F->dn.mode = CRAW_K_DN_SPATIAL;
+    for (int s = 0; s < 4; s++) {
+        F->dn.inv_range[s] = 16.0f;
+        F->dn.range[s] = 0.0625f;
+    }
+    F->dio.src = mosaic;
+    F->dio.src_pitch = b->clean_pitch;
+    F->dio.dst = b->clean[0];
+    F->dio.dst_pitch = b->clean_pitch;
+    for (int shape = 0; shape < CRAW_K_DN_SHAPE_NB; shape++) {
         float t = 0.0f, ms = 1e30f;
-        b->shape = shape;
-        memset(F, 0, sizeof(*F));
-        F->dn.pw = (int32_t)(w / 2);
-        F->dn.ph = (int32_t)(h / 2);
-        F->dn.gat_a = 1e-3f; F->dn.gat_c = 1e-6f; F->dn.gat_sc = 1e-3f; F->dn.gat_fwd = 2000.0f;
-        F->dn.gat_inv = 2.5e-4f; F->dn.gat_off = 1e-3f; F->dn.gat_t0 = 2.0f;
-        F->dn.inv_h2 = 1.0f; F->dn.guard_lo = 0.9f; F->dn.guard_inv = 10.0f;
-        F->dn.mode = CRAW_K_DN_SPATIAL;
-        for (int s = 0; s < 4; s++) {
-            F->dn.inv_range[s] = 16.0f;
-            F->dn.range[s] = 0.0625f;
-            F->dv.inv_range[s] = 16.0f;
-            F->dv.wbs[s] = 1.0f;
-        }
-        F->dio.src = mosaic;
-        F->dio.src_pitch = b->clean_pitch;
-        F->dio.dst = b->clean[0];
-        F->dio.dst_pitch = b->clean_pitch;
-        F->dv.width = (int32_t)w;
-        F->dv.height = (int32_t)h;
-        F->dv.clip = 1.0f;
-        F->dv.method = b->params.debayer;
-        F->dv.color.m[0][0] = F->dv.color.m[1][1] = F->dv.color.m[2][2] = 1.0f;
-        F->vio.src = b->clean[0];
-        F->vio.src_pitch = b->clean_pitch;
-        F->vio.dst = out;
-        F->vio.dst_pitch = out_pitch;
-        batch_layout(b, 1, &w, &h, &dn, F, &dn_items, &dv_items);
         for (int r = 0; r < 3; r++) {
             cudaEventRecord(e0, ctx->stream);
-            if (craw_k_batch(b->table, 1, dn_items, dv_items, b->params.debayer, shape, b->fused,
-                             ctx->stream) < 0) {
+            if (craw_k_denoise(&F->dn, &F->dio, shape, NULL, NULL, NULL, ctx->stream) < 0) {
                 ret = CRAW_ERROR(EIO);
                 goto done;
             }
             cudaEventRecord(e1, ctx->stream);
-            if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&t, e0, e1) != cudaSuccess) {
+            if (cudaEventSynchronize(e1) != cudaSuccess ||
+                cudaEventElapsedTime(&t, e0, e1) != cudaSuccess) {
                 ret = CRAW_ERROR(EIO);
                 goto done;
             }
@@ -159,48 +122,17 @@ static int batch_autotune(CRAWBatch *b)
         }
         if (ms < best) {
             best = ms;
-            ret = shape;
+            b->direct_shape = shape;
         }
     }
-    b->shape = ret;
-    craw_log(ctx, CRAW_LOG_VERBOSE, "batch autotune %ux%u: denoise shape %d, %.3f ms\n", w, h,
-             b->shape, (double)best);
-    ret = 0;
-    /* The single-frame kernel's shapes, for frames developed directly. */
-    b->direct_shape = -1;
-    if ((uint64_t)w * h >= b->direct_pixels) {
-        best = 1e30f;
-        for (int shape = 0; shape < CRAW_K_DN_SHAPE_NB; shape++) {
-            float t = 0.0f, ms = 1e30f;
-            for (int r = 0; r < 3; r++) {
-                cudaEventRecord(e0, ctx->stream);
-                if (craw_k_denoise(&F->dn, &F->dio, shape, NULL, NULL, NULL, ctx->stream) < 0) {
-                    ret = CRAW_ERROR(EIO);
-                    goto done;
-                }
-                cudaEventRecord(e1, ctx->stream);
-                if (cudaEventSynchronize(e1) != cudaSuccess ||
-                    cudaEventElapsedTime(&t, e0, e1) != cudaSuccess) {
-                    ret = CRAW_ERROR(EIO);
-                    goto done;
-                }
-                if (r > 0 && t < ms)
-                    ms = t;
-            }
-            if (ms < best) {
-                best = ms;
-                b->direct_shape = shape;
-            }
-        }
-        craw_log(ctx, CRAW_LOG_VERBOSE, "batch autotune %ux%u: direct denoise shape %d, %.3f ms\n", w, h,
-                 b->direct_shape, (double)best);
-    }
+    craw_log(ctx, CRAW_LOG_VERBOSE, "batch autotune %ux%u: direct denoise shape %d, %.3f ms\n", w, h,
+             b->direct_shape, (double)best);
 done:
     if (e0)
         cudaEventDestroy(e0);
     if (e1)
         cudaEventDestroy(e1);
-    craw_dev_free(ctx, out);
+    craw_dev_free(ctx, mosaic);
     if (craw_dev_sync(ctx) < 0 && ret == 0)
         ret = CRAW_ERROR(EIO);
     return ret;
@@ -255,8 +187,17 @@ CRAW_API int craw_batch_create(CRAWContext *ctx, const CRAWBatchParams *params, 
     }
     if ((ret = craw_dev_sync(ctx)) < 0)
         goto fail;
-    if (b->denoise && (ret = batch_autotune(b)) < 0)
-        goto fail;
+    if (b->denoise) {
+        CRAWKBatchFrame *F = &b->table->f[0];
+        int32_t dn_items, dv_items;
+        F->dv.width = (int32_t)params->max_width;
+        F->dv.height = (int32_t)params->max_height;
+        F->dn.mode = CRAW_K_DN_SPATIAL;
+        craw_k_batch_layout(F, 1, params->debayer, &dn_items, &dv_items);
+        b->shape = craw_k_batch_shape(dn_items);
+        if ((uint64_t)params->max_width * params->max_height >= b->direct_pixels && (ret = batch_autotune(b)) < 0)
+            goto fail;
+    }
     *out = b;
     return 0;
 fail:
@@ -296,8 +237,8 @@ static int batch_capture(CRAWBatch *b, uint32_t nb, int32_t dn_items, int32_t dv
 
     if (cudaStreamBeginCapture(b->cap_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return CRAW_ERROR(EIO);
-    ret = craw_k_batch(b->table, (int32_t)nb, dn_items, dv_items, b->params.debayer, b->shape,
-                       b->fused, b->cap_stream);
+    ret = craw_k_batch(b->table, (int32_t)nb, dn_items, dv_items, b->params.debayer, b->fused,
+                       b->cap_stream);
     if (cudaStreamEndCapture(b->cap_stream, &g) != cudaSuccess || ret < 0) {
         if (g)
             cudaGraphDestroy(g);
@@ -423,7 +364,8 @@ static int batch_persistent(CRAWBatch *b, cudaStream_t s, uint32_t nb, const uin
     bool same;
     int ret;
 
-    batch_layout(b, nb, w, h, dn, F, &dn_items, &dv_items);
+    craw_k_batch_layout(F, (int32_t)nb, b->params.debayer, &dn_items, &dv_items);
+    b->shape = craw_k_batch_shape(dn_items);
 
     same = b->exec && b->sig_nb == nb;
     for (uint32_t i = 0; same && i < nb; i++)
@@ -450,8 +392,7 @@ static int batch_persistent(CRAWBatch *b, cudaStream_t s, uint32_t nb, const uin
             return CRAW_ERROR(EIO);
         }
         b->replays++;
-    } else if (craw_k_batch(b->table, (int32_t)nb, dn_items, dv_items, b->params.debayer, b->shape,
-                            b->fused, s) < 0) {
+    } else if (craw_k_batch(b->table, (int32_t)nb, dn_items, dv_items, b->params.debayer, b->fused, s) < 0) {
         return CRAW_ERROR(EIO);
     }
     return 0;

@@ -342,27 +342,32 @@ int craw_k_noise_lts(const double *m, const double *v, const double *lv, int32_t
 
 /* ------------------------------------------------------------- batch */
 
-/* One frame of a batch: its constants and buffers, how many tiles each
- * phase has, and where its tiles start in each phase's item list. */
+/* One frame of a batch: its constants and buffers, and where its items
+ * start in each phase's list (craw_k_batch_layout). */
 typedef struct CRAWKBatchFrame {
     CRAWKDenoise dn;            /* dn.mode == 0: the frame is not denoised */
     CRAWKDenoiseIO dio;
     CRAWKDevelop dv;
     CRAWKDevelopIO vio;         /* vio.src is dio.dst when denoised */
-    int32_t dn_tx, dn_ty, dn_first;
-    int32_t dv_tx, dv_ty, dv_first;
+    int32_t dn_tx, dn_first;    /* denoise tiles: across, the first */
+    int32_t dv_first, dv_tx;    /* develop: the first item (RCD: of the interior); tiles across (not RCD) */
+    int32_t dv_border;          /* RCD: the first item of the border */
+    int32_t dv_cut, dv_cut_border;   /* RCD: quad rows of a segment at most, alike for all frames */
 } CRAWKBatchFrame;
 
-/* Denoise tile shapes of the batch kernel (256 threads). */
+/* Denoise tile shapes of the batch kernel. */
 enum CRAWKBatchShape {
     CRAW_K_BATCH_DN_2x4 = 0,    /* 2 columns x 4 rows a thread, 32x16 tiles, packed f32x2 */
-    CRAW_K_BATCH_DN_2x8,        /* 2 x 8, 32x32 tiles, packed f32x2 */
+    CRAW_K_BATCH_DN_2x8,        /* 2 x 8, 32x16 tiles, packed f32x2 */
     CRAW_K_BATCH_DN_NB,
 };
 
-/* Tiles per phase for a frame of w x h with a denoise shape. */
-void craw_k_batch_tiles(int32_t w, int32_t h, int shape, int32_t *dn_tx, int32_t *dn_ty,
-                        int32_t *dv_tx, int32_t *dv_ty);
+/* Lays out the items of `nb` frames (their dv sizes and dn modes set): every
+ * frame's place in them, and each phase's count. */
+void craw_k_batch_layout(CRAWKBatchFrame *f, int32_t nb, int method, int32_t *dn_items, int32_t *dv_items);
+
+/* The denoise shape (CRAW_K_BATCH_DN_*) of a launch of `dn_items` tiles. */
+int craw_k_batch_shape(int32_t dn_items);
 
 /* The frames of one batch launch, passed by value as a kernel parameter
  * (30 KB of the 32 KB a launch may carry): the kernels read a frame's
@@ -373,12 +378,13 @@ typedef struct CRAWKBatchTable {
 } CRAWKBatchTable;
 
 /* Develops the first `nb` frames of `table` (host memory, copied into the
- * launch) in one persistent launch: every denoise tile of every frame, a
- * grid-wide barrier, every develop tile (`fused`); or as two persistent
- * launches. Grid: as many CTAs as fit on the device at once. All frames
- * use the same debayer, RCD or MHC or bilinear, `method`. */
+ * launch): every denoise tile of every frame, a grid-wide barrier, every
+ * develop item, in one persistent launch of as many CTAs as fit on the
+ * device at once (`fused`); or as two launches of a CTA an item. All frames
+ * use the same debayer, RCD or MHC or bilinear, `method`, and one output
+ * layout. */
 int craw_k_batch(const CRAWKBatchTable *table, int32_t nb, int32_t dn_items, int32_t dv_items,
-                 int method, int shape, int fused, cudaStream_t s);
+                 int method, int fused, cudaStream_t s);
 
 /* Points every batch kernel node of an instantiated graph (one captured
  * craw_k_batch call) at a new table and item counts. */

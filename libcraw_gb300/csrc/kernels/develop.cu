@@ -136,7 +136,7 @@ k_develop_rcd_quads_tma(const CRAWKDevelop k, const CRAWKDevelopIO io, const Qua
  * to 340 bytes of spills). */
 constexpr int WALK_CTAS = 3;
 
-template <int FMT, bool RGC, bool MORE>
+template <int FMT, int RGC, bool MORE>
 __global__ void __launch_bounds__(WALK_NT, WALK_CTAS)
 k_develop_rcd_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
 {
@@ -146,14 +146,27 @@ k_develop_rcd_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid
     rcd_walk<FMT, RGC, MORE>(k, io, g, blockIdx.x * WALK_WARPS + warp, smem[warp]);
 }
 
+/* The border's parts and the first warp of each. */
+struct RingGrid {
+    WalkGrid g[4];
+    int first[5];
+};
+
 /* The border by walking warps, in the same CTAs. */
-template <int FMT, bool RGC, bool MORE>
+template <int FMT, int RGC, bool MORE>
 __global__ void __launch_bounds__(WALK_NT, WALK_CTAS)
 k_develop_rcd_ring(const CRAWKDevelop k, const CRAWKDevelopIO io, const __grid_constant__ RingGrid ring)
 {
     __shared__ WalkSmem<RW_NQ> smem[WALK_WARPS];
     const int warp = threadIdx.x >> 5;
-    ring_walk<FMT, RGC, MORE>(k, io, ring, blockIdx.x * WALK_WARPS + warp, smem[warp]);
+    const int wid = blockIdx.x * WALK_WARPS + warp;
+    int part = 0;
+#pragma unroll
+    for (int i = 1; i < 4; i++)
+        if (wid >= ring.first[i])
+            part = i;
+    if (wid < ring.first[4])
+        ring_walk<FMT, RGC, MORE>(k, io, ring.g[part], wid - ring.first[part], smem[warp]);
     await_interior();
 }
 
@@ -220,25 +233,6 @@ unsigned walk_segments(WalkGrid &g, int ctas, int least)
     return (unsigned)((warps + WALK_WARPS - 1) / WALK_WARPS);
 }
 
-/* A part of the frame, in quads, as strips; false if it is empty. */
-bool walk_part(WalkGrid &g, int x0, int x1, int y0, int y1)
-{
-    g.qx0 = x0;
-    g.nqx = x1 - x0;
-    g.qy0 = y0;
-    g.nqy = y1 - y0;
-    g.nx = (g.nqx + RW_NQ - 1) / RW_NQ;
-    return g.nqx > 0 && g.nqy > 0;
-}
-
-/* Segments of at most `most` quad rows, alike; returns the part's warps. */
-int walk_cut(WalkGrid &g, int most)
-{
-    const int n = (g.nqy + most - 1) / most;
-    g.seg = 4 * (((g.nqy + 3) / 4 + n - 1) / n);
-    return g.nx * ((g.nqy + g.seg - 1) / g.seg);
-}
-
 /* The RCD of a w x h frame as strips: the interior's (w, its CTAs in inner;
  * none if the frame has none) and the border's. Segments are a multiple of 4
  * quad rows, at least 8. Either the interior takes one wave of WALK_CTAS
@@ -248,32 +242,30 @@ int walk_cut(WalkGrid &g, int most)
  * n + 5 in the border: the fewer in all. Frame times, sharing against taking
  * turns: 115 and 124 us (1920x1080, denoise with history, AP0), 280 and 284
  * (3840x2160, denoise); 737 and 706 (5760x3240, exact denoise, AP1). */
-void rcd_grids(int width, int height, const QuadGrid &q, WalkGrid &w, RingGrid &ring, int &inner, int &border)
+void rcd_grids(int width, int height, WalkGrid &w, RingGrid &ring, int &inner, int &border)
 {
-    const int w2 = width / 2, h2 = height / 2, room = craw_sm_count() * WALK_CTAS;
-    const bool in = q.interior_x() > 0 && q.interior_y() > 0;
-    const int x0 = in ? q.c_lo * (QTW / 2) : w2, x1 = in ? (q.c_hi + 1) * (QTW / 2) : w2;
-    const int y0 = in ? q.r_lo * (QTH / 2) : h2, y1 = in ? (q.r_hi + 1) * (QTH / 2) : h2;
-    walk_part(w, x0, x1, y0, y1);
-    const bool any[4] = { walk_part(ring.g[0], 0, w2, 0, y0), walk_part(ring.g[1], 0, w2, y1, h2),
-                          walk_part(ring.g[2], 0, x0, y0, y1), walk_part(ring.g[3], x1, w2, y0, y1) };
+    const int h2 = height / 2, room = craw_sm_count() * WALK_CTAS;
+    w = rcd_part(width, height, 0);
+    for (int i = 0; i < 4; i++)
+        ring.g[i] = rcd_part(width, height, 1 + i);
+    const bool in = w.nqx > 0 && w.nqy > 0;
     auto ctas = [](int warps) { return (warps + WALK_WARPS - 1) / WALK_WARPS; };
     auto cut_ring = [&](int most) {
         ring.first[0] = 0;
         for (int i = 0; i < 4; i++)
-            ring.first[i + 1] = ring.first[i] + (any[i] ? walk_cut(ring.g[i], most) : 0);
+            ring.first[i + 1] = ring.first[i] + walk_cut(ring.g[i], most);
         return ctas(ring.first[4]);
     };
     int turn = 8, turn_ring = 8, both = 8;
-    while (turn < h2 && in && ctas(walk_cut(w, turn)) > room)
+    while (turn < h2 && ctas(walk_cut(w, turn)) > room)
         turn += 4;
     while (turn_ring < h2 && cut_ring(turn_ring) > room)
         turn_ring += 4;
     auto half = [](int n) { return n / 8 * 4 > 8 ? n / 8 * 4 : 8; };
-    while (both < h2 && in && ctas(walk_cut(w, both)) + cut_ring(half(both)) > room)
+    while (both < h2 && ctas(walk_cut(w, both)) + cut_ring(half(both)) > room)
         both += 4;
     const bool share = in && both + 6 < turn + 6 + turn_ring + 5;
-    inner = in ? ctas(walk_cut(w, share ? both : turn)) : 0;
+    inner = ctas(walk_cut(w, share ? both : turn));
     border = cut_ring(share ? half(both) : turn_ring);
 }
 
@@ -342,13 +334,13 @@ int launch_border(void (*kernel)(P...), int ctas, int threads, size_t smem, bool
 }
 
 /* The walking kernels of a frame. */
-template <int FMT, bool RGC, bool MORE>
-int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, const QuadGrid &g, cudaStream_t s)
+template <int FMT, int RGC, bool MORE>
+int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
 {
     WalkGrid w;
     RingGrid ring;
     int inner, border;
-    rcd_grids(k->width, k->height, g, w, ring, inner, border);
+    rcd_grids(k->width, k->height, w, ring, inner, border);
     if (inner > 0) {
         k_develop_rcd_walk<FMT, RGC, MORE><<<inner, WALK_NT, 0, s>>>(*k, *io, w);
         if (cudaGetLastError() != cudaSuccess)
@@ -357,13 +349,13 @@ int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, const QuadGrid 
     return launch_border(k_develop_rcd_ring<FMT, RGC, MORE>, border, WALK_NT, 0, inner > 0, s, *k, *io, ring);
 }
 
-template <bool RGC>
-int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, const QuadGrid &g, cudaStream_t s)
+template <int RGC>
+int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
 {
     switch (io->dst_fmt) {
-    case CRAW_K_OUT_RGBA16F: return launch_walk<CRAW_K_OUT_RGBA16F, RGC, false>(k, io, g, s);
-    case CRAW_K_OUT_RGB32F:  return launch_walk<CRAW_K_OUT_RGB32F, RGC, false>(k, io, g, s);
-    default:                 return launch_walk<CRAW_K_OUT_RGBA32F, RGC, false>(k, io, g, s);
+    case CRAW_K_OUT_RGBA16F: return launch_walk<CRAW_K_OUT_RGBA16F, RGC, false>(k, io, s);
+    case CRAW_K_OUT_RGB32F:  return launch_walk<CRAW_K_OUT_RGB32F, RGC, false>(k, io, s);
+    default:                 return launch_walk<CRAW_K_OUT_RGBA32F, RGC, false>(k, io, s);
     }
 }
 
@@ -372,13 +364,13 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
     constexpr size_t smem = RcdQuads<QTW, QTH, QNT>::floats * sizeof(float);
     if (prepare_rcd() < 0)
         return -5;
-    QuadGrid g;
-    g.init(k->width, k->height);
     if (craw_k_rcd_strips) {
         if (k->fp16 || io->inter || io->quarter || !io->dst)
-            return launch_walk<0, false, true>(k, io, g, s);
-        return k->color.flags & CRAW_K_COLOR_RGC ? launch_walk<true>(k, io, g, s) : launch_walk<false>(k, io, g, s);
+            return launch_walk<0, -1, true>(k, io, s);
+        return k->color.flags & CRAW_K_COLOR_RGC ? launch_walk<1>(k, io, s) : launch_walk<0>(k, io, s);
     }
+    QuadGrid g;
+    g.init(k->width, k->height);
     const bool interior = g.interior_x() > 0 && g.interior_y() > 0;
     if (interior) {
         const dim3 grid(g.interior_x(), g.interior_y());

@@ -136,10 +136,10 @@ struct WalkSmem {
 
 /* The epilogue of one warp: takes the camera RGB of the four pixels of each
  * lane's quad, a quad row at a time. FMT (a CRAW_K_OUT_* layout), RGC (the
- * gamut compression): fixed per kernel, so that a step's code stays small
+ * gamut compression: with it, without, or -1 by its flag): fixed per kernel, so that a step's code stays small
  * enough for the instruction cache; MORE: any layout, FP16 storage, the
  * kept intermediate and the chroma path's block means, by tests. */
-template <int NQ, int A, int FMT, bool RGC, bool MORE>
+template <int NQ, int A, int FMT, int RGC, bool MORE>
 struct WalkOut {
     using S = WalkSmem<NQ>;
     const CRAWKDevelop &k;
@@ -172,7 +172,7 @@ struct WalkOut {
 #pragma unroll
             for (int c = 0; c < 3; c++)
                 q[i][c] = v[i >> 1][i & 1][c];
-        walk_colour<MORE ? -1 : RGC>(k.color, mine, q);
+        walk_colour<RGC>(k.color, mine, q);
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -375,6 +375,37 @@ CRAW_DEV float2 walk_prep(const CRAWKDevelop &k, const CRAWKDevelopIO &io, uint3
  * inside the frame; reads past the frame's edge are clamped to it and only
  * feed values nothing reads. */
 constexpr int RW_NQ = 24, RW_A = 4;
+
+/* A part of a w x h frame as strips, without segments: the interior (0),
+ * whose 64x16 tiles have their aprons inside the frame, and the border above,
+ * below, left and right of it (1 to 4; of a frame without an interior, all in
+ * 1). nqx or nqy is 0 where a part is empty. */
+__host__ CRAW_DEV WalkGrid rcd_part(int width, int height, int i)
+{
+    const int w2 = width / 2, h2 = height / 2, c_hi = (width - QTW - 6) / QTW, r_hi = (height - QTH - 6) / QTH;
+    const bool in = c_hi >= 1 && r_hi >= 1;
+    const int x0 = in ? QTW / 2 : w2, x1 = in ? (c_hi + 1) * (QTW / 2) : w2;
+    const int y0 = in ? QTH / 2 : h2, y1 = in ? (r_hi + 1) * (QTH / 2) : h2;
+    WalkGrid g;
+    g.qx0 = i == 0 ? x0 : (i == 4 ? x1 : 0);
+    g.nqx = (i == 0 ? x1 : (i == 3 ? x0 : w2)) - g.qx0;
+    g.qy0 = i == 1 ? 0 : (i == 2 ? y1 : y0);
+    g.nqy = (i == 1 ? y0 : (i == 2 ? h2 : y1)) - g.qy0;
+    g.nx = (g.nqx + RW_NQ - 1) / RW_NQ;
+    g.seg = 4;
+    return g;
+}
+
+/* Cuts a part into segments of at most `most` quad rows (a multiple of 4),
+ * all alike; returns its warps. */
+__host__ CRAW_DEV int walk_cut(WalkGrid &g, int most)
+{
+    if (g.nqx <= 0 || g.nqy <= 0)
+        return 0;
+    const int n = (g.nqy + most - 1) / most;
+    g.seg = 4 * (((g.nqy + 3) / 4 + n - 1) / n);
+    return g.nx * ((g.nqy + g.seg - 1) / g.seg);
+}
 
 /* The weights, and the colours at a green site, with the roundings of the
  * per-pixel tiles (RcdTile), where the two forms differ. */
@@ -670,26 +701,11 @@ struct RingWalk {
     }
 };
 
-/* The border's parts (above, below, left and right of the interior, or the
- * whole of a frame without one) and the first warp of each. */
-struct RingGrid {
-    WalkGrid g[4];
-    int first[5];
-};
-
-template <int FMT, bool RGC, bool MORE>
-CRAW_DEV void ring_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const RingGrid &ring, int wid,
+/* The strip of warp `wid` of one of the border's parts. */
+template <int FMT, int RGC, bool MORE>
+CRAW_DEV void ring_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const WalkGrid &g, int wid,
                         WalkSmem<RW_NQ> &smem)
 {
-    if (wid >= ring.first[4])
-        return;
-    int part = 0;
-#pragma unroll
-    for (int i = 1; i < 4; i++)
-        if (wid >= ring.first[i])
-            part = i;
-    const WalkGrid &g = ring.g[part];
-    wid -= ring.first[part];
     const int sx = wid % g.nx, sy = wid / g.nx;
     const int nrows = min(g.seg, g.nqy - sy * g.seg);
     WalkOut<RW_NQ, RW_A, FMT, RGC, MORE> out(k, io, smem, min(RW_NQ, g.nqx - sx * RW_NQ), g.qx0 + sx * RW_NQ,
@@ -742,7 +758,7 @@ CRAW_DEV void ring_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const R
 }
 
 /* The strip of warp `wid` of the grid. */
-template <int FMT, bool RGC, bool MORE>
+template <int FMT, int RGC, bool MORE>
 CRAW_DEV void rcd_walk(const CRAWKDevelop &k, const CRAWKDevelopIO &io, const WalkGrid &g, int wid,
                        WalkSmem<RW_NQ> &smem)
 {
