@@ -32,16 +32,14 @@ namespace {
 constexpr float kULo = 0.92f, kUHi = 0.98f, kEps = 1e-4f, kLogMax = 2.0f, kWSat = 1.0f;
 constexpr int kDilate = 3;
 
-CRAW_DEV int site_chan(int s) { return s == 0 ? 0 : (s == 3 ? 2 : 1); }
-
-/* smoothstep(kULo, kUHi, v); below kULo the quotient is <= 0 and clamps
- * to 0, which the early return gives without the division. */
+/* smoothstep(kULo, kUHi, v). The quotient by Markstein's correction of the
+ * product with the correctly rounded reciprocal, which rounds as the division
+ * does; below kULo it is not positive and clamps to 0. */
 CRAW_DEV float smooth(float v)
 {
-    if (v <= kULo)
-        return 0.0f;
-    float t = __fdiv_rn(v - kULo, kUHi - kULo);
-    t = t < 0.0f ? 0.0f : (t > 1.0f ? 1.0f : t);
+    constexpr float c = kUHi - kULo, rc = 1.0f / c;
+    const float x = v - kULo, q = x * rc;
+    const float t = __saturatef(__fmaf_rn(__fmaf_rn(-c, q, x), rc, q));
     return t * t * (3.0f - 2.0f * t);
 }
 
@@ -57,121 +55,132 @@ CRAW_DEV float clampf(float v, float lo, float hi)
     return fminf(fmaxf(v, lo), hi);
 }
 
-/* Level 0 of the colour field, straight from the mosaic. A CTA makes
- * kF0W x kF0H texels (2x2 quads each, so a kQW x kQH quad region):
- *   1. the clip ramp qa (the largest of the quad's four) of every quad of
- *      the region and kDilate quads around it (0 outside the grid, which
- *      is what skipping those quads gives, all ramps being >= 0), and the
- *      balanced channel sums and largest u of the region's own quads;
- *   2. the largest qa over +-kDilate along x, then along y: the 7x7 max;
- *   3. each quad's weight (1 - amax) * min(umax, 1)^2 and log chroma;
- *   4. per texel, the weighted sums over its quads in the reference's order.
- * The two 16-bit samples of a quad row are one 32-bit load (rows are
- * 16-byte aligned, a quad starts at an even column). */
-constexpr int kF0W = 16, kF0H = 8, kF0Threads = 256;
-constexpr int kQW = 2 * kF0W, kQH = 2 * kF0H;
-constexpr int kAW = kQW + 2 * kDilate, kAH = kQH + 2 * kDilate;
+/* Part of the frame's quads for walking warps: strips of columns, `nx`
+ * across, in segments of `seg` quad rows. */
+struct HlGrid {
+    int nx, seg;
+};
 
-__global__ void __launch_bounds__(kF0Threads) k_hl_level0(const CRAWKHighlight k, const CRAWKHighlightIO io)
+constexpr int kWalkWarps = 4, kWalkNT = 32 * kWalkWarps;
+
+/* Level 0 of the colour field, straight from the mosaic, by walking warps: a
+ * lane owns two quad columns (a column of texels) and walks down a segment of
+ * quad rows. A quad row's clip ramps qa (the largest of a quad's four; 0
+ * outside the grid, which is what skipping those quads gives, all ramps being
+ * >= 0) give their largest over +-kDilate along x by shuffles and along y
+ * from the rows before, so that kDilate rows later a quad's weight
+ * (1 - amax) min(umax, 1)^2 is known, and its log chroma is formed where the
+ * weight is not 0. A texel sums its quads in the reference's order: rows,
+ * then columns. kL0N lanes have outputs; two on either side are their apron.
+ *
+ * Bound: instruction issue (two IEEE divisions and two logarithms a quad with
+ * a weight). 6000x4000: 55 us, where 32x16 tiles staged in shared memory with
+ * their apron (1.6 times the quads) took 72. */
+constexpr int kL0N = 28, kL0Ctas = 6;
+static_assert(kDilate == 3, "two lanes of apron, a window of 7");
+
+__global__ void __launch_bounds__(kWalkNT, kL0Ctas)
+k_hl_level0(const CRAWKHighlight k, const CRAWKHighlightIO io, const HlGrid g)
 {
-    __shared__ float qa_s[kAH][kAW];
-    __shared__ float hx_s[kAH][kQW];
-    __shared__ float4 q_s[kQH][kQW];
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
+    const int sx = wid % g.nx, y0 = wid / g.nx * g.seg;
     const int qw = k.width / 2, qh = k.height / 2;
-    const int qx0 = blockIdx.x * kQW, qy0 = blockIdx.y * kQH;
-
-    /* Every load of the thread first, then their use. */
-    constexpr int kIt = (kAW * kAH + kF0Threads - 1) / kF0Threads;
-    uint32_t p0s[kIt], p1s[kIt];
-#pragma unroll
-    for (int it = 0; it < kIt; it++) {
-        const int i = threadIdx.x + it * kF0Threads, ay = i / kAW, ax = i - ay * kAW;
-        const int qx = qx0 - kDilate + ax, qy = qy0 - kDilate + ay;
-        if (i < kAW * kAH && qx >= 0 && qy >= 0 && qx < qw && qy < qh) {
-            const char *row = (const char *)io.src + (size_t)(2 * qy) * io.src_pitch + (size_t)qx * 4;
-            p0s[it] = __ldg(reinterpret_cast<const uint32_t *>(row));
-            p1s[it] = __ldg(reinterpret_cast<const uint32_t *>(row + io.src_pitch));
-        }
-    }
-#pragma unroll
-    for (int it = 0; it < kIt; it++) {
-        const int i = threadIdx.x + it * kF0Threads, ay = i / kAW, ax = i - ay * kAW;
-        const int qx = qx0 - kDilate + ax, qy = qy0 - kDilate + ay;
-        if (i >= kAW * kAH)
-            break;
-        float m = 0.0f;
-        if (qx >= 0 && qy >= 0 && qx < qw && qy < qh) {
-            const uint32_t p0 = p0s[it], p1 = p1s[it];
-            const float u[4] = { site_u(k, (uint16_t)(p0 & 0xffffu), 0), site_u(k, (uint16_t)(p0 >> 16), 1),
-                                 site_u(k, (uint16_t)(p1 & 0xffffu), 2), site_u(k, (uint16_t)(p1 >> 16), 3) };
-#pragma unroll
-            for (int s = 0; s < 4; s++)
-                m = fmax0(m, smooth(u[s]));
-            const int cx = ax - kDilate, cy = ay - kDilate;
-            if (cx >= 0 && cy >= 0 && cx < kQW && cy < kQH) {
-                float rgb[3] = { 0.0f, 0.0f, 0.0f }, umax = 0.0f;
-#pragma unroll
-                for (int s = 0; s < 4; s++) {
-                    const int c = site_chan(s);
-                    rgb[c] += u[s] * k.wb[c];
-                    umax = fmax0(umax, u[s]);
-                }
-                q_s[cy][cx] = make_float4(rgb[0], rgb[1], rgb[2], umax);
+    if (y0 >= qh)
+        return;
+    const int y1 = min(y0 + g.seg, qh);
+    const int tx = sx * kL0N + lane - 2, qx = 2 * tx;        /* the lane's texel, its first quad */
+    const bool in0 = qx >= 0 && qx < qw, in1 = qx >= 0 && qx + 1 < qw;
+    const bool mine = lane >= 2 && lane < 2 + kL0N && tx < k.lw[0];
+    /* Quad row y of the lane's quads: top rows' samples, then bottom rows'. */
+    auto fetch = [&](int y) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (in0 && y >= 0 && y < qh) {
+            const char *row = (const char *)io.src + (size_t)(2 * y) * io.src_pitch + (size_t)qx * 4;
+            if (in1) {
+                const uint2 a = __ldg(reinterpret_cast<const uint2 *>(row));
+                const uint2 b = __ldg(reinterpret_cast<const uint2 *>(row + io.src_pitch));
+                v = make_uint4(a.x, a.y, b.x, b.y);
+            } else {
+                v.x = __ldg(reinterpret_cast<const uint32_t *>(row));
+                v.z = __ldg(reinterpret_cast<const uint32_t *>(row + io.src_pitch));
             }
         }
-        qa_s[ay][ax] = m;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kAH * kQW; i += kF0Threads) {
-        const int r = i / kQW, c = i - r * kQW;
-        float m = 0.0f;
+        return v;
+    };
+    auto levels = [&](const uint4 &v, int i, float u[4]) {
+        const uint32_t p0 = i ? v.y : v.x, p1 = i ? v.w : v.z;
+        u[0] = site_u(k, (uint16_t)(p0 & 0xffffu), 0);
+        u[1] = site_u(k, (uint16_t)(p0 >> 16), 1);
+        u[2] = site_u(k, (uint16_t)(p1 & 0xffffu), 2);
+        u[3] = site_u(k, (uint16_t)(p1 >> 16), 3);
+    };
+    /* Of the rows before: the samples of three, and the running maxima over
+     * one, two and four rows that the seven are made of. */
+    uint4 raw1 = make_uint4(0u, 0u, 0u, 0u), raw2 = raw1, raw3 = raw1, next = fetch(y0 - kDilate);
+    float h1[2] = { 0.0f, 0.0f }, m2a[2] = { 0.0f, 0.0f }, m2b[2] = { 0.0f, 0.0f };
+    float m4a[2] = { 0.0f, 0.0f }, m4b[2] = { 0.0f, 0.0f }, m4c[2] = { 0.0f, 0.0f };
+    float acc[3] = { 0.0f, 0.0f, 0.0f };
+#pragma unroll 1
+    for (int y = y0 - kDilate; y < y1 + kDilate; y++) {
+        const uint4 raw = next;
+        next = fetch(y + 1);
+        float m[2];
 #pragma unroll
-        for (int d = 0; d <= 2 * kDilate; d++)
-            m = fmax0(m, qa_s[r][c + d]);
-        hx_s[r][c] = m;
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < kQH * kQW; i += kF0Threads) {
-        const int r = i / kQW, c = i - r * kQW;
-        float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (qx0 + c < qw && qy0 + r < qh) {
-            float amax = 0.0f;
+        for (int i = 0; i < 2; i++) {
+            float u[4];
+            levels(raw, i, u);
+            const float t = fmaxf(fmaxf(smooth(u[0]), smooth(u[1])), fmaxf(smooth(u[2]), smooth(u[3])));
+            m[i] = (i ? in1 : in0) && y >= 0 && y < qh ? t : 0.0f;
+        }
+        const float p = fmaxf(m[0], m[1]);
+        const float t = fmaxf(fmaxf(__shfl_up_sync(0xffffffffu, p, 1), p), __shfl_down_sync(0xffffffffu, p, 1));
+        const float h[2] = { fmaxf(t, __shfl_up_sync(0xffffffffu, m[1], 2)),
+                             fmaxf(t, __shfl_down_sync(0xffffffffu, m[0], 2)) };
+        const int r = y - kDilate;
+        float amax[2];
 #pragma unroll
-            for (int d = 0; d <= 2 * kDilate; d++)
-                amax = fmax0(amax, hx_s[r + d][c]);
-            const float4 q = q_s[r][c];
-            const float g0 = q.y * 0.5f, umax = q.w;
-            const float m = umax < 1.0f ? umax : 1.0f;
-            const float wq = (1.0f - amax) * m * m;
-            /* At weight 0 the products are +-0 (the logs are clamped, so
-             * finite) and add nothing to a sum that is never -0. */
-            if (wq != 0.0f) {
-                const float g = fmax0(g0, kEps);
-                const float lr = clampf(logf(__fdiv_rn(fmax0(q.x, kEps), g)), -kLogMax, kLogMax);
-                const float lb = clampf(logf(__fdiv_rn(fmax0(q.z, kEps), g)), -kLogMax, kLogMax);
-                t = make_float4(wq * lr, wq * lb, wq, 0.0f);
+        for (int i = 0; i < 2; i++) {
+            const float m2 = fmaxf(h[i], h1[i]), m4 = fmaxf(m2, m2b[i]);
+            amax[i] = fmaxf(m4, m4c[i]);         /* rows y - 6 .. y */
+            h1[i] = h[i];
+            m2b[i] = m2a[i];
+            m2a[i] = m2;
+            m4c[i] = m4b[i];
+            m4b[i] = m4a[i];
+            m4a[i] = m4;
+        }
+        if (r >= y0) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                float u[4];
+                levels(raw3, i, u);
+                float umax = 0.0f;
+#pragma unroll
+                for (int s = 0; s < 4; s++)
+                    umax = fmaxf(umax, u[s]);
+                const float w = umax < 1.0f ? umax : 1.0f;
+                const float wq = mine && (i ? in1 : in0) ? (1.0f - amax[i]) * w * w : 0.0f;
+                /* At weight 0 the products are +-0 (the logs are clamped, so
+                 * finite) and add nothing to a sum that is never -0. */
+                if (wq != 0.0f) {
+                    const float g0 = (u[1] * k.wb[1] + u[2] * k.wb[1]) * 0.5f, gg = fmax0(g0, kEps);
+                    const float lr = clampf(logf(__fdiv_rn(fmax0(u[0] * k.wb[0], kEps), gg)), -kLogMax, kLogMax);
+                    const float lb = clampf(logf(__fdiv_rn(fmax0(u[3] * k.wb[2], kEps), gg)), -kLogMax, kLogMax);
+                    acc[0] += wq * lr;
+                    acc[1] += wq * lb;
+                    acc[2] += wq;
+                }
+            }
+            if ((r & 1) || r == qh - 1) {
+                if (mine)
+                    reinterpret_cast<float4 *>(io.levels)[k.off[0] + (size_t)(r >> 1) * k.lw[0] + tx] =
+                        make_float4(acc[0], acc[1], acc[2], 0.0f);
+                acc[0] = acc[1] = acc[2] = 0.0f;
             }
         }
-        q_s[r][c] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x < kF0W * kF0H) {
-        const int tx = threadIdx.x % kF0W, ty = threadIdx.x / kF0W;
-        const int bx = blockIdx.x * kF0W + tx, by = blockIdx.y * kF0H + ty;
-        if (bx < k.lw[0] && by < k.lh[0]) {
-            float acc0 = 0.0f, acc1 = 0.0f, acc2 = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 2; j++)
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const float4 q = q_s[2 * ty + j][2 * tx + i];
-                    acc0 += q.x;
-                    acc1 += q.y;
-                    acc2 += q.z;
-                }
-            float4 *l0 = reinterpret_cast<float4 *>(io.levels) + k.off[0];
-            l0[(size_t)by * k.lw[0] + bx] = make_float4(acc0, acc1, acc2, 0.0f);
-        }
+        raw3 = raw2;
+        raw2 = raw1;
+        raw1 = raw;
     }
 }
 
@@ -300,25 +309,17 @@ CRAW_DEV float lift(float xc, float a, float s1, float inv_n1, float m1, float s
     const float lc = logf(fmax0(xc, kEps)) - rhoc;
     const float A = a1 + a2;
     const float lfull = expf(fmax0(lc, fmax0(l1, l2)));
-    const float lpart = A > 0.0f ? expf(__fdiv_rn(a1 * l1 + a2 * l2, A)) : lfull;
-    const float L = lfull + (A < 1.0f ? A : 1.0f) * (lpart - lfull);
+    float L = lfull;
+    if (A > 0.0f) {
+        const float lpart = expf(__fdiv_rn(a1 * l1 + a2 * l2, A));
+        L = lfull + (A < 1.0f ? A : 1.0f) * (lpart - lfull);
+    }
     return xc + a * fmax0(L * expf(rhoc) - xc, 0.0f);
 }
 
-/* A CTA rebuilds kFillW x kFillH quads, one a thread. The u and ramp of
- * its samples and a one-sample apron (mirrored at the frame's edge;
- * mirroring keeps parity) are staged in shared memory once; staged
- * column j holds frame column X0 - 2 + j, so a quad's own pair is an
- * aligned float2. A quad none of whose sites is near the clip only scales
- * its four samples; otherwise its 4x4 window (cell (r, c) = frame position
- * (x0 - 1 + c, y0 - 1 + r), CFA site ((r + 1) & 1) * 2 + ((c + 1) & 1),
- * known at compile time) is read and each site whose ramp is above 0 is
- * lifted. Neighbours of each channel are summed in the reference's scan
- * order (rows, then columns). */
-/* The mirror of a staged position: one reflection, which is exact for
- * the positions a window reads (at most one sample outside the frame),
- * then a clamp that keeps the positions no window reads (a tile hanging
- * past a small frame) inside it. */
+/* The mirror of a row: one reflection, which is exact for the rows a window
+ * reads (at most one outside the frame), then a clamp that keeps the rows no
+ * window reads inside it. */
 CRAW_DEV int edge(int v, int n)
 {
     v = v < 0 ? -v : v;
@@ -326,133 +327,153 @@ CRAW_DEV int edge(int v, int n)
     return v < 0 ? 0 : v;
 }
 
-constexpr int kFillW = 32, kFillH = 8, kFillThreads = kFillW * kFillH;
-constexpr int kStH = 2 * kFillH + 2, kStPitch = 2 * kFillW + 4, kStPairs = kStPitch / 2;
-constexpr int kStN = kStPairs * kStH, kStIt = (kStN + kFillThreads - 1) / kFillThreads;
+/* One row of a quad's 4x4 window: u and the ramp of its own pair of samples
+ * (cells 1 and 2) and of the neighbours' (0 and 3), mirrored at the frame's
+ * edge (mirroring keeps parity). */
+struct HlRow {
+    float u[4], a[4];
+};
 
-__global__ void __launch_bounds__(kFillThreads) k_hl_fill(const CRAWKHighlight k, const CRAWKHighlightIO io)
+/* The rebuilt mosaic by walking warps: a lane owns a quad column and walks
+ * down a segment of quad rows, a lane of apron on either side; the 4x4 window
+ * of the quad (cell (r, c) = frame position (x0 - 1 + c, y0 - 1 + r), CFA
+ * site ((r + 1) & 1) * 2 + ((c + 1) & 1)) stays in its registers. A quad none
+ * of whose sites is near the clip only scales its four samples; otherwise
+ * each site whose ramp is above 0 is lifted. Neighbours of each channel are
+ * summed in the reference's scan order (rows, then columns).
+ *
+ * Bound: instruction issue, the lifts' logarithms and exponentials above all
+ * where a frame is clipped: so short segments, which the hardware hands out
+ * as CTAs end (one wave of 67 rows each took 152 us, 16 rows 113). 6000x4000,
+ * most of it clipped: 105 us, where tiles staged in shared memory took 126. */
+constexpr int kFillN = 30, kFillCtas = 7, kFillSeg = 8;
+
+__global__ void __launch_bounds__(kWalkNT, kFillCtas)
+k_hl_fill(const CRAWKHighlight k, const CRAWKHighlightIO io, const HlGrid g)
 {
-    __shared__ __align__(16) float u_s[kStH][kStPitch];
-    __shared__ __align__(16) float a_s[kStH][kStPitch];
-    const int X0 = blockIdx.x * 2 * kFillW, Y0 = blockIdx.y * 2 * kFillH;
-    const int tid = threadIdx.y * kFillW + threadIdx.x;
-    /* Staged in pairs of samples (an even frame column and the next: one
-     * 32-bit load inside the frame, two mirrored loads past its edge), all
-     * of a thread's loads first, then their use. X0 and Y0 are even, so a
-     * staged sample's CFA site follows from its staged row and column. */
-    uint32_t raw[kStIt];
-#pragma unroll
-    for (int it = 0; it < kStIt; it++) {
-        const int i = tid + it * kFillThreads, r = i / kStPairs, xa = X0 - 2 + 2 * (i - r * kStPairs);
-        if (i < kStN) {
-            const int yr = edge(Y0 - 1 + r, k.height);
-            const uint16_t *row = reinterpret_cast<const uint16_t *>(
-                (const char *)io.src + (size_t)yr * io.src_pitch);
-            if (!craw_in_bounds(yr >= 0 && yr < k.height, io.err))
-                raw[it] = 0u;
-            else if (xa >= 0 && xa + 1 < k.width)
-                raw[it] = __ldg(reinterpret_cast<const uint32_t *>(row + xa));
-            else
-                raw[it] = (uint32_t)__ldg(row + edge(xa, k.width)) |
-                          ((uint32_t)__ldg(row + edge(xa + 1, k.width)) << 16);
-        }
-    }
-#pragma unroll
-    for (int it = 0; it < kStIt; it++) {
-        const int i = tid + it * kFillThreads, r = i / kStPairs, j = 2 * (i - r * kStPairs);
-        if (i < kStN) {
-            /* The sites' constants by selects, not a runtime index into
-             * the parameter block. */
-            const bool odd_row = !(r & 1);
-            const float b0 = odd_row ? k.black[2] : k.black[0], b1 = odd_row ? k.black[3] : k.black[1];
-            const float i0 = odd_row ? k.inv_range[2] : k.inv_range[0];
-            const float i1 = odd_row ? k.inv_range[3] : k.inv_range[1];
-            const float v0 = ((float)(raw[it] & 0xffffu) * (1.0f / 65535.0f) - b0) * i0;
-            const float v1 = ((float)(raw[it] >> 16) * (1.0f / 65535.0f) - b1) * i1;
-            *reinterpret_cast<float2 *>(&u_s[r][j]) = make_float2(v0, v1);
-            *reinterpret_cast<float2 *>(&a_s[r][j]) = make_float2(smooth(v0), smooth(v1));
-        }
-    }
-    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
+    const int sx = wid % g.nx, q0 = wid / g.nx * g.seg;
     const int qw = k.width / 2, qh = k.height / 2;
-    const int qx = blockIdx.x * kFillW + threadIdx.x, qy = blockIdx.y * kFillH + threadIdx.y;
-    if (qx >= qw || qy >= qh)
+    if (q0 >= qh)
         return;
-    const int x0 = 2 * qx, y0 = 2 * qy;
-    const int sr = 2 * threadIdx.y, sc = 2 * threadIdx.x + 1;   /* window cell (0, 0) */
-    const float2 uc0 = *reinterpret_cast<const float2 *>(&u_s[sr + 1][sc + 1]);
-    const float2 uc1 = *reinterpret_cast<const float2 *>(&u_s[sr + 2][sc + 1]);
-    const float2 ac0 = *reinterpret_cast<const float2 *>(&a_s[sr + 1][sc + 1]);
-    const float2 ac1 = *reinterpret_cast<const float2 *>(&a_s[sr + 2][sc + 1]);
+    const int q1 = min(q0 + g.seg, qh), qx = sx * kFillN + lane - 1, x0 = 2 * qx;
+    const bool in = qx >= 0 && qx < qw, mine = in && lane >= 1 && lane <= kFillN;
+    const bool first = qx == 0, last = qx == qw - 1;
+    auto fetch = [&](int y) {
+        const int yr = edge(y, k.height);
+        if (!in || !craw_in_bounds(yr >= 0 && yr < k.height, io.err))
+            return 0u;
+        return __ldg(reinterpret_cast<const uint32_t *>((const char *)io.src + (size_t)yr * io.src_pitch) + qx);
+    };
+    auto row = [&](uint32_t raw, int odd) {
+        HlRow r;
+        r.u[1] = site_u(k, (uint16_t)(raw & 0xffffu), 2 * odd);
+        r.u[2] = site_u(k, (uint16_t)(raw >> 16), 2 * odd + 1);
+        r.a[1] = smooth(r.u[1]);
+        r.a[2] = smooth(r.u[2]);
+        const float ul = __shfl_up_sync(0xffffffffu, r.u[2], 1), ur = __shfl_down_sync(0xffffffffu, r.u[1], 1);
+        const float al = __shfl_up_sync(0xffffffffu, r.a[2], 1), ar = __shfl_down_sync(0xffffffffu, r.a[1], 1);
+        r.u[0] = first ? r.u[2] : ul;
+        r.a[0] = first ? r.a[2] : al;
+        r.u[3] = last ? r.u[1] : ur;
+        r.a[3] = last ? r.a[1] : ar;
+        return r;
+    };
     const float wr = k.wb[0], wg = k.wb[1], wbl = k.wb[2];
-    float out[2][2];
-    out[0][0] = uc0.x * wr;
-    out[0][1] = uc0.y * wg;
-    out[1][0] = uc1.x * wg;
-    out[1][1] = uc1.y * wbl;
-    if (ac0.x > 0.0f || ac0.y > 0.0f || ac1.x > 0.0f || ac1.y > 0.0f) {
-        float u[4][4], ar[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                u[r][c] = u_s[sr + r][sc + c];
-                ar[r][c] = a_s[sr + r][sc + c];
+    HlRow w[4];                          /* rows 2q - 1 .. 2q + 2 */
+    {
+        const uint32_t a = fetch(2 * q0 - 1), b = fetch(2 * q0);
+        w[2] = row(a, 1);
+        w[3] = row(b, 0);
+    }
+    uint32_t next[2] = { fetch(2 * q0 + 1), fetch(2 * q0 + 2) };
+#pragma unroll 1
+    for (int q = q0; q < q1; q++) {
+        w[0] = w[2];
+        w[1] = w[3];
+        w[2] = row(next[0], 1);
+        w[3] = row(next[1], 0);
+        next[0] = fetch(2 * q + 3);
+        next[1] = fetch(2 * q + 4);
+        float out[2][2];
+        out[0][0] = w[1].u[1] * wr;
+        out[0][1] = w[1].u[2] * wg;
+        out[1][0] = w[2].u[1] * wg;
+        out[1][1] = w[2].u[2] * wbl;
+        if (mine && (w[1].a[1] > 0.0f || w[1].a[2] > 0.0f || w[2].a[1] > 0.0f || w[2].a[2] > 0.0f)) {
+#define U(r, c) w[r].u[c]
+#define A(r, c) w[r].a[c]
+            float lf[2];
+            bilinear(reinterpret_cast<const float4 *>(io.levels) + k.off[0], k.lw[0], k.lh[0],
+                     (float)qx * 0.5f - 0.25f, (float)q * 0.5f - 0.25f, false, lf);
+            /* R at cell (1, 1): G on the cross, B on the diagonals. */
+            if (A(1, 1) > 0.0f) {
+                float sg = 0.0f, mg = 0.0f, sb = 0.0f, mb = 0.0f;
+                sb += U(0, 0) * wbl; mb = fmax0(mb, A(0, 0));
+                sg += U(0, 1) * wg;  mg = fmax0(mg, A(0, 1));
+                sb += U(0, 2) * wbl; mb = fmax0(mb, A(0, 2));
+                sg += U(1, 0) * wg;  mg = fmax0(mg, A(1, 0));
+                sg += U(1, 2) * wg;  mg = fmax0(mg, A(1, 2));
+                sb += U(2, 0) * wbl; mb = fmax0(mb, A(2, 0));
+                sg += U(2, 1) * wg;  mg = fmax0(mg, A(2, 1));
+                sb += U(2, 2) * wbl; mb = fmax0(mb, A(2, 2));
+                out[0][0] = lift(out[0][0], A(1, 1), sg, 0.25f, mg, sb, 0.25f, mb, 0.0f, lf[1], lf[0]);
             }
-        float lf[2];
-        bilinear(reinterpret_cast<const float4 *>(io.levels) + k.off[0], k.lw[0], k.lh[0],
-                 (float)qx * 0.5f - 0.25f, (float)qy * 0.5f - 0.25f, false, lf);
-        /* R at cell (1, 1): G on the cross, B on the diagonals. */
-        if (ar[1][1] > 0.0f) {
-            float sg = 0.0f, mg = 0.0f, sb = 0.0f, mb = 0.0f;
-            sb += u[0][0] * wbl; mb = fmax0(mb, ar[0][0]);
-            sg += u[0][1] * wg;  mg = fmax0(mg, ar[0][1]);
-            sb += u[0][2] * wbl; mb = fmax0(mb, ar[0][2]);
-            sg += u[1][0] * wg;  mg = fmax0(mg, ar[1][0]);
-            sg += u[1][2] * wg;  mg = fmax0(mg, ar[1][2]);
-            sb += u[2][0] * wbl; mb = fmax0(mb, ar[2][0]);
-            sg += u[2][1] * wg;  mg = fmax0(mg, ar[2][1]);
-            sb += u[2][2] * wbl; mb = fmax0(mb, ar[2][2]);
-            out[0][0] = lift(out[0][0], ar[1][1], sg, 0.25f, mg, sb, 0.25f, mb, 0.0f, lf[1], lf[0]);
+            /* Gr at cell (1, 2): R left and right, B above and below. */
+            if (A(1, 2) > 0.0f) {
+                float sr = 0.0f, mr = 0.0f, sb = 0.0f, mb = 0.0f;
+                sb += U(0, 2) * wbl; mb = fmax0(mb, A(0, 2));
+                sr += U(1, 1) * wr;  mr = fmax0(mr, A(1, 1));
+                sr += U(1, 3) * wr;  mr = fmax0(mr, A(1, 3));
+                sb += U(2, 2) * wbl; mb = fmax0(mb, A(2, 2));
+                out[0][1] = lift(out[0][1], A(1, 2), sr, 0.5f, mr, sb, 0.5f, mb, lf[0], lf[1], 0.0f);
+            }
+            /* Gb at cell (2, 1): R above and below, B left and right. */
+            if (A(2, 1) > 0.0f) {
+                float sr = 0.0f, mr = 0.0f, sb = 0.0f, mb = 0.0f;
+                sr += U(1, 1) * wr;  mr = fmax0(mr, A(1, 1));
+                sb += U(2, 0) * wbl; mb = fmax0(mb, A(2, 0));
+                sb += U(2, 2) * wbl; mb = fmax0(mb, A(2, 2));
+                sr += U(3, 1) * wr;  mr = fmax0(mr, A(3, 1));
+                out[1][0] = lift(out[1][0], A(2, 1), sr, 0.5f, mr, sb, 0.5f, mb, lf[0], lf[1], 0.0f);
+            }
+            /* B at cell (2, 2): R on the diagonals, G on the cross. */
+            if (A(2, 2) > 0.0f) {
+                float sr = 0.0f, mr = 0.0f, sg = 0.0f, mg = 0.0f;
+                sr += U(1, 1) * wr;  mr = fmax0(mr, A(1, 1));
+                sg += U(1, 2) * wg;  mg = fmax0(mg, A(1, 2));
+                sr += U(1, 3) * wr;  mr = fmax0(mr, A(1, 3));
+                sg += U(2, 1) * wg;  mg = fmax0(mg, A(2, 1));
+                sg += U(2, 3) * wg;  mg = fmax0(mg, A(2, 3));
+                sr += U(3, 1) * wr;  mr = fmax0(mr, A(3, 1));
+                sg += U(3, 2) * wg;  mg = fmax0(mg, A(3, 2));
+                sr += U(3, 3) * wr;  mr = fmax0(mr, A(3, 3));
+                out[1][1] = lift(out[1][1], A(2, 2), sr, 0.25f, mr, sg, 0.25f, mg, lf[0], 0.0f, lf[1]);
+            }
+#undef U
+#undef A
         }
-        /* Gr at cell (1, 2): R left and right, B above and below. */
-        if (ar[1][2] > 0.0f) {
-            float sr = 0.0f, mr = 0.0f, sb = 0.0f, mb = 0.0f;
-            sb += u[0][2] * wbl; mb = fmax0(mb, ar[0][2]);
-            sr += u[1][1] * wr;  mr = fmax0(mr, ar[1][1]);
-            sr += u[1][3] * wr;  mr = fmax0(mr, ar[1][3]);
-            sb += u[2][2] * wbl; mb = fmax0(mb, ar[2][2]);
-            out[0][1] = lift(out[0][1], ar[1][2], sr, 0.5f, mr, sb, 0.5f, mb, lf[0], lf[1], 0.0f);
-        }
-        /* Gb at cell (2, 1): R above and below, B left and right. */
-        if (ar[2][1] > 0.0f) {
-            float sr = 0.0f, mr = 0.0f, sb = 0.0f, mb = 0.0f;
-            sr += u[1][1] * wr;  mr = fmax0(mr, ar[1][1]);
-            sb += u[2][0] * wbl; mb = fmax0(mb, ar[2][0]);
-            sb += u[2][2] * wbl; mb = fmax0(mb, ar[2][2]);
-            sr += u[3][1] * wr;  mr = fmax0(mr, ar[3][1]);
-            out[1][0] = lift(out[1][0], ar[2][1], sr, 0.5f, mr, sb, 0.5f, mb, lf[0], lf[1], 0.0f);
-        }
-        /* B at cell (2, 2): R on the diagonals, G on the cross. */
-        if (ar[2][2] > 0.0f) {
-            float sr = 0.0f, mr = 0.0f, sg = 0.0f, mg = 0.0f;
-            sr += u[1][1] * wr;  mr = fmax0(mr, ar[1][1]);
-            sg += u[1][2] * wg;  mg = fmax0(mg, ar[1][2]);
-            sr += u[1][3] * wr;  mr = fmax0(mr, ar[1][3]);
-            sg += u[2][1] * wg;  mg = fmax0(mg, ar[2][1]);
-            sg += u[2][3] * wg;  mg = fmax0(mg, ar[2][3]);
-            sr += u[3][1] * wr;  mr = fmax0(mr, ar[3][1]);
-            sg += u[3][2] * wg;  mg = fmax0(mg, ar[3][2]);
-            sr += u[3][3] * wr;  mr = fmax0(mr, ar[3][3]);
-            out[1][1] = lift(out[1][1], ar[2][2], sr, 0.25f, mr, sg, 0.25f, mg, lf[0], 0.0f, lf[1]);
-        }
-    }
+        __syncwarp();
+        if (mine)
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-        __half2 hv = __floats2half2_rn(out[r][0], out[r][1]);
-        if (craw_in_bounds(x0 >= 0 && x0 + 1 < k.width && y0 + r >= 0 && y0 + r < k.height, io.err))
-            *reinterpret_cast<__half2 *>((char *)io.dst + (size_t)(y0 + r) * io.dst_pitch + (size_t)x0 * 2) = hv;
+            for (int r = 0; r < 2; r++) {
+                const __half2 hv = __floats2half2_rn(out[r][0], out[r][1]);
+                if (craw_in_bounds(x0 >= 0 && x0 + 1 < k.width && 2 * q + r < k.height, io.err))
+                    *reinterpret_cast<__half2 *>((char *)io.dst + (size_t)(2 * q + r) * io.dst_pitch +
+                                                 (size_t)x0 * 2) = hv;
+            }
     }
+}
+
+/* Segments of one wave of `ctas` CTAs an SM for strips of `cols` quads, a
+ * multiple of 2 quad rows (texels have two), at least 8; returns the CTAs. */
+int hl_grid(HlGrid &g, int qw, int qh, int cols, int ctas)
+{
+    g.nx = (qw + cols - 1) / cols;
+    const int room = 152 * ctas * kWalkWarps / g.nx, n = room > 1 ? room : 1;
+    g.seg = ((qh + n - 1) / n + 1) / 2 * 2;
+    g.seg = g.seg < 8 ? 8 : g.seg;
+    return (g.nx * ((qh + g.seg - 1) / g.seg) + kWalkWarps - 1) / kWalkWarps;
 }
 
 dim3 grid2(int w, int h) { return dim3((w + 31) / 32, (h + 7) / 8); }
@@ -484,8 +505,9 @@ extern "C" int craw_k_highlights(const CRAWKHighlight *k, const CRAWKHighlightIO
         return -5;
     const int qw = k->width / 2, qh = k->height / 2;
     const dim3 blk(32, 8);
-    k_hl_level0<<<dim3((k->lw[0] + kF0W - 1) / kF0W, (k->lh[0] + kF0H - 1) / kF0H), kF0Threads, 0, s>>>(
-        *k, *io);
+    HlGrid g;
+    int ctas = hl_grid(g, qw, qh, 2 * kL0N, kL0Ctas);
+    k_hl_level0<<<ctas, kWalkNT, 0, s>>>(*k, *io, g);
     /* The levels from lc up are small enough for one CTA. */
     int lc = 0;
     while (lc + 1 < k->nb_levels && (int64_t)k->lw[lc] * k->lh[lc] > kCoarseTexels)
@@ -496,6 +518,8 @@ extern "C" int craw_k_highlights(const CRAWKHighlight *k, const CRAWKHighlightIO
         k_hl_coarse<<<1, kCoarseThreads, 0, s>>>(*k, *io, lc);
     for (int l = lc - 1; l >= 0; l--)
         k_hl_push<<<grid2(k->lw[l], k->lh[l]), blk, 0, s>>>(*k, *io, l);
-    k_hl_fill<<<grid2(qw, qh), blk, 0, s>>>(*k, *io);
+    g = HlGrid{ (qw + kFillN - 1) / kFillN, kFillSeg };
+    ctas = (g.nx * ((qh + g.seg - 1) / g.seg) + kWalkWarps - 1) / kWalkWarps;
+    k_hl_fill<<<ctas, kWalkNT, 0, s>>>(*k, *io, g);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }
