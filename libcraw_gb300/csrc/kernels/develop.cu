@@ -202,37 +202,6 @@ k_develop_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
     t.run(g, blockIdx.x * WALK_WARPS + (threadIdx.x >> 5));
 }
 
-/* The current device's SM count, kept per device ordinal below 64 (152,
- * GB300's, if the query fails). */
-int craw_sm_count()
-{
-    static std::atomic<int> known[64];
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess)
-        return 152;
-    if (dev >= 0 && dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0)
-        return sms;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-        return 152;
-    if (dev >= 0 && dev < 64)
-        known[dev].store(sms, std::memory_order_relaxed);
-    return sms;
-}
-
-/* Segments of one wave of `ctas` CTAs an SM: as tall as that allows (a
- * segment reads, and for the RCD computes, its first rows' surroundings
- * again), a multiple of 4 quad rows, at least `least`; g.nx strips are
- * set. Returns the CTAs. */
-unsigned walk_segments(WalkGrid &g, int ctas, int least)
-{
-    const int room = craw_sm_count() * ctas * WALK_WARPS / g.nx;
-    const int nseg = room > 1 ? room : 1;
-    g.seg = 4 * (((g.nqy + 3) / 4 + nseg - 1) / nseg);
-    g.seg = g.seg < least ? least : g.seg;
-    const int warps = g.nx * ((g.nqy + g.seg - 1) / g.seg);
-    return (unsigned)((warps + WALK_WARPS - 1) / WALK_WARPS);
-}
-
 /* The RCD of a w x h frame as strips: the interior's (w, its CTAs in inner;
  * none if the frame has none) and the border's. Segments are a multiple of 4
  * quad rows, at least 8. Either the interior takes one wave of WALK_CTAS
@@ -277,7 +246,7 @@ int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t 
     g.nqx = k->width / 2;
     g.nqy = k->height / 2;
     g.nx = (k->width + LW_P * LW_N - 1) / (LW_P * LW_N);
-    const unsigned grid = walk_segments(g, linear_ctas<METHOD, EPI>(), 4);
+    const unsigned grid = walk_segments(g, craw_sm_count(), linear_ctas<METHOD, EPI>(), 4);
     k_develop_walk<METHOD, EPI><<<grid, WALK_NT, 0, s>>>(*k, *io, g);
     return cudaGetLastError() == cudaSuccess ? 0 : -5;
 }

@@ -39,6 +39,20 @@ struct WalkGrid {
 
 constexpr int WALK_WARPS = 4, WALK_NT = 32 * WALK_WARPS;   /* warps (strips) a CTA */
 
+/* Segments of one wave of `ctas` CTAs an SM: as tall as that allows (a
+ * segment reads, and for the RCD computes, its first rows' surroundings
+ * again), a multiple of 4 quad rows, at least `least`; g.nx strips are
+ * set. Returns the CTAs. */
+inline unsigned walk_segments(WalkGrid &g, int sms, int ctas, int least)
+{
+    const int room = sms * ctas * WALK_WARPS / g.nx;
+    const int nseg = room > 1 ? room : 1;
+    g.seg = 4 * (((g.nqy + 3) / 4 + nseg - 1) / nseg);
+    g.seg = g.seg < least ? least : g.seg;
+    const int warps = g.nx * ((g.nqy + g.seg - 1) / g.seg);
+    return (unsigned)((warps + WALK_WARPS - 1) / WALK_WARPS);
+}
+
 CRAW_DEV float walk_left(float v)    /* the left neighbour's v */
 {
     return __shfl_up_sync(0xffffffffu, v, 1);
@@ -1073,14 +1087,16 @@ struct LinearWalk {
         }
     }
 
-    /* The strip of warp `wid` of the grid: the whole frame's, in strips of
-     * LW_N lanes and segments of g.seg quad rows. */
-    CRAW_DEV void run(const WalkGrid &g, int wid)
+    /* The lane's place in the strip of warp `wid` of the grid (the whole
+     * frame's, in strips of LW_N lanes and segments of g.seg quad rows): its
+     * segment's pixel rows are y0 .. y0 + rows; false where there is none. */
+    CRAW_DEV bool place(const WalkGrid &g, int wid, int &y0, int &rows)
     {
         const int lane = threadIdx.x & 31, sx = wid % g.nx, sy = wid / g.nx;
         if (sy * g.seg >= g.nqy)
-            return;
-        const int y0 = 2 * sy * g.seg, rows = 2 * min(g.seg, g.nqy - sy * g.seg);
+            return false;
+        y0 = 2 * sy * g.seg;
+        rows = 2 * min(g.seg, g.nqy - sy * g.seg);
         x0 = LW_P * (sx * LW_N - 1 + lane);
         edge = sx == 0 || LW_P * (sx * LW_N + 31) >= k.width;
         inside = x0 >= 0 && x0 + LW_P <= k.width;
@@ -1096,7 +1112,14 @@ struct LinearWalk {
         dst = (char *)io.dst + (size_t)y0 * io.dst_pitch +
               (ptrdiff_t)x0 * (f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16));
         inter = (char *)io.inter + (size_t)y0 * io.inter_pitch + (ptrdiff_t)x0 * (k.fp16 ? 8 : 16);
+        return true;
+    }
 
+    CRAW_DEV void run(const WalkGrid &g, int wid)
+    {
+        int y0, rows;
+        if (!place(g, wid, y0, rows))
+            return;
         int y = y0;
         const char *src = (const char *)io.src + (size_t)y0 * io.src_pitch;
         auto fetch = [&]() {
