@@ -345,7 +345,7 @@ CRAW_API int craw_batch_record(CRAWBatch *b, cudaStream_t s, uint32_t nb, const 
     for (uint32_t d = 0; d < nd; d++) {
         if ((ddn[d] && craw_k_denoise(&b->direct[d].dn, &b->direct[d].dio, b->direct_shape, NULL, NULL,
                                       b->direct[d].vio.err, s) < 0) ||
-            craw_k_develop(&b->direct[d].dv, &b->direct[d].vio, 0, s) < 0)
+            craw_k_develop(&b->direct[d].dv, &b->direct[d].vio, ddn[d], s) < 0)
             return CRAW_ERROR(EIO);
         b->direct_frames++;
     }

@@ -85,7 +85,7 @@ struct CRAWPipeline {
     uint16_t *hl_mosaic;         /* the rebuilt mosaic, fp16 */
     size_t hl_pitch;
     void *hl_levels;            /* the colour field's pyramid */
-    int dn_shape[2], dev_shape;   /* denoise tile shape without / with a history */
+    int dn_shape[2];              /* denoise tile shape without / with a history */
     bool tune_held;              /* holds its size's autotuner cache entry */
 
     /* Device memory. */
@@ -858,7 +858,7 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
             dio.inter_pitch = p->inter_pitch;
         }
         prof_begin(&pc, ST_DEVELOP);
-        ret = craw_k_develop(&dk, &dio, p->dev_shape, s);
+        ret = craw_k_develop(&dk, &dio, denoise || dio.src_f16, s);
         prof_end(&pc);
         if (ret < 0)
             goto launch_fail;
@@ -870,7 +870,7 @@ CRAW_API int craw_pipeline_record(CRAWPipeline *p, cudaStream_t s, const CRAWIma
         dio.quarter_pitch = p->q_pitch;
         dio.awb = none;
         prof_begin(&pc, ST_DEVELOP);
-        ret = craw_k_develop(&dk, &dio, p->dev_shape, s);
+        ret = craw_k_develop(&dk, &dio, denoise || dio.src_f16, s);
         prof_end(&pc);
         if (ret < 0)
             goto launch_fail;

@@ -222,8 +222,10 @@ typedef struct CRAWKDevelopIO {
 #define CRAW_K_ERR_BOUNDS 2u
 
 /* Prep + debayer + (colour to dst | chroma block means) + AWB statistic +
- * optional intermediate, in one kernel. */
-int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int shape,
+ * optional intermediate, in one kernel. `early`: the stream's last work is a
+ * kernel of this library, which the first develop kernel may be launched as
+ * a programmatic dependent of. */
+int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int early,
                    cudaStream_t s);
 
 /* Readies the develop kernels of a debayer method on the current device

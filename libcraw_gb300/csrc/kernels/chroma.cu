@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(BX * BY)
 k_chroma_blur(const CRAWKChroma c, const void *q, size_t q_pitch, void *qf, size_t qf_pitch)
 {
     __shared__ float4 t[(BY + 2 * kR) * (BX + 2 * kR)];
+    craw_let_next_start();
     constexpr int SX = BX + 2 * kR;
     const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY;
     for (int i = threadIdx.x; i < (BY + 2 * kR) * SX; i += BX * BY) {
@@ -254,6 +255,9 @@ k_chroma_up_color(const CRAWKDevelop k, const CRAWKDevelopIO io, const CRAWKChro
                   size_t inter_pitch, const void *q, const void *qf, size_t q_pitch, const WalkGrid g)
 {
     __shared__ __align__(16) char ring[WALK_WARPS][kUpRows * kUpRowBytes];
+    craw_await_previous();
+    if (io.awb.hist)
+        craw_let_next_start();
     ChromaWalk<EPI> t(k, io, c);
     t.ring = ring[threadIdx.x >> 5];
     t.inter_in = (const char *)inter;
@@ -304,6 +308,6 @@ extern "C" int craw_k_chroma_up_color(const CRAWKDevelop *k, const CRAWKChroma *
         kernel = dst_fmt == CRAW_K_OUT_RGBA16F  ? k_chroma_up_color<CRAW_K_OUT_RGBA16F>
                  : dst_fmt == CRAW_K_OUT_RGB32F ? k_chroma_up_color<CRAW_K_OUT_RGB32F>
                                                 : k_chroma_up_color<CRAW_K_OUT_RGBA32F>;
-    kernel<<<ctas, WALK_NT, 0, s>>>(*k, io, *c, inter, inter_pitch, q, qf, q_pitch, g);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return craw_launch_early(kernel, (int)ctas, WALK_NT, 0, true, s, *k, io, *c, inter, inter_pitch, q, qf, q_pitch,
+                             g);
 }

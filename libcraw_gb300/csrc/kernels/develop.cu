@@ -72,21 +72,15 @@ struct QuadGrid {
  * begin at once (programmatic dependent launch): the two write disjoint
  * tiles, and the border CTAs take the SM slots that the interior leaves
  * free. The border ends no earlier than the interior, so that what comes
- * after it on the stream, or depends on it in a graph, waits for both. */
-CRAW_DEV void release_border()
-{
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-CRAW_DEV void await_interior()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+ * after it on the stream, or depends on it in a graph, waits for both. The
+ * border and the linear kernels let the AWB histogram's publication, which
+ * waits for them, be launched meanwhile. */
 
 __global__ void __launch_bounds__(QNT)
 k_develop_rcd_quads(const CRAWKDevelop k, const CRAWKDevelopIO io, const QuadGrid g)
 {
     extern __shared__ __align__(16) float smem[];
-    release_border();
+    craw_let_next_start();
     rcd_quad_tile(k, io, (g.c_lo + blockIdx.x) * QTW, (g.r_lo + blockIdx.y) * QTH, smem);
 }
 
@@ -106,7 +100,7 @@ k_develop_rcd_quads_tma(const CRAWKDevelop k, const CRAWKDevelopIO io, const Qua
 {
     extern __shared__ __align__(16) float smem[];
     __shared__ __align__(8) uint64_t bar_s;
-    release_border();
+    craw_let_next_start();
     const int x0 = (g.c_lo + blockIdx.x) * QTW, y0 = (g.r_lo + blockIdx.y) * QTH;
     RcdQuads<QTW, QTH, QNT> t;
     t.carve(smem);
@@ -141,7 +135,8 @@ __global__ void __launch_bounds__(WALK_NT, WALK_CTAS)
 k_develop_rcd_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
 {
     __shared__ WalkSmem<RW_NQ> smem[WALK_WARPS];
-    release_border();
+    craw_await_previous();
+    craw_let_next_start();
     const int warp = threadIdx.x >> 5;
     rcd_walk<FMT, RGC, MORE>(k, io, g, blockIdx.x * WALK_WARPS + warp, smem[warp]);
 }
@@ -158,6 +153,8 @@ __global__ void __launch_bounds__(WALK_NT, WALK_CTAS)
 k_develop_rcd_ring(const CRAWKDevelop k, const CRAWKDevelopIO io, const __grid_constant__ RingGrid ring)
 {
     __shared__ WalkSmem<RW_NQ> smem[WALK_WARPS];
+    if (io.awb.hist)
+        craw_let_next_start();
     const int warp = threadIdx.x >> 5;
     const int wid = blockIdx.x * WALK_WARPS + warp;
     int part = 0;
@@ -167,7 +164,7 @@ k_develop_rcd_ring(const CRAWKDevelop k, const CRAWKDevelopIO io, const __grid_c
             part = i;
     if (wid < ring.first[4])
         ring_walk<FMT, RGC, MORE>(k, io, ring.g[part], wid - ring.first[part], smem[warp]);
-    await_interior();
+    craw_await_previous();
 }
 
 /* The per-pixel RCD on the ring of border quad tiles, BTW x BTH pixels a
@@ -183,7 +180,7 @@ k_develop_rcd_border(const CRAWKDevelop k, const CRAWKDevelopIO io, const QuadGr
     const int x0 = col * QTW + (blockIdx.x % PER) * BTW, y0 = row * QTH;
     if (x0 < k.width)
         pixel_tile<kRcd, BTW, BTH, 256>(k, io, x0, y0, smem);
-    await_interior();
+    craw_await_previous();
 }
 
 /* Every bilinear and MHC frame: CTAs an SM (5 of 96 registers for MHC and 6
@@ -198,6 +195,9 @@ template <int METHOD, int EPI>
 __global__ void __launch_bounds__(WALK_NT, (linear_ctas<METHOD, EPI>()))
 k_develop_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
 {
+    craw_await_previous();
+    if (io.awb.hist)
+        craw_let_next_start();
     LinearWalk<METHOD, EPI> t(k, io);
     t.run(g, blockIdx.x * WALK_WARPS + (threadIdx.x >> 5));
 }
@@ -239,7 +239,7 @@ void rcd_grids(int width, int height, WalkGrid &w, RingGrid &ring, int &inner, i
 }
 
 template <int METHOD, int EPI>
-int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cudaStream_t s)
 {
     WalkGrid g;
     g.qx0 = g.qy0 = 0;
@@ -247,21 +247,20 @@ int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t 
     g.nqy = k->height / 2;
     g.nx = (k->width + LW_P * LW_N - 1) / (LW_P * LW_N);
     const unsigned grid = walk_segments(g, craw_sm_count(), linear_ctas<METHOD, EPI>(), 4);
-    k_develop_walk<METHOD, EPI><<<grid, WALK_NT, 0, s>>>(*k, *io, g);
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
+    return craw_launch_early(k_develop_walk<METHOD, EPI>, (int)grid, WALK_NT, 0, early, s, *k, *io, g);
 }
 
 template <int METHOD>
-int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cudaStream_t s)
 {
     if (io->quarter && io->inter)
-        return launch_linear<METHOD, LW_CHROMA>(k, io, s);
+        return launch_linear<METHOD, LW_CHROMA>(k, io, early, s);
     if (io->inter || !io->dst)
-        return launch_linear<METHOD, LW_ANY>(k, io, s);
+        return launch_linear<METHOD, LW_ANY>(k, io, early, s);
     switch (io->dst_fmt) {
-    case CRAW_K_OUT_RGBA16F: return launch_linear<METHOD, CRAW_K_OUT_RGBA16F>(k, io, s);
-    case CRAW_K_OUT_RGB32F:  return launch_linear<METHOD, CRAW_K_OUT_RGB32F>(k, io, s);
-    default:                 return launch_linear<METHOD, CRAW_K_OUT_RGBA32F>(k, io, s);
+    case CRAW_K_OUT_RGBA16F: return launch_linear<METHOD, CRAW_K_OUT_RGBA16F>(k, io, early, s);
+    case CRAW_K_OUT_RGB32F:  return launch_linear<METHOD, CRAW_K_OUT_RGB32F>(k, io, early, s);
+    default:                 return launch_linear<METHOD, CRAW_K_OUT_RGBA32F>(k, io, early, s);
     }
 }
 
@@ -277,66 +276,40 @@ int prepare_rcd()
     return 0;
 }
 
-/* The border's launch after an interior launch (`after`), which it may
- * overlap, or by itself. */
-template <typename... P, typename... A>
-int launch_border(void (*kernel)(P...), int ctas, int threads, size_t smem, bool after, cudaStream_t s, const A &...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute early[1];
-    early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = early;
-    cfg.numAttrs = after ? 1 : 0;
-    if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess && cfg.numAttrs) {
-        /* A driver that refuses the early start: the plain launch after the
-         * interior, the launch's own error cleared. */
-        (void)cudaGetLastError();
-        cfg.numAttrs = 0;
-        (void)cudaLaunchKernelEx(&cfg, kernel, args...);
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : -5;
-}
-
 /* The walking kernels of a frame. */
 template <int FMT, int RGC, bool MORE>
-int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cudaStream_t s)
 {
     WalkGrid w;
     RingGrid ring;
     int inner, border;
     rcd_grids(k->width, k->height, w, ring, inner, border);
     if (inner > 0) {
-        k_develop_rcd_walk<FMT, RGC, MORE><<<inner, WALK_NT, 0, s>>>(*k, *io, w);
-        if (cudaGetLastError() != cudaSuccess)
+        if (craw_launch_early(k_develop_rcd_walk<FMT, RGC, MORE>, inner, WALK_NT, 0, early, s, *k, *io, w) < 0)
             return -5;
     }
-    return launch_border(k_develop_rcd_ring<FMT, RGC, MORE>, border, WALK_NT, 0, inner > 0, s, *k, *io, ring);
+    return craw_launch_early(k_develop_rcd_ring<FMT, RGC, MORE>, border, WALK_NT, 0, inner > 0, s, *k, *io, ring);
 }
 
 template <int RGC>
-int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cudaStream_t s)
 {
     switch (io->dst_fmt) {
-    case CRAW_K_OUT_RGBA16F: return launch_walk<CRAW_K_OUT_RGBA16F, RGC, false>(k, io, s);
-    case CRAW_K_OUT_RGB32F:  return launch_walk<CRAW_K_OUT_RGB32F, RGC, false>(k, io, s);
-    default:                 return launch_walk<CRAW_K_OUT_RGBA32F, RGC, false>(k, io, s);
+    case CRAW_K_OUT_RGBA16F: return launch_walk<CRAW_K_OUT_RGBA16F, RGC, false>(k, io, early, s);
+    case CRAW_K_OUT_RGB32F:  return launch_walk<CRAW_K_OUT_RGB32F, RGC, false>(k, io, early, s);
+    default:                 return launch_walk<CRAW_K_OUT_RGBA32F, RGC, false>(k, io, early, s);
     }
 }
 
-int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
+int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cudaStream_t s)
 {
     constexpr size_t smem = RcdQuads<QTW, QTH, QNT>::floats * sizeof(float);
     if (prepare_rcd() < 0)
         return -5;
     if (craw_k_rcd_strips) {
         if (k->fp16 || io->inter || io->quarter || !io->dst)
-            return launch_walk<0, -1, true>(k, io, s);
-        return k->color.flags & CRAW_K_COLOR_RGC ? launch_walk<1>(k, io, s) : launch_walk<0>(k, io, s);
+            return launch_walk<0, -1, true>(k, io, early, s);
+        return k->color.flags & CRAW_K_COLOR_RGC ? launch_walk<1>(k, io, early, s) : launch_walk<0>(k, io, early, s);
     }
     QuadGrid g;
     g.init(k->width, k->height);
@@ -351,7 +324,7 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
         if (cudaGetLastError() != cudaSuccess)
             return -5;
     }
-    return g.border_quads() > 0 ? launch_border(k_develop_rcd_border, g.border_quads() * (QTW / BTW), 256,
+    return g.border_quads() > 0 ? craw_launch_early(k_develop_rcd_border, g.border_quads() * (QTW / BTW), 256,
                                                 PixelSmem<kRcd, BTW, BTH, 256>::floats * sizeof(float), interior, s,
                                                 *k, *io, g)
                                 : 0;
@@ -367,16 +340,15 @@ extern "C" int craw_k_develop_prepare(int method)
     return 0;
 }
 
-extern "C" int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int shape,
+extern "C" int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int early,
                               cudaStream_t s)
 {
     if (craw_launch_ready() < 0)
         return -5;
-    (void)shape;
     switch (k->method) {
-    case kBilinear: return launch_linear<kBilinear>(k, io, s);
-    case kMhc:      return launch_linear<kMhc>(k, io, s);
-    case kRcd:      return launch_rcd(k, io, s);
+    case kBilinear: return launch_linear<kBilinear>(k, io, early, s);
+    case kMhc:      return launch_linear<kMhc>(k, io, early, s);
+    case kRcd:      return launch_rcd(k, io, early, s);
     default:        return -22;
     }
 }
