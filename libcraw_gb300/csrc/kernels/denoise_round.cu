@@ -168,8 +168,18 @@ CRAW_DEV bool decide(const CRAWKDenoise &k, const CRAWKDenoiseExact &e, const CR
                 const float d = D[(4 + ky) * WIN + 4 + kx];
                 pc = fmaf(d, d, pc);
             }
-        for (int o = g; o < 49; o += GA) {
-            const int dy = o / 7 - 3, dx = o % 7 - 3;
+        /* The centre's own offset has distance 0 and weight 1: the other 48
+         * are a whole number of rounds. */
+        if (g == 0) {
+            const float dc = D[4 * WIN + 4], rho = U * fmaf(0.7f, fabsf(e.c0), 8.0f);
+            s = dc;
+            es = a = fabsf(dc);
+            wt = 1.0f;
+            b = rho * fabsf(dc);
+            r = rho;
+        }
+        for (int i = g; i < 48; i += GA) {
+            const int o = i + (i >= 24), dy = o / 7 - 3, dx = o % 7 - 3;
             float d2 = 0.0f, pi = 0.0f;
 #pragma unroll
             for (int ky = -1; ky <= 1; ky++)
@@ -469,8 +479,12 @@ CRAW_DEV void exact_sample(const CRAWKDenoiseExact &e, const CRAWKDenoiseIO &io,
     __syncwarp();
     dfl acc = df_from(0.0f), wsum = df_from(0.0f);
     if (valid) {
-        for (int o = g; o < 49; o += G) {
-            const int dy = o / 7 - 3, dx = o % 7 - 3;
+        if (g == 0) {      /* the centre's own offset: distance 0, weight 1 */
+            acc = df_make(Th[4 * WIN + 4], Tl[4 * WIN + 4]);
+            wsum = df_from(1.0f);
+        }
+        for (int i = g; i < 48; i += G) {
+            const int o = i + (i >= 24), dy = o / 7 - 3, dx = o % 7 - 3;
             dfl d2 = df_from(0.0f);
 #pragma unroll
             for (int ky = -1; ky <= 1; ky++)
