@@ -35,6 +35,11 @@ void craw_gamut_compress_params(CRAWGamutCompress *g);
  * allocations so a test can make the k-th one fail. */
 int craw_dev_alloc(CRAWContext *ctx, void **ptr, size_t bytes);
 void craw_dev_free(CRAWContext *ctx, void *ptr);
+
+/* Gives back what a pipeline with nothing in flight can do without, at some
+ * speed and the same results; whether there was anything. */
+bool craw_pipeline_shrink(CRAWPipeline *p);
+
 int craw_dev_sync(CRAWContext *ctx);
 
 /* craw_debug_force_denoise_shape(): -1, or the shape every new pipeline uses. */

@@ -267,6 +267,29 @@ static int time_denoise(CRAWPipeline *p, const CRAWKDenoise *k, const CRAWKDenoi
     return ret < 0 ? CRAW_ERROR(EIO) : 0;
 }
 
+/* The history's planes, if there is memory for them: without, the 2x8 shape
+ * runs the 2x4 shape's kernel (the same bits). */
+static void alloc_planes(CRAWPipeline *p, float **planes)
+{
+    if (craw_dev_alloc(p->ctx, (void **)planes, craw_k_denoise_planes((int32_t)(p->params.width / 2),
+                                                                  (int32_t)(p->params.height / 2))) < 0) {
+        (void)cudaGetLastError();
+        *planes = NULL;
+        return;
+    }
+    if (craw_dev_sync(p->ctx) < 0)
+        *planes = NULL;
+}
+
+bool craw_pipeline_shrink(CRAWPipeline *p)
+{
+    if (!p->dn_planes)
+        return false;
+    craw_dev_free(p->ctx, p->dn_planes);
+    p->dn_planes = NULL;
+    return craw_dev_sync(p->ctx) == 0;
+}
+
 static int autotune(CRAWPipeline *p)
 {
     CRAWContext *ctx = p->ctx;
@@ -299,10 +322,10 @@ static int autotune(CRAWPipeline *p)
 
     if ((ret = alloc_pitched(p, (void **)&mosaic, &mp, (size_t)w * 2, h)) < 0 ||
         (ret = alloc_pitched(p, (void **)&lvl, &lp, (size_t)w * 4, h)) < 0 ||
-        (ret = alloc_pitched(p, (void **)&var, &vp, (size_t)w, h)) < 0 ||
-        (need[1] && !p->dn_planes &&
-         (ret = craw_dev_alloc(ctx, (void **)&planes, craw_k_denoise_planes((int32_t)(w / 2), (int32_t)(h / 2)))) < 0))
+        (ret = alloc_pitched(p, (void **)&var, &vp, (size_t)w, h)) < 0)
         goto done;
+    if (need[1] && !p->dn_planes)
+        alloc_planes(p, &planes);
     /* A mid-grey mosaic, a state of level 0.25 and unit variance. */
     cudaMemset2DAsync(mosaic, mp, 0x08, (size_t)w * 2, h, ctx->stream);
     cudaMemset2DAsync(lvl, lp, 0, (size_t)w * 4, h, ctx->stream);
@@ -513,10 +536,6 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
                 (ret = alloc_pitched(p, (void **)&p->var[i], &p->var_pitch, (size_t)w, h)) < 0)
                 goto fail;
         }
-        if (p->has_denoise && !p->plain &&
-            (ret = craw_dev_alloc(ctx, (void **)&p->dn_planes,
-                                  craw_k_denoise_planes((int32_t)(w / 2), (int32_t)(h / 2)))) < 0)
-            goto fail;
     }
     if (p->has_chroma || p->keep || p->plain) {
         size_t bpp = p->fp16 ? 8 : 16;
@@ -615,12 +634,16 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
         ret = CRAW_ERROR(EIO);
         goto fail;
     }
+    if (p->has_denoise && p->has_temporal && !p->plain)
+        alloc_planes(p, &p->dn_planes);
     if (craw_forced_denoise_shape >= 0) {
         p->dn_shape[0] = p->dn_shape[1] = craw_forced_denoise_shape;
     } else if ((p->has_denoise || p->has_temporal) && !p->plain &&
                !(params->flags & CRAW_PIPELINE_FLAG_NO_AUTOTUNE) && (ret = autotune(p)) < 0) {
         goto fail;
     }
+    if (p->dn_shape[1] != CRAW_K_DN_SHAPE_2x8_X2)
+        craw_pipeline_shrink(p);
     craw_log(ctx, CRAW_LOG_VERBOSE, "pipeline %ux%u debayer %d flags 0x%x storage %s impl %s\n",
              w, h, params->debayer, params->flags, p->fp16 ? "fp16" : "fp32",
              p->plain ? "plain" : "fused");

@@ -583,6 +583,15 @@ CRAW_API int craw_server_stream_open(CRAWServer *s, const CRAWServerStreamParams
     st->bytes = after > before ? after - before : 0;
 
     pthread_mutex_lock(&s->lock);
+    if (s->resident + st->bytes > s->params.hbm_budget) {
+        /* Over the budget: without what it can do without, perhaps not. */
+        pthread_mutex_unlock(&s->lock);
+        if (craw_pipeline_shrink(st->pipe)) {
+            after = pool_used(s);
+            st->bytes = after > before ? after - before : 0;
+        }
+        pthread_mutex_lock(&s->lock);
+    }
     for (int i = 0; i < MAX_STREAMS && free_idx < 0; i++)
         if (!s->streams[i])
             free_idx = i;

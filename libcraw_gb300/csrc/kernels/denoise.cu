@@ -104,8 +104,6 @@ int launch_history(const CRAWKDenoise *k, const CRAWKDenoiseIO *io, float *tv, u
     auto fn = k_dn_history;
     const size_t smem = (size_t)C::smem_floats * sizeof(float);
     static std::atomic<uint64_t> attr_done{ 0 };
-    if (!tv)
-        return -22;
     if (craw_smem_attr(fn, smem, attr_done) < 0)
         return -5;
     const HistPlanes P(k->pw, k->ph);
@@ -140,6 +138,8 @@ int dispatch(const CRAWKDenoise *k, const CRAWKDenoiseIO *io, const CRAWKRound *
     if (sp && !te)  return launch<BW, M, WP, true, false, false, X2>(k, io, rd, err, s);
     if (sp && !hi)  return launch<BW, M, WP, true, true, false, X2>(k, io, rd, err, s);
     if constexpr (X2 && M == 8) {
+        if (sp && !tv)   /* no memory for the planes: the 2x4 shape's tiles, the same bits */
+            return launch<2, 4, 2, true, true, true, true>(k, io, rd, err, s);
         if (sp)     return launch_history(k, io, tv, err, s);
     } else {
         if (sp)     return launch<BW, M, WP, true, true, true, X2>(k, io, rd, err, s);
