@@ -80,7 +80,7 @@ def parse():
     ap.add_argument("--force-shape", type=int, default=-1,
                     help="denoise tile shape index instead of the autotuner's (profiling)")
     ap.add_argument("--rcd", default="auto", choices=["auto", "tiles", "strips"],
-                    help="RCD interior by 64x16 tiles or by strips instead of the library's choice "
+                    help="RCD by 64x16 tiles or by walking warps (strips) instead of the library's choice "
                          "(profiling)")
     ap.add_argument("--e2e-lanes", type=int, default=0,
                     help="pipelines the end-to-end leg rotates over (0: the default)")
@@ -375,7 +375,7 @@ def run_gpu(args):
         # A fixed denoise shape and no autotuner launches, for profiling runs.
         L.debug_force_denoise_shape(args.force_shape)
     if args.rcd != "auto":
-        # The RCD interior by tiles or by strips whatever the colour stage.
+        # The RCD by tiles, or by the walking warps that are the default.
         L.debug_rcd_strips(0 if args.rcd == "tiles" else 2)
     stream = torch.cuda.Stream()
     sptr = stream.cuda_stream
@@ -603,8 +603,8 @@ def run_gpu(args):
             "roofline": roof, "roofline_fp32": roof32,
             "e2e": e2e,
             # Our kernels per step: fused = denoise, [the rounding's compaction,
-            # decision and double-float kernels,] RCD interior (tiles or strips),
-            # RCD border tiles, awb_reduce; plain = vst + nlm, prep + 8 RCD
+            # decision and double-float kernels,] RCD interior, RCD border, the
+            # AWB publication; plain = vst + nlm, prep + 8 RCD
             # sweeps + awb + colour.
             "gpu_launches": args.steps * ((7 if exact else 4) if impl == L.IMPL_FUSED else 13),
             "clocks": {k: clk_s[k] for k in ("sm_mhz", "sm_max_mhz", "reasons")},
