@@ -3,8 +3,8 @@
  * reference, which develops one frame per recording).
  *
  * A batch develops up to max_frames independent frames of different sizes
- * in persistent launches: every denoise tile of every frame, then every
- * develop tile of every frame. The launches are captured into a CUDA
+ * in one launch a phase: every denoise tile of every frame, then every
+ * develop item of every frame. The launches are captured into a CUDA
  * graph the first time a set of frame shapes is seen and replayed for
  * every later recording with the same shapes; each replay gets the
  * recording's per-frame constants as new parameters of the captured
@@ -19,8 +19,8 @@
 
 typedef struct CRAWBatch CRAWBatch;
 
-/* The persistent part runs as two launches (every denoise tile, then every
- * develop tile) by default: measured faster than one launch with a
+/* They run as two launches (every denoise tile, then every develop item) by
+ * default: measured faster than one launch with a
  * grid-wide barrier, which carries the denoise phase's registers into the
  * develop phase and halves its occupancy. CRAW_BATCH_FLAG_FUSED asks for the
  * one launch; CRAW_BATCH_FLAG_UNFUSED names the default. */
@@ -38,10 +38,10 @@ typedef struct CRAWBatchParams {
     uint32_t flags;                  /* CRAW_PIPELINE_FLAG_DENOISE, CRAW_BATCH_FLAG_* */
     /* Frames of at least this many pixels are developed by the single-frame
      * kernels, launched one frame after another on the recording's stream
-     * after the persistent launch of the others: on frames that large the
-     * persistent kernel's per-tile cost is higher and its saved launches
-     * worth nothing. 0: CRAW_BATCH_DIRECT_PIXELS; UINT32_MAX: every frame in
-     * the persistent launch. */
+     * after the launches of the others: on frames that large a batch's
+     * per-item cost is higher and its saved launches worth nothing. 0:
+     * CRAW_BATCH_DIRECT_PIXELS; UINT32_MAX: every frame in the batch's
+     * launches. */
     uint32_t direct_pixels;
     uint8_t padding[64 - 8 * 4];
 } CRAWBatchParams;
@@ -61,8 +61,8 @@ typedef struct CRAWBatchInfo {
 CRAW_API void craw_batch_params_init(CRAWBatchParams *p);
 
 /* Allocates a denoised-mosaic buffer per frame slot, the constant table,
- * and times the denoise tile shapes on a max_width x max_height scratch
- * frame to pick the faster. */
+ * and, where frames may be developed directly, times the single-frame
+ * denoise shapes on a max_width x max_height scratch frame. */
 CRAW_API int craw_batch_create(CRAWContext *ctx, const CRAWBatchParams *params, CRAWBatch **out);
 
 /* Enqueues the development of `nb_frames` frames on `stream`: src[i]

@@ -261,7 +261,7 @@ class BatchParams(C.Structure):
 
 #: Frames of a batch with at least this many pixels go to the single-frame
 #: kernels (BatchParams.direct_pixels = 0); BATCH_ALL_PERSISTENT keeps every
-#: frame in the persistent launch.
+#: frame in the batch's launches.
 BATCH_DIRECT_PIXELS = 4000000
 BATCH_ALL_PERSISTENT = 0xFFFFFFFF
 
@@ -649,7 +649,7 @@ class Pipeline:
         n = h.bins * h.bins
         at = [C.addressof(p.contents) for p in (h.count, h.weight, h.weight_bright)]
         if at[1] - at[0] == at[2] - at[1] == 4 * n:
-            # The three lie one after another: one copy of them (a 960x540
+            # The three lie one after another: one copy of them (a 640x360
             # frame developed and its histogram read: 41 us, three 47).
             a = np.frombuffer((C.c_uint32 * (3 * n)).from_address(at[0]), np.uint32).copy()
             return AwbHistogram(*a.reshape(3, h.bins, h.bins))
@@ -858,7 +858,7 @@ def batch_params(max_width: int, max_height: int, **kw) -> BatchParams:
 
 class Batch:
     """craw_batch_create / record / free: many frames of uneven sizes in
-    one persistent launch replayed from a CUDA graph."""
+    one launch a phase, replayed from a CUDA graph."""
 
     def __init__(self, ctx: Context, params: BatchParams):
         self.ctx = ctx

@@ -1,6 +1,6 @@
 /*
- * Batched development of frames of uneven sizes: one persistent launch per
- * recording, captured once into a CUDA graph per set of frame shapes and
+ * Batched development of frames of uneven sizes: one launch a phase (or one
+ * in all) per recording, captured once into a CUDA graph per set of frame shapes and
  * replayed after a copy of the per-frame constant table. See
  * include/craw/batch.h.
  */

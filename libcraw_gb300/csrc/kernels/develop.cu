@@ -210,7 +210,7 @@ k_develop_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
  * interior's (its steps take longer). A segment of n rows takes n + 6 steps,
  * n + 5 in the border: the fewer in all. Frame times, sharing against taking
  * turns: 115 and 124 us (1920x1080, denoise with history, AP0), 280 and 284
- * (3840x2160, denoise); 737 and 706 (5760x3240, exact denoise, AP1). */
+ * (4098x2162, denoise); 737 and 706 (5760x3240, exact denoise, AP1). */
 void rcd_grids(int width, int height, WalkGrid &w, RingGrid &ring, int &inner, int &border)
 {
     const int h2 = height / 2, room = craw_sm_count() * WALK_CTAS;

@@ -1,5 +1,7 @@
 /*
- * The fused develop stage, tile bodies: prep + debayer + epilogue in one launch.
+ * The fused develop stage, tile bodies: prep + debayer + epilogue in one launch
+ * (frames develop by walking warps, develop_walk.cuh; the tiles are a bilinear
+ * or MHC batch's, and the RCD's for comparison).
  *
  * One CTA develops a TW x TH tile of the frame. It loads the tile's
  * mosaic with the debayer's apron into shared memory, prepped (normalise,
@@ -778,9 +780,9 @@ template <int METHOD, int TW, int TH, int NT> struct PixelSmem {
 };
 
 /* Interior tiles of the RCD by quads (QTW x QH pixels, all aprons inside
- * the frame); the per-pixel kernel below takes the rest. The single-frame
- * kernel uses QTH-row tiles with one thread per quad (QNT threads); the
- * batch kernel its own height and thread count. */
+ * the frame) with one thread per quad (QNT threads); the per-pixel tiles
+ * below take the rest. The RCD runs so for comparison and in tests; frames
+ * run by walking warps, which keep the two forms where they were. */
 constexpr int QTW = 64, QTH = 16, QNT = 256, BTW = 32, BTH = 16;
 
 template <int QH = QTH>
@@ -803,8 +805,8 @@ CRAW_DEV void rcd_quad_tile(const CRAWKDevelop &k, const CRAWKDevelopIO &io, int
     epilogue<QTW, QH, NQ>(k, io, x0, y0, t.rgb);
 }
 
-/* Per-pixel tiles: every bilinear and MHC tile, and the RCD tiles that the
- * quad kernel leaves (those whose QTW x QTH tile touches a border). */
+/* Per-pixel tiles: a batch's bilinear and MHC tiles, and the RCD tiles that
+ * the quad kernel leaves (those whose QTW x QTH tile touches a border). */
 /* One per-pixel tile at (x0, y0); NT threads, `smem` holds
  * PixelSmem<METHOD, TW, TH, NT>::floats floats. An RCD tile inside a
  * QTW x QH quad tile that rcd_quad_tile<QH>() takes is skipped. */
