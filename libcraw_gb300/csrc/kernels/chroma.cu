@@ -302,7 +302,7 @@ extern "C" int craw_k_chroma_up_color(const CRAWKDevelop *k, const CRAWKChroma *
     g.nqx = c->width / 2;
     g.nqy = c->height / 2;
     g.nx = (c->width + LW_P * LW_N - 1) / (LW_P * LW_N);
-    const unsigned ctas = walk_segments(g, craw_sm_count(), kUpCtas, 4);
+    const unsigned ctas = walk_segments(g, craw_sm_count(), kUpCtas, awb->hist ? 4 : 2);
     auto kernel = k_chroma_up_color<LW_ANY>;
     if (!inter_out)
         kernel = dst_fmt == CRAW_K_OUT_RGBA16F  ? k_chroma_up_color<CRAW_K_OUT_RGBA16F>

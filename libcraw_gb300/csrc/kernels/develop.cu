@@ -203,15 +203,15 @@ k_develop_walk(const CRAWKDevelop k, const CRAWKDevelopIO io, const WalkGrid g)
 }
 
 /* The RCD of a w x h frame as strips: the interior's (w, its CTAs in inner;
- * none if the frame has none) and the border's. Segments are a multiple of 4
- * quad rows, at least 8. Either the interior takes one wave of WALK_CTAS
+ * none if the frame has none) and the border's. Segments are a multiple of
+ * `unit` quad rows. Either the interior takes one wave of WALK_CTAS
  * CTAs an SM and the border, in segments as short as one wave of it allows,
  * the next; or both share a wave, the border in segments half as long as the
  * interior's (its steps take longer). A segment of n rows takes n + 6 steps,
  * n + 5 in the border: the fewer in all. Frame times, sharing against taking
  * turns: 115 and 124 us (1920x1080, denoise with history, AP0), 280 and 284
  * (4098x2162, denoise); 737 and 706 (5760x3240, exact denoise, AP1). */
-void rcd_grids(int width, int height, WalkGrid &w, RingGrid &ring, int &inner, int &border)
+void rcd_grids(int width, int height, int unit, WalkGrid &w, RingGrid &ring, int &inner, int &border)
 {
     const int h2 = height / 2, room = craw_sm_count() * WALK_CTAS;
     w = rcd_part(width, height, 0);
@@ -222,19 +222,20 @@ void rcd_grids(int width, int height, WalkGrid &w, RingGrid &ring, int &inner, i
     auto cut_ring = [&](int most) {
         ring.first[0] = 0;
         for (int i = 0; i < 4; i++)
-            ring.first[i + 1] = ring.first[i] + walk_cut(ring.g[i], most);
+            ring.first[i + 1] = ring.first[i] + walk_cut(ring.g[i], most, unit);
         return ctas(ring.first[4]);
     };
-    int turn = 8, turn_ring = 8, both = 8;
-    while (turn < h2 && ctas(walk_cut(w, turn)) > room)
-        turn += 4;
+    auto more = [&](int n) { return n < 4 ? 4 : n + 4; };
+    auto half = [&](int n) { return n / 8 * 4 > unit ? n / 8 * 4 : unit; };
+    int turn = unit, turn_ring = unit, both = unit;
+    while (turn < h2 && ctas(walk_cut(w, turn, unit)) > room)
+        turn = more(turn);
     while (turn_ring < h2 && cut_ring(turn_ring) > room)
-        turn_ring += 4;
-    auto half = [](int n) { return n / 8 * 4 > 8 ? n / 8 * 4 : 8; };
-    while (both < h2 && ctas(walk_cut(w, both)) + cut_ring(half(both)) > room)
-        both += 4;
+        turn_ring = more(turn_ring);
+    while (both < h2 && ctas(walk_cut(w, both, unit)) + cut_ring(half(both)) > room)
+        both = more(both);
     const bool share = in && both + 6 < turn + 6 + turn_ring + 5;
-    inner = ctas(walk_cut(w, share ? both : turn));
+    inner = ctas(walk_cut(w, share ? both : turn, unit));
     border = cut_ring(share ? half(both) : turn_ring);
 }
 
@@ -246,7 +247,7 @@ int launch_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, c
     g.nqx = k->width / 2;
     g.nqy = k->height / 2;
     g.nx = (k->width + LW_P * LW_N - 1) / (LW_P * LW_N);
-    const unsigned grid = walk_segments(g, craw_sm_count(), linear_ctas<METHOD, EPI>(), 4);
+    const unsigned grid = walk_segments(g, craw_sm_count(), linear_ctas<METHOD, EPI>(), walk_unit(*io, 1));
     return craw_launch_early(k_develop_walk<METHOD, EPI>, (int)grid, WALK_NT, 0, early, s, *k, *io, g);
 }
 
@@ -283,7 +284,7 @@ int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cud
     WalkGrid w;
     RingGrid ring;
     int inner, border;
-    rcd_grids(k->width, k->height, w, ring, inner, border);
+    rcd_grids(k->width, k->height, walk_unit(*io, 2), w, ring, inner, border);
     if (inner > 0) {
         if (craw_launch_early(k_develop_rcd_walk<FMT, RGC, MORE>, inner, WALK_NT, 0, early, s, *k, *io, w) < 0)
             return -5;

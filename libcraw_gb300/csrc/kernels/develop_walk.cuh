@@ -31,24 +31,31 @@ namespace craw_dev {
 
 /* The frame's part the strips cover, in quads: columns qx0 .. qx0 + nqx,
  * rows qy0 .. qy0 + nqy, in segments of `seg` rows a warp, `nx` strips
- * across. qx0, qy0, seg and a strip's output columns are multiples of 4, so
- * that strips and segments start on 8x8 AWB blocks. */
+ * across. qx0, qy0 and a strip's output columns are multiples of 4, and seg
+ * of what walk_unit() says, so that strips and segments start on 8x8 AWB
+ * blocks (4x4 blocks of the chroma path) where a frame has them. */
 struct WalkGrid {
     int qx0, nqx, qy0, nqy, seg, nx;
 };
 
 constexpr int WALK_WARPS = 4, WALK_NT = 32 * WALK_WARPS;   /* warps (strips) a CTA */
 
+/* The quad rows that a segment is a multiple of: whole AWB blocks, or whole
+ * blocks of the chroma path. */
+inline int walk_unit(const CRAWKDevelopIO &io, int least)
+{
+    return io.awb.hist ? 4 : (io.quarter ? 2 : least);
+}
+
 /* Segments of one wave of `ctas` CTAs an SM: as tall as that allows (a
  * segment reads, and for the RCD computes, its first rows' surroundings
- * again), a multiple of 4 quad rows, at least `least`; g.nx strips are
- * set. Returns the CTAs. */
-inline unsigned walk_segments(WalkGrid &g, int sms, int ctas, int least)
+ * again), a multiple of `unit` quad rows; g.nx strips are set. Returns the
+ * CTAs. */
+inline unsigned walk_segments(WalkGrid &g, int sms, int ctas, int unit)
 {
     const int room = sms * ctas * WALK_WARPS / g.nx;
     const int nseg = room > 1 ? room : 1;
-    g.seg = 4 * (((g.nqy + 3) / 4 + nseg - 1) / nseg);
-    g.seg = g.seg < least ? least : g.seg;
+    g.seg = unit * (((g.nqy + unit - 1) / unit + nseg - 1) / nseg);
     const int warps = g.nx * ((g.nqy + g.seg - 1) / g.seg);
     return (unsigned)((warps + WALK_WARPS - 1) / WALK_WARPS);
 }
@@ -410,14 +417,14 @@ __host__ CRAW_DEV WalkGrid rcd_part(int width, int height, int i)
     return g;
 }
 
-/* Cuts a part into segments of at most `most` quad rows (a multiple of 4),
- * all alike; returns its warps. */
-__host__ CRAW_DEV int walk_cut(WalkGrid &g, int most)
+/* Cuts a part into segments of at most `most` quad rows (a multiple of
+ * `unit`, as they are), all alike; returns its warps. */
+__host__ CRAW_DEV int walk_cut(WalkGrid &g, int most, int unit = 4)
 {
     if (g.nqx <= 0 || g.nqy <= 0)
         return 0;
     const int n = (g.nqy + most - 1) / most;
-    g.seg = 4 * (((g.nqy + 3) / 4 + n - 1) / n);
+    g.seg = unit * (((g.nqy + unit - 1) / unit + n - 1) / n);
     return g.nx * ((g.nqy + g.seg - 1) / g.seg);
 }
 
