@@ -623,17 +623,17 @@ k_noise_lts_float(const double *m, const double *v, const double *lv, int nb, in
 }
 
 /* The least of the double costs of the pairs that the floats leave in
- * question, the first of equals in (i, j) order. A warp looks at kLtsSpan
+ * question, the first of equals in (i, j) order. A warp looks at `span`
  * pairs, far apart (those in question come together); of one that may be the least it sorts the squared residuals
  * ascending in shared memory (bitonic; they are not negative, so their bits
  * sort as they do), and one lane adds the `keep` smallest in order. The
  * pairs that came this far gather in `found`; the last CTA to finish picks
  * from them. count: the pairs found, the CTAs done. */
-constexpr int kLtsExactWarps = 8, kLtsSpan = 8;
+constexpr int kLtsExactWarps = 8, kLtsSpan = 8, kLtsFew = 48;
 
 __global__ void __launch_bounds__(32 * kLtsExactWarps)
-k_noise_lts(const double *m, const double *v, const double *lv, int nb, int np2, int keep, const float *root,
-            const uint32_t *bound, ulonglong2 *found, uint32_t *count, int2 *best)
+k_noise_lts(const double *m, const double *v, const double *lv, int nb, int np2, int keep, int span,
+            const float *root, const uint32_t *bound, ulonglong2 *found, uint32_t *count, int2 *best)
 {
     __shared__ unsigned long long d2[kLtsExactWarps][CRAW_K_NOISE_MAX_BINS];
     __shared__ bool last;
@@ -649,7 +649,7 @@ k_noise_lts(const double *m, const double *v, const double *lv, int nb, int np2,
         lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, d));
     bool maybe = false;
     const int mine = p0 + lane * step;
-    if (lane < kLtsSpan && mine < nb * nb && mine / nb < mine % nb) {
+    if (lane < span && mine < nb * nb && mine / nb < mine % nb) {
         const float c = root[mine];
         maybe = c < INFINITY && c - lts_slack(c, lmax, sqrtf((float)keep)) <= __uint_as_float(*bound);
     }
@@ -809,14 +809,21 @@ extern "C" int craw_k_noise_lts(const double *m, const double *v, const double *
     float *root = reinterpret_cast<float *>(found + (size_t)nb * nb);
     if (cudaMemsetAsync(bound, 0x7f, 4, s) != cudaSuccess || cudaMemsetAsync(count, 0, 8, s) != cudaSuccess)
         return -5;
-    const int per = kLtsWarps * kLtsPairs, span = kLtsExactWarps * kLtsSpan;
+    const int per = kLtsWarps * kLtsPairs;
     const dim3 grid(nb, (nb + per - 1) / per);
-    if (nb <= 128)
+    /* A few bins' pairs are all evaluated in doubles at once, a warp each: a
+     * 640x360 estimate of 32 bins 299 us, 319 through the floats. */
+    const bool few = nb <= kLtsFew;
+    if (few) {
+        if (cudaMemsetAsync(root, 0, (size_t)nb * nb * sizeof(float), s) != cudaSuccess)
+            return -5;
+    } else if (nb <= 128)
         k_noise_lts_float<4><<<grid, 32 * kLtsWarps, 0, s>>>(m, v, lv, nb, keep, root, bound);
     else
         k_noise_lts_float<16><<<grid, 32 * kLtsWarps, 0, s>>>(m, v, lv, nb, keep, root, bound);
     if (cudaGetLastError() != cudaSuccess)
         return -5;
-    return craw_launch_early(k_noise_lts, (nb * nb + span - 1) / span, 32 * kLtsExactWarps, 0, true, s, m, v, lv, nb,
-                             np2, keep, root, bound, found, count, reinterpret_cast<int2 *>(best));
+    const int span = few ? 1 : kLtsSpan, cta = span * kLtsExactWarps;
+    return craw_launch_early(k_noise_lts, (nb * nb + cta - 1) / cta, 32 * kLtsExactWarps, 0, !few, s, m, v, lv, nb,
+                             np2, keep, span, root, bound, found, count, reinterpret_cast<int2 *>(best));
 }

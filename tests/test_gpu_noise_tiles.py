@@ -55,3 +55,17 @@ def test_estimate_matches_oracle(w, h, kind, nb, least):
     g, r = L.noise_estimate(m, PROF, p).as_tuple(), want.as_tuple()
     assert (g[2], g[3]) == (r[2], r[3]), (g, r)
     assert all(abs(x - y) <= 1e-6 * max(abs(y), 1e-30) for x, y in zip(g[:2] + g[4:], r[:2] + r[4:])), (g, r)
+
+
+@pytest.mark.parametrize("nb,least", [(54, 10), (55, 10), (56, 10)])
+def test_few_and_many_bins(nb, least):
+    """Numbers of used bins on either side of where the pairs' costs are
+    first bounded in floats."""
+    m = frame("ramp", 516, 260, 77)
+    p = L.NoiseEstimateParams()
+    p.nb_bins, p.min_bin_samples, p.max_level = nb, least, 0.98
+    ret, want = orc.noise_estimate(m, PROF, p)
+    assert ret == 0 and 46 <= want.as_tuple()[2] <= 50, want.as_tuple()
+    g, r = L.noise_estimate(m, PROF, p).as_tuple(), want.as_tuple()
+    assert (g[2], g[3]) == (r[2], r[3]), (g, r)
+    assert all(abs(x - y) <= 1e-6 * max(abs(y), 1e-30) for x, y in zip(g[:2] + g[4:], r[:2] + r[4:])), (g, r)
