@@ -270,7 +270,7 @@ namespace {
 /* An RCD batch's segments: the interiors' as short as one wave of SEG_CTAS
  * CTAs an SM allows; the borders', which follow as CTAs end, as long as the
  * steps that one of the wave's warps gets of them (a segment of n rows takes
- * n + 5). Multiples of 4 rows, at least 8. */
+ * n + 5). Multiples of 4 rows. */
 int layout_segments(CRAWKBatchFrame *f, int nb)
 {
     const int sms = device_sms(), room = (sms > 0 ? sms : 152) * SEG_CTAS * WALK_WARPS;
@@ -285,14 +285,14 @@ int layout_segments(CRAWKBatchFrame *f, int nb)
         }
         tall = f[i].dv.height / 2 > tall ? f[i].dv.height / 2 : tall;
     }
-    auto at_least = [](long n) { return n > 8 ? (int)((n + 3) / 4 * 4) : 8; };
+    auto at_least = [](long n) { return n > 4 ? (int)((n + 3) / 4 * 4) : 4; };
     auto interiors = [&](int most) {
         int n = 0;
         for (int i = 0; i < nb; i++)
             n += walk_cut(g[i][0], most);
         return n;
     };
-    int cut = at_least(rows[0] / room), border = 8;
+    int cut = at_least(rows[0] / room), border = 4;
     while (cut < tall && interiors(cut) > room)
         cut += 4;
     for (; border < cut; border += 4) {
