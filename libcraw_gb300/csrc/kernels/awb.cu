@@ -23,8 +23,8 @@ constexpr int kThreads = 256;
 /* One piece a thread; thread i also takes deferred block i. `head`: the
  * count, and a ticket that tells the last CTA to zero it. */
 __global__ void __launch_bounds__(kThreads)
-k_awb_publish(uint4 *__restrict__ hist, uint32_t *head, const uint4 *__restrict__ deferred, uint4 *host_hist,
-              uint32_t *host_head, uint4 *host_deferred)
+k_awb_publish(uint4 *hist, uint32_t *head, const uint4 *deferred, uint4 *host_hist, uint32_t *host_head,
+              uint4 *host_deferred)
 {
     craw_await_previous();
     const int i = blockIdx.x * kThreads + threadIdx.x;

@@ -222,8 +222,8 @@ CRAW_DEV void history_tile(const CRAWKDenoise &k, const CRAWKDenoiseIO &io, cons
         for (int i = tid; i < 8 * TN / 4; i += NT) {
             const int a = i / TN, e = 4 * (i % TN);        /* T or V; the element of its four planes */
             const int pl = e / TN, y = e % TN / TS, x = e % TS;
-            reinterpret_cast<float4 *>(T)[i] = __ldg(reinterpret_cast<const float4 *>(
-                tv + (size_t)(4 * a + pl) * P.n + (size_t)(ty0 + y) * P.w + tx0 + x));
+            reinterpret_cast<float4 *>(T)[i] = *reinterpret_cast<const float4 *>(
+                tv + (size_t)(4 * a + pl) * P.n + (size_t)(ty0 + y) * P.w + tx0 + x);
         }
         __syncthreads();
     }

@@ -70,11 +70,12 @@ CRAW_DEV float walk_right(float v)
 }
 
 /* A row's sample pair, a step before it is used: volatile, so that the load
- * stays where it is written. */
+ * stays where it is written; not by the read-only path, since the kernel
+ * that writes the row may still run when this one starts. */
 CRAW_DEV uint32_t walk_ld(const char *p)
 {
     uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 
@@ -861,7 +862,7 @@ constexpr int LW_N = 30, LW_P = 4;
 CRAW_DEV uint2 walk_ld4(const char *p)
 {
     uint2 v;
-    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
     return v;
 }
 

@@ -160,8 +160,8 @@ CRAW_DEV uint4 plane_quad(const char *row, int c, int w2)
 
 CRAW_DEV float4 plane_values(const float *lut, uint4 v, int sh)
 {
-    return make_float4(__ldg(lut + ((v.x >> sh) & 0xffffu)), __ldg(lut + ((v.y >> sh) & 0xffffu)),
-                       __ldg(lut + ((v.z >> sh) & 0xffffu)), __ldg(lut + ((v.w >> sh) & 0xffffu)));
+    return make_float4(lut[(v.x >> sh) & 0xffffu], lut[(v.y >> sh) & 0xffffu], lut[(v.z >> sh) & 0xffffu],
+                       lut[(v.w >> sh) & 0xffffu]);
 }
 
 /* [1 -2 1; -2 4 -2; 1 -2 1] / 6 at column c of three rows, in the
@@ -439,7 +439,7 @@ k_noise_refine(const CRAWKNoise k, const NoiseGrid g, const uint16_t *src, size_
             Q q;
             q.x = q.y = q.z = q.w = (B)nb;
             if (mine)
-                q = __ldg(reinterpret_cast<const Q *>(bidx + ((size_t)(2 * py + pl) * g.hh + ko) * g.wp + io));
+                q = *reinterpret_cast<const Q *>(bidx + ((size_t)(2 * py + pl) * g.hh + ko) * g.wp + io);
             b[pl][0] = q.x;
             b[pl][1] = q.y;
             b[pl][2] = q.z;
