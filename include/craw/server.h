@@ -110,7 +110,8 @@ CRAW_API int craw_server_create(CRAWContext *ctx, const CRAWServerParams *params
 CRAW_API void craw_server_free(CRAWServer **s);
 
 /* Admits a stream: creates its pipeline, CUDA stream and staging slots and
- * charges their device memory to the budget. CRAW_ERROR(EAGAIN) when the
+ * charges their device memory to the budget; what pipelines hold for speed
+ * alone is given back before a stream is refused. CRAW_ERROR(EAGAIN) when the
  * stream does not fit beside the open ones, CRAW_ERROR(ENOSPC) when it
  * would not fit alone; pipeline creation errors as craw_pipeline_create(). */
 CRAW_API int craw_server_stream_open(CRAWServer *s, const CRAWServerStreamParams *params,

@@ -40,6 +40,9 @@ void craw_dev_free(CRAWContext *ctx, void *ptr);
  * speed and the same results; whether there was anything. */
 bool craw_pipeline_shrink(CRAWPipeline *p);
 
+/* The bytes that craw_pipeline_shrink() would give back. */
+size_t craw_pipeline_spare(const CRAWPipeline *p);
+
 int craw_dev_sync(CRAWContext *ctx);
 
 /* craw_debug_force_denoise_shape(): -1, or the shape every new pipeline uses. */

@@ -281,6 +281,11 @@ static void alloc_planes(CRAWPipeline *p, float **planes)
         *planes = NULL;
 }
 
+size_t craw_pipeline_spare(const CRAWPipeline *p)
+{
+    return p->dn_planes ? craw_k_denoise_planes((int32_t)(p->params.width / 2), (int32_t)(p->params.height / 2)) : 0;
+}
+
 bool craw_pipeline_shrink(CRAWPipeline *p)
 {
     if (!p->dn_planes)

@@ -520,6 +520,35 @@ CRAW_API void craw_server_free(CRAWServer **ps)
     *ps = NULL;
 }
 
+/* Gives back at least `excess` bytes of what the open streams can do without
+ * (both locks held), or nothing if they do not have as much: a stream that
+ * fits without is not refused for what others hold beyond their needs. The
+ * frames of a stream that has some in flight are waited for. */
+static void reclaim_spare(CRAWServer *s, uint64_t excess)
+{
+    const uint64_t rounding = 2 << 20;   /* of the pool's, a buffer */
+    uint64_t spare = 0;
+
+    for (int i = 0; i < MAX_STREAMS; i++)
+        if (s->streams[i] && craw_pipeline_spare(s->streams[i]->pipe))
+            spare += craw_pipeline_spare(s->streams[i]->pipe) + rounding;
+    if (spare < excess)
+        return;
+    for (int i = 0; i < MAX_STREAMS && excess; i++) {
+        struct stream *st = s->streams[i];
+        uint64_t before, after, freed;
+        if (!st || !craw_pipeline_spare(st->pipe) || cudaStreamSynchronize(st->cs) != cudaSuccess)
+            continue;
+        before = pool_used(s);
+        craw_pipeline_shrink(st->pipe);
+        after = pool_used(s);
+        freed = CRAW_MIN(before > after ? before - after : 0, st->bytes);
+        st->bytes -= freed;
+        s->resident -= freed;
+        excess -= CRAW_MIN(freed, excess);
+    }
+}
+
 CRAW_API int craw_server_stream_open(CRAWServer *s, const CRAWServerStreamParams *params,
                                      uint32_t *stream_id)
 {
@@ -595,6 +624,8 @@ CRAW_API int craw_server_stream_open(CRAWServer *s, const CRAWServerStreamParams
     for (int i = 0; i < MAX_STREAMS && free_idx < 0; i++)
         if (!s->streams[i])
             free_idx = i;
+    if (free_idx >= 0 && st->bytes <= s->params.hbm_budget && s->resident + st->bytes > s->params.hbm_budget)
+        reclaim_spare(s, s->resident + st->bytes - s->params.hbm_budget);
     if (free_idx < 0 || s->resident + st->bytes > s->params.hbm_budget) {
         ret = free_idx < 0 ? CRAW_ERROR(EMFILE) :
               st->bytes > s->params.hbm_budget ? CRAW_ERROR(ENOSPC) : CRAW_ERROR(EAGAIN);
