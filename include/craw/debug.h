@@ -11,6 +11,11 @@
  * craw_pipeline_create() leaves nothing behind; 0 disarms it. */
 CRAW_API void craw_debug_fail_alloc(int k);
 
+/* Makes every device allocation that would take its context's memory in use
+ * above `bytes` fail with CRAW_ERROR(ENOMEM), so that tests can stand in for
+ * a full device; 0: none. */
+CRAW_API void craw_debug_limit_alloc(uint64_t bytes);
+
 /* Makes every pipeline created from now use denoise tile shape `shape`
  * (the index craw_pipeline_get_kernel_config() reports) instead of the
  * autotuner's pick, so that tests can check each shape; -1 restores the

@@ -284,7 +284,7 @@ for _s, _n in ((Profile, 1264), (FrameParams, 264), (PipelineParams, 256), (Cuda
 #: Every symbol the C ABI exports (include/craw/*.h).
 EXPORTS = (
     "craw_version_int", "craw_log", "craw_context_create", "craw_context_free",
-    "craw_cuda_check_device", "craw_debug_fail_alloc", "craw_debug_force_denoise_shape",
+    "craw_cuda_check_device", "craw_debug_fail_alloc", "craw_debug_limit_alloc", "craw_debug_force_denoise_shape",
     "craw_debug_rcd_tma", "craw_debug_rcd_strips", "craw_debug_denoise_tma", "craw_debug_kernel_errors", "craw_debug_denoise_round",
     "craw_debug_denoise_round_decide", "craw_debug_denoise_round_stats",
     "craw_pipeline_params_init", "craw_frame_params_init", "craw_pipeline_create",
@@ -367,6 +367,7 @@ def lib() -> C.CDLL:
         "craw_context_free": (None, [C.POINTER(vp)]),
         "craw_cuda_check_device": (i32, [i32, C.POINTER(C.c_char_p)]),
         "craw_debug_fail_alloc": (None, [i32]),
+        "craw_debug_limit_alloc": (None, [C.c_uint64]),
         "craw_debug_force_denoise_shape": (i32, [i32]),
         "craw_debug_rcd_tma": (i32, [i32]),
         "craw_debug_rcd_strips": (i32, [i32]),
@@ -901,6 +902,12 @@ class Batch:
 
 def debug_fail_alloc(k: int) -> None:
     lib().craw_debug_fail_alloc(k)
+
+
+def debug_limit_alloc(nbytes: int) -> None:
+    """Device allocations that would take a context's memory in use above
+    `nbytes` fail (0: none does)."""
+    lib().craw_debug_limit_alloc(nbytes)
 
 
 #: Denoise tile shapes by craw_pipeline_get_kernel_config() index.

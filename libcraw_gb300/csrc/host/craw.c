@@ -155,6 +155,10 @@ CRAW_API void craw_context_free(CRAWContext **pctx)
  * rest of the library. */
 static int craw_fail_countdown;
 
+/* Another: an allocation that would take its context's pool above this many
+ * bytes in use fails; 0: none does. */
+static uint64_t craw_alloc_limit;
+
 int craw_forced_denoise_shape = -1;
 
 CRAW_API int craw_debug_force_denoise_shape(int shape)
@@ -191,6 +195,11 @@ CRAW_API void craw_debug_fail_alloc(int k)
     craw_fail_countdown = k;
 }
 
+CRAW_API void craw_debug_limit_alloc(uint64_t bytes)
+{
+    craw_alloc_limit = bytes;
+}
+
 CRAW_API int craw_debug_rcd_tma(int on)
 {
     const int was = craw_k_rcd_tma;
@@ -218,6 +227,12 @@ int craw_dev_alloc(CRAWContext *ctx, void **ptr, size_t bytes)
     *ptr = NULL;
     if (craw_fail_countdown > 0 && --craw_fail_countdown == 0)
         return CRAW_ERROR(ENOMEM);
+    if (craw_alloc_limit) {
+        uint64_t used = 0;
+        if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+            used + bytes > craw_alloc_limit)
+            return CRAW_ERROR(ENOMEM);
+    }
     return craw_cuda_err(cudaMallocFromPoolAsync(ptr, bytes, ctx->pool, ctx->stream));
 }
 

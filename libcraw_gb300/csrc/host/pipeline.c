@@ -267,6 +267,12 @@ static int time_denoise(CRAWPipeline *p, const CRAWKDenoise *k, const CRAWKDenoi
     return ret < 0 ? CRAW_ERROR(EIO) : 0;
 }
 
+/* Whether the pipeline's frames use the history's planes. */
+static bool wants_planes(const CRAWPipeline *p)
+{
+    return p->has_denoise && p->has_temporal && !p->plain && p->dn_shape[1] == CRAW_K_DN_SHAPE_2x8_X2;
+}
+
 /* The history's planes, if there is memory for them: without, the 2x8 shape
  * runs the 2x4 shape's kernel (the same bits). */
 static void alloc_planes(CRAWPipeline *p, float **planes)
@@ -329,7 +335,8 @@ static int autotune(CRAWPipeline *p)
         (ret = alloc_pitched(p, (void **)&lvl, &lp, (size_t)w * 4, h)) < 0 ||
         (ret = alloc_pitched(p, (void **)&var, &vp, (size_t)w, h)) < 0)
         goto done;
-    if (need[1] && !p->dn_planes)
+    /* After what the timing cannot do without. */
+    if (need[1])
         alloc_planes(p, &planes);
     /* A mid-grey mosaic, a state of level 0.25 and unit variance. */
     cudaMemset2DAsync(mosaic, mp, 0x08, (size_t)w * 2, h, ctx->stream);
@@ -358,7 +365,7 @@ static int autotune(CRAWPipeline *p)
             continue;
         for (int shape = 0; shape < CRAW_K_DN_SHAPE_NB; shape++) {
             float ms;
-            if ((ret = time_denoise(p, &k, &io, shape, p->dn_planes ? p->dn_planes : planes, &ms)) < 0)
+            if ((ret = time_denoise(p, &k, &io, shape, planes, &ms)) < 0)
                 goto done;
             if (ms < best) {
                 best = ms;
@@ -386,6 +393,10 @@ static int autotune(CRAWPipeline *p)
         p->tune_held = true;
     }
     pthread_mutex_unlock(&tune_lock);
+    if (wants_planes(p)) {
+        p->dn_planes = planes;
+        planes = NULL;
+    }
 done:
     craw_dev_free(ctx, mosaic);
     craw_dev_free(ctx, planes);
@@ -639,16 +650,16 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
         ret = CRAW_ERROR(EIO);
         goto fail;
     }
-    if (p->has_denoise && p->has_temporal && !p->plain)
-        alloc_planes(p, &p->dn_planes);
     if (craw_forced_denoise_shape >= 0) {
         p->dn_shape[0] = p->dn_shape[1] = craw_forced_denoise_shape;
     } else if ((p->has_denoise || p->has_temporal) && !p->plain &&
                !(params->flags & CRAW_PIPELINE_FLAG_NO_AUTOTUNE) && (ret = autotune(p)) < 0) {
         goto fail;
     }
-    if (p->dn_shape[1] != CRAW_K_DN_SHAPE_2x8_X2)
-        craw_pipeline_shrink(p);
+    /* The planes last: nothing that the pipeline needs goes without memory
+     * for them. */
+    if (wants_planes(p) && !p->dn_planes)
+        alloc_planes(p, &p->dn_planes);
     craw_log(ctx, CRAW_LOG_VERBOSE, "pipeline %ux%u debayer %d flags 0x%x storage %s impl %s\n",
              w, h, params->debayer, params->flags, p->fp16 ? "fp16" : "fp32",
              p->plain ? "plain" : "fused");
