@@ -376,7 +376,9 @@ static int autotune(CRAWPipeline *p)
                  hist ? "temporal" : "spatial", p->dn_shape[hist], (double)best);
     }
     /* Another thread may have tuned the same size meanwhile: its shapes
-     * win, so that every pipeline of the size agrees. */
+     * win, so that every pipeline of the size agrees. A history timed
+     * without its planes, which one shape is the faster for, is not
+     * remembered: the next pipeline times it again. */
     pthread_mutex_lock(&tune_lock);
     if (ret == 0 && (e = tune_entry(w, h, true))) {
         for (int hist = 0; hist < 2; hist++) {
@@ -384,7 +386,7 @@ static int autotune(CRAWPipeline *p)
                 continue;
             if (e->known[hist]) {
                 p->dn_shape[hist] = e->shape[hist];
-            } else {
+            } else if (!hist || planes) {
                 e->shape[hist] = p->dn_shape[hist];
                 e->known[hist] = true;
             }

@@ -1,6 +1,8 @@
 """GPU: creating a pipeline with a temporal history on a device that is nearly
 full (craw_debug_limit_alloc): its averaged planes are optional, so they never
 take the memory of what it needs."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -91,3 +93,31 @@ def test_same_frames_with_and_without(ctx):
         L.debug_force_denoise_shape(-1)
     for a, b in zip(want, got):
         assert np.array_equal(a, b)
+
+
+class ContextWithLog(L.Context):
+    """A context that keeps the formats of what is logged."""
+
+    def __init__(self):
+        self.said = []
+        self._cb = C.CFUNCTYPE(None, C.c_void_p, C.c_int, C.c_char_p, C.c_void_p)(
+            lambda opaque, level, fmt, args: self.said.append(fmt.decode()))
+        opts = L.ContextOptions()
+        opts.log_cb = C.cast(self._cb, C.c_void_p).value
+        opts.log_level = 8             # verbose
+        self._h, self._children, self.device = C.c_void_p(), [], 0
+        assert L.lib().craw_context_create(C.byref(self._h), C.byref(L.CudaInitParams(0, None)), C.byref(opts)) == 0
+
+
+def test_shape_timed_without_planes_is_not_remembered():
+    """The history's shape timed where its planes did not fit is timed again
+    by the next pipeline of the size, and that one's is remembered."""
+    h = H2 + 18
+    with ContextWithLog() as ctx:
+        least = need(ctx, h) + 7 * W2 * h + 3 * 256 * h + SLACK
+        timed = []
+        for limit in (least, 0, 0):
+            ctx.said.clear()
+            created(ctx, limit, h).close()
+            timed.append(sum(m.startswith("autotune") for m in ctx.said))
+    assert timed == [2, 1, 0]          # with and without a history; with; neither
