@@ -273,18 +273,26 @@ static bool wants_planes(const CRAWPipeline *p)
     return p->has_denoise && p->has_temporal && !p->plain && p->dn_shape[1] == CRAW_K_DN_SHAPE_2x8_X2;
 }
 
-/* The history's planes, if there is memory for them: without, the 2x8 shape
- * runs the 2x4 shape's kernel (the same bits). */
-static void alloc_planes(CRAWPipeline *p, float **planes)
+/* The history's planes, if there is memory for them: without (*planes NULL),
+ * the 2x8 shape runs the 2x4 shape's kernel (the same bits). Negative: an
+ * error other than that. */
+static int alloc_planes(CRAWPipeline *p, float **planes)
 {
-    if (craw_dev_alloc(p->ctx, (void **)planes, craw_k_denoise_planes((int32_t)(p->params.width / 2),
-                                                                  (int32_t)(p->params.height / 2))) < 0) {
-        (void)cudaGetLastError();
+    int ret = craw_dev_alloc(p->ctx, (void **)planes, craw_k_denoise_planes((int32_t)(p->params.width / 2),
+                                                                      (int32_t)(p->params.height / 2)));
+    if (ret < 0) {
         *planes = NULL;
-        return;
+        if (ret != CRAW_ERROR(ENOMEM))
+            return ret;
+        if (cudaPeekAtLastError() == cudaErrorMemoryAllocation)
+            (void)cudaGetLastError();
+        return 0;
     }
-    if (craw_dev_sync(p->ctx) < 0)
+    if ((ret = craw_dev_sync(p->ctx)) < 0) {
+        craw_dev_free(p->ctx, *planes);
         *planes = NULL;
+    }
+    return ret;
 }
 
 size_t craw_pipeline_spare(const CRAWPipeline *p)
@@ -336,8 +344,8 @@ static int autotune(CRAWPipeline *p)
         (ret = alloc_pitched(p, (void **)&var, &vp, (size_t)w, h)) < 0)
         goto done;
     /* After what the timing cannot do without. */
-    if (need[1])
-        alloc_planes(p, &planes);
+    if (need[1] && (ret = alloc_planes(p, &planes)) < 0)
+        goto done;
     /* A mid-grey mosaic, a state of level 0.25 and unit variance. */
     cudaMemset2DAsync(mosaic, mp, 0x08, (size_t)w * 2, h, ctx->stream);
     cudaMemset2DAsync(lvl, lp, 0, (size_t)w * 4, h, ctx->stream);
@@ -660,8 +668,8 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
     }
     /* The planes last: nothing that the pipeline needs goes without memory
      * for them. */
-    if (wants_planes(p) && !p->dn_planes)
-        alloc_planes(p, &p->dn_planes);
+    if (wants_planes(p) && !p->dn_planes && (ret = alloc_planes(p, &p->dn_planes)) < 0)
+        goto fail;
     craw_log(ctx, CRAW_LOG_VERBOSE, "pipeline %ux%u debayer %d flags 0x%x storage %s impl %s\n",
              w, h, params->debayer, params->flags, p->fp16 ? "fp16" : "fp32",
              p->plain ? "plain" : "fused");
