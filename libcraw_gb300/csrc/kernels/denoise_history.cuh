@@ -152,7 +152,9 @@ CRAW_DEV void temporal_walk(const CRAWKDenoise &k, const CRAWKDenoiseIO &io, flo
                 uint8_t *vr = io.var_next + (size_t)(2 * qy + py) * io.var_pitch;
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
-                    if (qx + j < 0 || qx + j >= k.pw)
+                    if (qx + j < 0 || qx + j >= k.pw ||
+                        !craw_in_bounds((size_t)(qx + j + 1) * 8 <= io.lvl_pitch &&
+                                        (size_t)(qx + j + 1) * 2 <= io.var_pitch, err))
                         continue;
                     reinterpret_cast<float2 *>(lr)[qx + j] = make_float2(gat_inv(k, t[2 * j]), gat_inv(k, t[2 * j + 1]));
                     uint32_t code = 0;
@@ -222,8 +224,9 @@ CRAW_DEV void history_tile(const CRAWKDenoise &k, const CRAWKDenoiseIO &io, cons
         for (int i = tid; i < 8 * TN / 4; i += NT) {
             const int a = i / TN, e = 4 * (i % TN);        /* T or V; the element of its four planes */
             const int pl = e / TN, y = e % TN / TS, x = e % TS;
-            reinterpret_cast<float4 *>(T)[i] = *reinterpret_cast<const float4 *>(
-                tv + (size_t)(4 * a + pl) * P.n + (size_t)(ty0 + y) * P.w + tx0 + x);
+            if (craw_in_bounds(a < 2 && pl < 4 && ty0 + y < P.h && tx0 + x + 3 < P.w, err))
+                reinterpret_cast<float4 *>(T)[i] = *reinterpret_cast<const float4 *>(
+                    tv + (size_t)(4 * a + pl) * P.n + (size_t)(ty0 + y) * P.w + tx0 + x);
         }
         __syncthreads();
     }

@@ -79,6 +79,12 @@ CRAW_DEV uint32_t walk_ld(const char *p)
     return v;
 }
 
+/* Bytes of a pixel of an RGB image of layout f. */
+CRAW_DEV int walk_bytes(int f)
+{
+    return f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16);
+}
+
 /* Eight floats to a 32-byte aligned address in one store. */
 CRAW_DEV void walk_store8(float *p, float a, float b, float c, float d, float e, float f, float g, float h)
 {
@@ -178,12 +184,11 @@ struct WalkOut {
         : k(k_), io(io_), s(s_), lane(threadIdx.x & 31), nout(nout_), qx(qx_), qy(qy_), held(0)
     {
         mine = lane >= A && lane < A + nout;
-        dst = (char *)io.dst + (size_t)(2 * qy) * io.dst_pitch + (size_t)(2 * qx) * bytes(fmt());
+        dst = (char *)io.dst + (size_t)(2 * qy) * io.dst_pitch + (size_t)(2 * qx) * walk_bytes(fmt());
         inter = (char *)io.inter + (size_t)(2 * qy) * io.inter_pitch +
                 (size_t)(2 * qx) * (k.fp16 ? 8 : 16);
         qs[0] = qs[1] = qs[2] = 0.0f;
     }
-    CRAW_DEV static int bytes(int f) { return f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16); }
     CRAW_DEV int fmt() const { return MORE ? io.dst_fmt : FMT; }
 
     CRAW_DEV void colour(const float v[2][2][3], float o[2][2][3]) const
@@ -944,10 +949,12 @@ struct LinearWalk {
             v[r][RAD + i] = p[i];
     }
 
-    /* The lane's pixels of a row of an RGB image of layout f at `d`. */
-    CRAW_DEV void store(char *d, int f, const float o[LW_P][3]) const
+    /* The lane's pixels of row y of the RGB image at `base` (layout f), which
+     * are at `d`. */
+    CRAW_DEV void store(char *d, const void *base, size_t pitch, int y, int f, const float o[LW_P][3]) const
     {
-        if (!mine)
+        if (!mine || !craw_in_bounds(y >= 0 && y < k.height && x0 >= 0 && x0 + nv <= k.width &&
+                                     d == (const char *)base + (size_t)y * pitch + (size_t)x0 * walk_bytes(f), io.err))
             return;
         if (nv == LW_P) {
             float *p = reinterpret_cast<float *>(d);
@@ -1079,7 +1086,7 @@ struct LinearWalk {
                     o[i][c] = craw_round_half(o[i][c]);
         }
         if (CHROMA || (ANY && io.inter)) {
-            store(inter, k.fp16 ? CRAW_K_OUT_RGBA16F : CRAW_K_OUT_RGBA32F, o);
+            store(inter, io.inter, io.inter_pitch, y, k.fp16 ? CRAW_K_OUT_RGBA16F : CRAW_K_OUT_RGBA32F, o);
             inter += io.inter_pitch;
         }
         if constexpr (CHROMA) {
@@ -1090,7 +1097,7 @@ struct LinearWalk {
             awb_row(y, end, odd, o);
         if (!ANY || io.dst) {
             walk_colour<-1>(k.color, mine, o);
-            store(dst, ANY ? io.dst_fmt : EPI, o);
+            store(dst, io.dst, io.dst_pitch, y, ANY ? io.dst_fmt : EPI, o);
             dst += io.dst_pitch;
         }
     }
@@ -1117,8 +1124,7 @@ struct LinearWalk {
         for (int c = 0; c < 3; c++)
             as[c] = hs[c] = qs[c] = 0.0f;
         const int f = ANY ? io.dst_fmt : EPI;
-        dst = (char *)io.dst + (size_t)y0 * io.dst_pitch +
-              (ptrdiff_t)x0 * (f == CRAW_K_OUT_RGB32F ? 12 : (f == CRAW_K_OUT_RGBA16F ? 8 : 16));
+        dst = (char *)io.dst + (size_t)y0 * io.dst_pitch + (ptrdiff_t)x0 * walk_bytes(f);
         inter = (char *)io.inter + (size_t)y0 * io.inter_pitch + (ptrdiff_t)x0 * (k.fp16 ? 8 : 16);
         return true;
     }

@@ -96,7 +96,8 @@ k_hl_level0(const CRAWKHighlight k, const CRAWKHighlightIO io, const HlGrid g)
     /* Quad row y of the lane's quads: top rows' samples, then bottom rows'. */
     auto fetch = [&](int y) {
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (in0 && y >= 0 && y < qh) {
+        if (in0 && y >= 0 && y < qh &&
+            craw_in_bounds(qx >= 0 && 2 * qx + (in1 ? 3 : 1) < k.width && 2 * y + 1 < k.height, io.err)) {
             const char *row = (const char *)io.src + (size_t)(2 * y) * io.src_pitch + (size_t)qx * 4;
             if (in1) {
                 const uint2 a = __ldg(reinterpret_cast<const uint2 *>(row));
@@ -174,7 +175,7 @@ k_hl_level0(const CRAWKHighlight k, const CRAWKHighlightIO io, const HlGrid g)
                 }
             }
             if ((r & 1) || r == qh - 1) {
-                if (mine)
+                if (mine && craw_in_bounds(tx >= 0 && tx < k.lw[0] && (r >> 1) < k.lh[0], io.err))
                     reinterpret_cast<float4 *>(io.levels)[k.off[0] + (size_t)(r >> 1) * k.lw[0] + tx] =
                         make_float4(acc[0], acc[1], acc[2], 0.0f);
                 acc[0] = acc[1] = acc[2] = 0.0f;
