@@ -34,11 +34,12 @@ constexpr int kDilate = 3;
 
 /* smoothstep(kULo, kUHi, v). The quotient by Markstein's correction of the
  * product with the correctly rounded reciprocal, which rounds as the division
- * does; below kULo it is not positive and clamps to 0. */
+ * does; below kULo it is not positive and clamps to 0. A product above 1 need
+ * not be near (and one that overflows must not go on as infinity). */
 CRAW_DEV float smooth(float v)
 {
     constexpr float c = kUHi - kULo, rc = 1.0f / c;
-    const float x = v - kULo, q = x * rc;
+    const float x = v - kULo, q = fminf(x * rc, 4.0f);
     const float t = __saturatef(__fmaf_rn(__fmaf_rn(-c, q, x), rc, q));
     return t * t * (3.0f - 2.0f * t);
 }
