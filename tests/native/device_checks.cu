@@ -48,6 +48,48 @@ struct GamutQuotient {
     __device__ bool operator()(float x) const { return differ(craw_gamut_quotient(x, scl, iscl), __fdiv_rn(x, scl)); }
 };
 
+/* The compression by divisions and the fast power. */
+__device__ void gamut_compress(const CRAWKColor &c, float o[3])
+{
+    const float ach = fmaxf(o[0], fmaxf(o[1], o[2]));
+    if (ach == 0.0f)
+        return;
+    const float mag = fabsf(ach), inv_mag = 1.0f / mag;
+    for (int i = 0; i < 3; i++) {
+        float d = (ach - o[i]) * inv_mag;
+        if (d < c.gc_thr[i])
+            continue;
+        const float nd = __fdiv_rn(d - c.gc_thr[i], c.gc_scl[i]), p = __powf(nd, c.gc_pwr);
+        d = c.gc_thr[i] + c.gc_scl[i] * nd * __powf(1.0f + p, -c.gc_inv_pwr);
+        o[i] = ach - d * mag;
+    }
+}
+
+/* A pixel of each x: its colours x times small and large ratios, and one of
+ * zeros, infinities, NaN and x. */
+struct Gamut {
+    CRAWKColor c;
+    __device__ bool operator()(float x) const
+    {
+        const float ratio[8] = { 1.0f, 0.9f, 0.19f, 0.05f, 0.0f, -0.2f, -3.0f, -1e4f };
+        const float odd[5] = { 0.0f, -0.0f, INFINITY, -INFINITY, NAN };
+        uint32_t h = __float_as_uint(x) * 2654435761u;
+        float a[3], b[3];
+        for (int i = 0; i < 3; i++, h = h * 747796405u + 2891336453u) {
+            a[i] = x * ratio[(h >> 16) & 7] * (1.0f + (float)(h >> 8 & 0xff) / 4096.0f);
+            if (!(h >> 20 & 15))
+                a[i] = odd[(h >> 24) % 5];
+            b[i] = a[i];
+        }
+        craw_gamut_compress(c, a);
+        gamut_compress(c, b);
+        for (int i = 0; i < 3; i++)
+            if (differ(a[i], b[i]) && !(isnan(a[i]) && isnan(b[i])))
+                return true;
+        return false;
+    }
+};
+
 struct ClipRamp {
     __device__ bool operator()(float v) const
     {
@@ -89,11 +131,25 @@ long long over(uint32_t first, uint32_t last, F f)
 
 #define CHECK extern "C" __attribute__((visibility("default"))) long long
 
-/* Every positive float and +infinity. */
-CHECK check_reciprocal() { return over(1u, 0x7f800000u, Reciprocal{}); }
+/* The floats whose bits are first .. last. */
+CHECK check_reciprocal(uint32_t first, uint32_t last) { return over(first, last, Reciprocal{}); }
 
 /* Every float from 2^-30 to 2^100. */
 CHECK check_gamut_quotient(float scl) { return over(97u << 23, 227u << 23, GamutQuotient{ scl, 1.0f / scl }); }
+
+/* The same, as pixels, with the channels' thresholds and scales. */
+CHECK check_gamut_compress(uint32_t first, uint32_t last, const float thr[3], const float scl[3], float pwr)
+{
+    Gamut g = {};
+    for (int i = 0; i < 3; i++) {
+        g.c.gc_thr[i] = thr[i];
+        g.c.gc_scl[i] = scl[i];
+        g.c.gc_iscl[i] = 1.0f / scl[i];
+    }
+    g.c.gc_pwr = pwr;
+    g.c.gc_inv_pwr = (float)(1.0 / 1.2);
+    return over(first, last, g);
+}
 
 /* Every float but NaN, of either sign. */
 CHECK check_clip_ramp()

@@ -21,16 +21,37 @@ def lib(tmp_path_factory):
     subprocess.run([NVCC, *NVCC_FLAGS, "-fmad=false", "-shared", "-cudart", "static", str(SRC), "-o", str(so)],
                    check=True)
     lib = C.CDLL(str(so))
-    for f in ("check_gamut_quotient", "check_clip_ramp", "check_noise_lut"):
+    for f in ("check_reciprocal", "check_gamut_quotient", "check_gamut_compress", "check_clip_ramp", "check_noise_lut"):
         getattr(lib, f).restype = C.c_longlong
     return lib
 
 
-# The three channels' scales of the reference gamut compression (lib/gamut.c:11-25).
-@pytest.mark.parametrize("lim,thr", [(1.147, 0.815), (1.264, 0.803), (1.312, 0.880)])
-def test_gamut_quotient(lib, lim, thr):
-    r = ((1.0 - thr) / (lim - thr)) ** -1.2 - 1.0
-    assert lib.check_gamut_quotient(C.c_float((lim - thr) / r ** (1.0 / 1.2))) == 0
+def bits(x):
+    return int(np.array(x, np.float32).view(np.uint32))
+
+
+# The three channels of the reference gamut compression (lib/gamut.c:11-25).
+THR, LIM, PWR = np.array([0.815, 0.803, 0.880]), np.array([1.147, 1.264, 1.312]), 1.2
+SCL = (LIM - THR) / (((1.0 - THR) / (LIM - THR)) ** -PWR - 1.0) ** (1.0 / PWR)
+
+
+def test_reciprocal(lib):
+    """Every float above 2^-128 and below 1.34e38."""
+    assert lib.check_reciprocal(C.c_uint32(bits(2.0 ** -128) + 1), C.c_uint32(bits(1.34e38))) == 0
+
+
+@pytest.mark.parametrize("scl", SCL)
+def test_gamut_quotient(lib, scl):
+    assert lib.check_gamut_quotient(C.c_float(scl)) == 0
+
+
+def test_gamut_compress(lib):
+    """Pixels of every positive float up to 1e37 (those whose reciprocals are
+    infinite among them), with zeros, infinities and NaN beside it."""
+    thr, scl = THR.astype(np.float32), SCL.astype(np.float32)
+    fp = C.POINTER(C.c_float)
+    assert lib.check_gamut_compress(C.c_uint32(1), C.c_uint32(bits(1e37)), thr.ctypes.data_as(fp),
+                                    scl.ctypes.data_as(fp), C.c_float(PWR)) == 0
 
 
 def test_clip_ramp(lib):
