@@ -229,8 +229,8 @@ int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int early,
                    cudaStream_t s);
 
 /* Readies the develop kernels of a debayer method on the current device
- * (their launch attributes, which also loads them): called when a
- * pipeline is created, so that its first frame starts at once. 0 or -5. */
+ * (loads them): called when a pipeline is created, so that its first frame
+ * starts at once. 0 or -5. */
 int craw_k_develop_prepare(int method);
 
 /* 1 (default): the RCD's interior tiles bring their mosaic in with one TMA
