@@ -187,6 +187,10 @@ CRAW_API int craw_batch_create(CRAWContext *ctx, const CRAWBatchParams *params, 
     }
     if ((ret = craw_dev_sync(ctx)) < 0)
         goto fail;
+    if (craw_k_batch_prepare() < 0) {
+        ret = CRAW_ERROR(EIO);
+        goto fail;
+    }
     if (b->denoise) {
         CRAWKBatchFrame *F = &b->table->f[0];
         int32_t dn_items, dv_items;

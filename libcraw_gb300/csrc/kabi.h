@@ -388,6 +388,10 @@ typedef struct CRAWKBatchTable {
 int craw_k_batch(const CRAWKBatchTable *table, int32_t nb, int32_t dn_items, int32_t dv_items,
                  int method, int fused, cudaStream_t s);
 
+/* Loads the batch kernels on the current device: called when a batch is
+ * created, so that its first recording starts at once. 0 or -5. */
+int craw_k_batch_prepare(void);
+
 /* Points every batch kernel node of an instantiated graph (one captured
  * craw_k_batch call) at a new table and item counts. */
 int craw_k_batch_update(cudaGraphExec_t exec, cudaGraph_t graph, const CRAWKBatchTable *table,

@@ -348,6 +348,12 @@ extern "C" int craw_k_batch_shape(int32_t dn_items)
     return dn_items > 2 * (sms > 0 ? sms : 152) ? CRAW_K_BATCH_DN_2x8 : CRAW_K_BATCH_DN_2x4;
 }
 
+extern "C" int craw_k_batch_prepare(void)
+{
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, k_batch_denoise<8>) == cudaSuccess ? 0 : -5;
+}
+
 extern "C" int craw_k_batch(const CRAWKBatchTable *table, int32_t nb, int32_t dn_items,
                             int32_t dv_items, int method, int fused, cudaStream_t s)
 {
