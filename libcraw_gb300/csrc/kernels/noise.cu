@@ -629,7 +629,7 @@ k_noise_lts_float(const double *m, const double *v, const double *lv, int nb, in
  * sort as they do), and one lane adds the `keep` smallest in order. The
  * pairs that came this far gather in `found`; the last CTA to finish picks
  * from them. count: the pairs found, the CTAs done. */
-constexpr int kLtsExactWarps = 8, kLtsSpan = 8, kLtsFew = 48;
+constexpr int kLtsExactWarps = 8, kLtsSpan = 8, kLtsFew = 40;
 
 __global__ void __launch_bounds__(32 * kLtsExactWarps)
 k_noise_lts(const double *m, const double *v, const double *lv, int nb, int np2, int keep, int span,
@@ -811,8 +811,9 @@ extern "C" int craw_k_noise_lts(const double *m, const double *v, const double *
         return -5;
     const int per = kLtsWarps * kLtsPairs;
     const dim3 grid(nb, (nb + per - 1) / per);
-    /* A few bins' pairs are all evaluated in doubles at once, a warp each: a
-     * 640x360 estimate of 32 bins 299 us, 319 through the floats. */
+    /* A few bins' pairs are all evaluated in doubles at once, a warp each:
+     * 8 bins 13.5 us (21.6 through the floats), 32 bins 20.8 (23.8), 40 bins
+     * 26.0 (26.1), 48 bins 30.1 (26.3), 64 bins 40.4 (27.0). */
     const bool few = nb <= kLtsFew;
     if (few) {
         if (cudaMemsetAsync(root, 0, (size_t)nb * nb * sizeof(float), s) != cudaSuccess)
