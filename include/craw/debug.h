@@ -27,10 +27,10 @@ CRAW_API int craw_debug_force_denoise_shape(int shape);
  * comparing the two. Returns the previous setting. */
 CRAW_API int craw_debug_rcd_tma(int on);
 
-/* How the RCD's interior runs: 0 by 64x16 tiles; 1 (the default)
- * and 2 by strips (a lane a quad column, a warp walking down a segment);
- * for comparing the two (they give the same bits). Another value only reads. Returns the previous
- * setting. */
+/* How the RCD runs: 0 by 64x16 tiles; 2 by strips (a lane a quad column, a
+ * warp walking down a segment); 1 (the default) by the sooner of the two for
+ * the frame; for comparing them (they give the same bits). Another value only
+ * reads. Returns the previous setting. */
 CRAW_API int craw_debug_rcd_strips(int mode);
 
 /* 1 (default): the denoise's interior tiles (packed kernels, spatial

@@ -940,8 +940,9 @@ def debug_rcd_tma(on: bool) -> bool:
 
 
 def debug_rcd_strips(mode: int) -> int:
-    """RCD interior by 64x16 tiles (0) or by walking strips (1, the default,
-    and 2); -1 only reads. Returns the previous setting."""
+    """RCD by 64x16 tiles (0), by walking strips (2), or by the sooner of the
+    two for the frame (1, the default); -1 only reads. Returns the previous
+    setting."""
     return int(lib().craw_debug_rcd_strips(int(mode)))
 
 

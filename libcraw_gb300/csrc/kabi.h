@@ -228,18 +228,18 @@ typedef struct CRAWKDevelopIO {
 int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int early,
                    cudaStream_t s);
 
-/* Readies the develop kernels of a debayer method on the current device
- * (loads them): called when a pipeline is created, so that its first frame
- * starts at once. 0 or -5. */
-int craw_k_develop_prepare(int method);
+/* Readies the develop kernels of a debayer method on the current device for
+ * frames of a size, with the gamut compression or not (loads them): called when
+ * a pipeline is created, so that its first frame starts at once. 0 or -5. */
+int craw_k_develop_prepare(int method, int32_t width, int32_t height, int rgc);
 
 /* 1 (default): the RCD's interior tiles bring their mosaic in with one TMA
  * tile copy; 0: with plain loads (craw_debug_rcd_tma). */
 extern int craw_k_rcd_tma;
 
-/* The RCD's interior by 64x16 tiles (0) or by walking strips (one quad
- * column a lane walking down a segment of quad rows: 1, the default, and
- * 2): craw_debug_rcd_strips. The two give the same bits. */
+/* The RCD by 64x16 tiles (0), by walking strips (one quad column a lane
+ * walking down a segment of quad rows: 2), or by the sooner of the two for
+ * the frame (1, the default): craw_debug_rcd_strips. They give the same bits. */
 extern int craw_k_rcd_strips;
 
 /* ------------------------------------------------------------- chroma */

@@ -2,7 +2,7 @@
  * The fused develop stage's launcher, and its RCD by walking warps
  * (develop_walk.cuh): prep + debayer + colour + AWB statistic, the interior and
  * the border in one launch each. The bilinear and MHC frames are
- * develop_linear.cu's, the RCD by tiles develop_rcd_tiles.cu's.
+ * develop_linear.cu's, the small RCD frames by tiles develop_rcd_tiles.cu's.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -12,8 +12,8 @@
 
 /* Whether the RCD interior tiles load their mosaic by TMA (1, the
  * default) or by plain loads (0, for comparison and tests); whether the
- * frame runs by 64x16 tiles with a per-pixel border (0, for comparison and
- * tests) or by walking warps (1, the default; 2). */
+ * frame runs by 64x16 tiles with a per-pixel border (0) or by walking warps
+ * (2), for comparison and tests, or as rcd_by_tiles() says (1, the default). */
 extern "C" {
 int craw_k_rcd_tma = 1;
 int craw_k_rcd_strips = 1;
@@ -135,11 +135,36 @@ int launch_walk(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cud
     }
 }
 
+/* Frames that tiles develop sooner than walking warps (the same bits). The
+ * gamut compression lengthens a warp's steps, and where a frame has work for
+ * a wave or less, its time is a segment's chain of steps; a tile has a thread
+ * a quad. RGBA32F, no denoise before it (after one the walk starts early, the
+ * tiles do not); us by tiles and by walking warps:
+ *                                  512x288    640x362    960x540   1280x720
+ *   AP1                            11.8 11.0  11.5 12.5  14.5 16.5  22.2 20.8
+ *   AP1, FP16 storage              12.3 12.4  11.7 14.5  14.5 18.6  22.1 24.9
+ *   AP1, AWB                       14.7 16.4  15.0 18.6  18.6 20.8  28.1 27.2
+ *   BT.709                         10.5 10.3  10.6 12.4  14.5 12.6  18.7 16.5
+ * (1920x1080: 37.2 31.9, 37.7 39.1, 43.3 40.6, 35.2 23.7.) Not where the
+ * border is two tiles wide (1026x578, AP1: 20.6 18.5), nor for the chroma
+ * path. */
+constexpr int64_t kTilesLeast = 180000, kTilesMost = 800000, kTilesMostMore = 1000000;
+
+bool rcd_by_tiles(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool more, bool early)
+{
+    const int64_t px = (int64_t)k->width * k->height;
+    auto one_wide = [](int n, int tile) { return n % tile == 0 || n % tile >= 6; };
+    return (k->color.flags & CRAW_K_COLOR_RGC) && !io->quarter && !early &&
+           px <= (more ? kTilesMostMore : kTilesMost) && (px >= kTilesLeast || io->awb.hist) &&
+           one_wide(k->width, QTW) && one_wide(k->height, QTH);
+}
+
 int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cudaStream_t s)
 {
-    if (!craw_k_rcd_strips)
+    const bool more = k->fp16 || io->inter || io->quarter || !io->dst;
+    if (craw_k_rcd_strips == 0 || (craw_k_rcd_strips == 1 && rcd_by_tiles(k, io, more, early)))
         return craw_develop_rcd_tiles(k, io, s);
-    if (k->fp16 || io->inter || io->quarter || !io->dst)
+    if (more)
         return launch_walk<0, -1, true>(k, io, early, s);
     return k->color.flags & CRAW_K_COLOR_RGC ? launch_walk<1>(k, io, early, s) : launch_walk<0>(k, io, early, s);
 }
@@ -149,12 +174,14 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cuda
 /* A debayer's kernels are a module each, which the runtime loads whole where
  * the first of them is asked for: some hundred microseconds, here rather
  * than in a pipeline's first frame. */
-extern "C" int craw_k_develop_prepare(int method)
+extern "C" int craw_k_develop_prepare(int method, int32_t width, int32_t height, int rgc)
 {
     cudaFuncAttributes a;
     (void)craw_sm_count();
     if (method != kRcd)
         return craw_develop_linear_prepare();
+    if (rgc && (int64_t)width * height <= kTilesMostMore && craw_develop_rcd_tiles_prepare() < 0)
+        return -5;
     return cudaFuncGetAttributes(&a, k_develop_rcd_walk<CRAW_K_OUT_RGBA32F, 0, false>) == cudaSuccess ? 0 : -5;
 }
 

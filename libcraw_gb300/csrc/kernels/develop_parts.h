@@ -14,6 +14,9 @@ int craw_develop_linear(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool ea
 /* Loads those kernels on the current device; 0 or -5. */
 int craw_develop_linear_prepare();
 
-/* An RCD frame by 64x16 tiles and a per-pixel border (develop_rcd_tiles.cu),
- * for comparison and tests; 0 or -5. */
+/* An RCD frame by 64x16 tiles and a per-pixel border (develop_rcd_tiles.cu);
+ * 0 or -5. */
 int craw_develop_rcd_tiles(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s);
+
+/* Loads those kernels on the current device; 0 or -5. */
+int craw_develop_rcd_tiles_prepare();

@@ -1,7 +1,7 @@
 /*
- * The RCD by 64x16 tiles (develop_tile.cuh), for comparison and tests
- * (craw_debug_rcd_strips(0)): the interior by CFA quads, its mosaic by a TMA
- * tile copy or by plain loads, the border a pixel a thread.
+ * The RCD by 64x16 tiles (develop_tile.cuh), where a frame is small and has the
+ * gamut compression (develop.cu's rule): the interior by CFA quads, its mosaic
+ * by a TMA tile copy or by plain loads, the border a pixel a thread.
  */
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -126,13 +126,22 @@ k_develop_rcd_border(const CRAWKDevelop k, const CRAWKDevelopIO io, const QuadGr
 
 } // namespace
 
+/* Their shared-memory sizes, set once per device, which also loads them. */
+int craw_develop_rcd_tiles_prepare()
+{
+    constexpr size_t smem = RcdQuads<QTW, QTH, QNT>::floats * sizeof(float);
+    static std::atomic<uint64_t> attr_plain{ 0 }, attr_tma{ 0 };
+    return craw_smem_attr(k_develop_rcd_quads, smem, attr_plain) < 0 ||
+                   craw_smem_attr(k_develop_rcd_quads_tma, smem, attr_tma) < 0
+               ? -5
+               : 0;
+}
+
 /* The border may begin beside the interior, and ends no earlier than it. */
 int craw_develop_rcd_tiles(const CRAWKDevelop *k, const CRAWKDevelopIO *io, cudaStream_t s)
 {
     constexpr size_t smem = RcdQuads<QTW, QTH, QNT>::floats * sizeof(float);
-    static std::atomic<uint64_t> attr_plain{ 0 }, attr_tma{ 0 };
-    if (craw_smem_attr(k_develop_rcd_quads, smem, attr_plain) < 0 ||
-        craw_smem_attr(k_develop_rcd_quads_tma, smem, attr_tma) < 0)
+    if (craw_develop_rcd_tiles_prepare() < 0)
         return -5;
     QuadGrid g;
     g.init(k->width, k->height);
