@@ -355,8 +355,9 @@ struct HlRow {
  * Bound: instruction issue, the lifts' logarithms and exponentials above all
  * where a frame is clipped: so short segments, which the hardware hands out
  * as CTAs end (one wave of 67 rows each took 152 us, 16 rows 113). 6000x4000,
- * most of it clipped: 105 us, where tiles staged in shared memory took 126. */
-constexpr int kFillN = 30, kFillCtas = 7, kFillSeg = 8;
+ * most of it clipped: 105 us, where tiles staged in shared memory took 126.
+ * A small frame's time is its segment's chain of rows: fill_rows(). */
+constexpr int kFillN = 30, kFillCtas = 7, kFillMost = 8, kFillWaves = 5;
 
 __global__ void __launch_bounds__(kWalkNT, kFillCtas)
 k_hl_fill(const CRAWKHighlight k, const CRAWKHighlightIO io, const HlGrid g)
@@ -477,14 +478,28 @@ k_hl_fill(const CRAWKHighlight k, const CRAWKHighlightIO io, const HlGrid g)
     }
 }
 
+/* The rows of k_hl_fill's segments: the fewest of 2, 4 and 8 that are at most
+ * kFillWaves waves of warps. A frame's highlights and bilinear develop with 8,
+ * 4 and 2: 320x240 33, 29 and 27 us; 1280x720 45, 40 and 40; 2560x1440 73, 69
+ * and 69; 3840x2160 121, 119 and 121. */
+int fill_rows(int nx, int qh)
+{
+    int seg = 2;
+    while (seg < kFillMost && (int64_t)nx * ((qh + seg - 1) / seg) > 152 * kFillCtas * kWalkWarps * kFillWaves)
+        seg *= 2;
+    return seg;
+}
+
 /* Segments of one wave of `ctas` CTAs an SM for strips of `cols` quads, a
- * multiple of 2 quad rows (texels have two), at least 8; returns the CTAs. */
+ * multiple of 2 quad rows (texels have two), at least 4 (6 rows more are read
+ * for each: 320x240 with 8 37 us, with 4 33, 1600x900 with 2 52 and with 4 50);
+ * returns the CTAs. */
 int hl_grid(HlGrid &g, int qw, int qh, int cols, int ctas)
 {
     g.nx = (qw + cols - 1) / cols;
     const int room = 152 * ctas * kWalkWarps / g.nx, n = room > 1 ? room : 1;
     g.seg = ((qh + n - 1) / n + 1) / 2 * 2;
-    g.seg = g.seg < 8 ? 8 : g.seg;
+    g.seg = g.seg < 4 ? 4 : g.seg;
     return (g.nx * ((qh + g.seg - 1) / g.seg) + kWalkWarps - 1) / kWalkWarps;
 }
 
@@ -536,7 +551,8 @@ extern "C" int craw_k_highlights(const CRAWKHighlight *k, const CRAWKHighlightIO
     for (int l = lc - 1; l >= 0; l--)
         if (craw_launch_early(k_hl_push, grid2(k->lw[l], k->lh[l]), blk, 0, true, s, *k, *io, l) < 0)
             return -5;
-    g = HlGrid{ (qw + kFillN - 1) / kFillN, kFillSeg };
+    g.nx = (qw + kFillN - 1) / kFillN;
+    g.seg = fill_rows(g.nx, qh);
     ctas = (g.nx * ((qh + g.seg - 1) / g.seg) + kWalkWarps - 1) / kWalkWarps;
     return craw_launch_early(k_hl_fill, ctas, kWalkNT, 0, true, s, *k, *io, g);
 }
