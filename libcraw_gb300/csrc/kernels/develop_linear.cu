@@ -15,10 +15,12 @@ using namespace craw_dev;
 
 /* Every bilinear and MHC frame: CTAs an SM (5 of 96 registers for MHC and 6
  * of 80 for bilinear, a few spilled, run 7 % faster at 5760x3240 than 4 and
- * 5 without a spill). */
+ * 5 without a spill). With a kept intermediate bilinear takes 121 us a
+ * 5760x3240 frame with 4 (RGBA32F, no AWB) and 128 with 3, MHC of RGB32F 117
+ * with 4 and 108 with 3. */
 template <int METHOD, int EPI> constexpr int linear_ctas()
 {
-    return EPI == LW_ANY ? 3 : (METHOD == kMhc ? 5 : 6);
+    return EPI == LW_ANY ? (METHOD == kMhc ? 3 : 4) : (METHOD == kMhc ? 5 : 6);
 }
 
 template <int METHOD, int EPI>
