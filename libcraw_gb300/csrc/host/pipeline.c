@@ -593,8 +593,8 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
     if (p->awb) {
         p->nb_blocks = ((w + 7) / 8) * ((h + 7) / 8);
         for (uint32_t i = 0; i < p->nb_slots; i++) {
-            /* Room for every block, and at least for the part the slot's
-             * async copy reads. */
+            /* Room for every block, and at least for the part that is
+             * published into the slot's host copy. */
             const size_t entries = CRAW_MAX((size_t)p->nb_blocks, (size_t)CRAW_K_AWB_DEFER_MAX);
             if ((ret = craw_dev_alloc(ctx, (void **)&p->slots[i].dev,
                                       ZERO_BYTES + entries * sizeof(CRAWKAwbDeferred))) < 0)

@@ -7,7 +7,7 @@
  *   k_hl_level0    one texel per 2x2 quads: weighted log chroma (ln R/G,
  *                  ln B/G) of the quads, and the weight, which falls to 0
  *                  within 3 quads of a clip (the quads' clip ramps and
- *                  their 7x7 max are made in shared memory on the way)
+ *                  their 7x7 max are made in registers on the way)
  *   k_hl_pull      each coarser level the sum of its four children, to 1x1
  *   k_hl_coarse    the levels of at most kCoarseTexels, pulled and pushed
  *                  in one CTA
