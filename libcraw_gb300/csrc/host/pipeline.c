@@ -656,8 +656,7 @@ CRAW_API int craw_pipeline_create(CRAWContext *ctx, const CRAWPipelineParams *pa
     }
     if ((ret = craw_dev_sync(ctx)) < 0)
         goto fail;
-    if (!p->plain && craw_k_develop_prepare(params->debayer, (int32_t)w, (int32_t)h,
-                                            params->out_space == CRAW_CS_ACES_AP1_LINEAR) < 0) {
+    if (!p->plain && craw_k_develop_prepare(params->debayer, (int32_t)w, (int32_t)h) < 0) {
         ret = CRAW_ERROR(EIO);
         goto fail;
     }

@@ -229,9 +229,9 @@ int craw_k_develop(const CRAWKDevelop *k, const CRAWKDevelopIO *io, int early,
                    cudaStream_t s);
 
 /* Readies the develop kernels of a debayer method on the current device for
- * frames of a size, with the gamut compression or not (loads them): called when
- * a pipeline is created, so that its first frame starts at once. 0 or -5. */
-int craw_k_develop_prepare(int method, int32_t width, int32_t height, int rgc);
+ * frames of a size (loads them): called when a pipeline is created, so that
+ * its first frame starts at once. 0 or -5. */
+int craw_k_develop_prepare(int method, int32_t width, int32_t height);
 
 /* 1 (default): the RCD's interior tiles bring their mosaic in with one TMA
  * tile copy; 0: with plain loads (craw_debug_rcd_tma). */

@@ -174,13 +174,14 @@ int launch_rcd(const CRAWKDevelop *k, const CRAWKDevelopIO *io, bool early, cuda
 /* A debayer's kernels are a module each, which the runtime loads whole where
  * the first of them is asked for: some hundred microseconds, here rather
  * than in a pipeline's first frame. */
-extern "C" int craw_k_develop_prepare(int method, int32_t width, int32_t height, int rgc)
+extern "C" int craw_k_develop_prepare(int method, int32_t width, int32_t height)
 {
     cudaFuncAttributes a;
     (void)craw_sm_count();
     if (method != kRcd)
         return craw_develop_linear_prepare();
-    if (rgc && (int64_t)width * height <= kTilesMostMore && craw_develop_rcd_tiles_prepare() < 0)
+    /* Whatever the pipeline's own output space: a frame may ask for another. */
+    if ((int64_t)width * height <= kTilesMostMore && craw_develop_rcd_tiles_prepare() < 0)
         return -5;
     return cudaFuncGetAttributes(&a, k_develop_rcd_walk<CRAW_K_OUT_RGBA32F, 0, false>) == cudaSuccess ? 0 : -5;
 }

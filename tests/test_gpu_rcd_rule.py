@@ -4,10 +4,11 @@ storage 1000000, borders two tiles wide, after a denoise): its choice, the
 tiles and the walking warps give the same bits."""
 import numpy as np
 import pytest
+import torch
 
 import libcraw_gb300 as L
 from libcraw_gb300 import workloads as W
-from gpu_util import develop, download_image
+from gpu_util import alloc_rgba, develop, download_image, upload_mosaic
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +56,46 @@ def test_choice_gives_the_same_bits(ctx, w, h, fmt, storage, flags):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert np.array_equal(np.ascontiguousarray(a).view(np.uint8), np.ascontiguousarray(b).view(np.uint8))
+
+
+FRAMES = 4
+
+
+def recorded(graph, out_space, frame_space):
+    """Frames of a clip recorded by tiles back to back into their own images
+    (in a graph, the process's first use of the kernels): outputs, histograms."""
+    w, h = 640, 362
+    srcs = [upload_mosaic(W.highlight_frame(w, h, 5 + i)) for i in range(FRAMES)]
+    outs = [alloc_rgba(w, h) for _ in srcs]
+    kw = {} if frame_space is None else dict(out_space=frame_space, out_space_set=True)
+    fp = L.frame_params(W.make_profile(), **kw)
+    pp = L.pipeline_params(w, h, debayer=L.DEBAYER_RCD, out_space=out_space, out_format=L.FORMAT_RGBA32F,
+                           flags=L.FLAG_AWB_HISTOGRAM, nb_awb_slots=FRAMES)
+    with L.Context(0) as c, L.Pipeline(c, pp) as pipe:
+        s = torch.cuda.Stream()
+        torch.cuda.synchronize()
+
+        def frames(wait):
+            for (_, src), (_, dst) in zip(srcs, outs):
+                pipe.record(s.cuda_stream, src, dst, fp)
+                if wait:
+                    torch.cuda.synchronize()
+        if graph:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                frames(False)
+            g.replay()
+        else:
+            frames(graph is None)
+        torch.cuda.synchronize()
+        assert pipe.kernel_errors() == 0
+        hist = [pipe.awb_histogram(i) for i in range(FRAMES)]
+    return [o.cpu().numpy() for o, _ in outs] + [a for x in hist for a in (x.count, x.weight, x.weight_bright)]
+
+
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("frame_space", [None, L.CS_ACES_AP1])
+def test_back_to_back(graph, frame_space):
+    space = L.CS_ACES_AP1 if frame_space is None else L.CS_BT709
+    got, want = recorded(graph, space, frame_space), recorded(None, L.CS_ACES_AP1, None)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
